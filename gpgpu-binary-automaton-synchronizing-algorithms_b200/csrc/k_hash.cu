@@ -20,9 +20,13 @@
 // synchronous, as GPGPU/CPU/SlimCPUUntweaked.cs:119-184), tests the images
 // against the set (atomicCAS insert), and appends the new ones compacted by
 // ballots in queue order.  An automaton that needs more than 3/4 of the set's
-// slots or kHashLevelCap levels (a Cerny automaton: (n-1)^2 levels) is handed
+// slots or kHashLevelCap levels is tried backwards by the same warp
+// (inverse_search below), which settles the slowly synchronizing families and
+// the automata that never synchronize; what is left -- wide both ways -- goes
 // to the CTA-wide kernel through a list.  Random n = 17..20: 1.7 % of the
-// automata pass 1536 subsets, 0.3 % pass 4096.
+// automata pass 1536 subsets, 0.3 % pass 4096.  200K mixed n = 6..20 with 1 %
+// Cerny automata: 3.04 ms with every such automaton on the CTA-wide kernel,
+// 1.20 ms with the inverse search.
 #include <atomic>
 
 #include "common.cuh"
@@ -31,13 +35,16 @@ namespace sbfs {
 namespace {
 
 constexpr uint32_t kHashLevelCap = 48;         // random n <= 20: at most ~40 levels
-constexpr uint32_t kSubsetMask = (1u << 20) - 1u;
+constexpr uint32_t kUnsettled = 1u << 31;
 
 template <int CAP_BITS>
 struct HashGeom {
     static constexpr int kCap = 1 << CAP_BITS;                  // hash slots per warp
     static constexpr uint32_t kLimit = 3u * (1u << CAP_BITS) / 4u;   // subsets a warp keeps
     static constexpr int kWarps = CAP_BITS <= 11 ? 5 : 2;        // warps per CTA (~75 KB)
+    static constexpr int kMaxN = 20;
+    static constexpr uint32_t kSubsetMask = (1u << kMaxN) - 1u;
+    static constexpr uint32_t kGens = 1u << (32 - kMaxN);        // generation 0 marks never-used slots
 };
 
 template <int CAP_BITS>
@@ -76,9 +83,192 @@ __device__ __forceinline__ int set_insert(uint32_t *set, uint32_t x, uint32_t ge
     return -1;   // unreachable: the set is never more than ~3/4 full
 }
 
+// Entries of the five nibble tables from one 64-bit mask pair per state (lane q
+// holds state q's, a's mask << 32 | b's): 80 entries in three passes that every
+// lane takes (the shuffles need the whole warp), the third storing lanes 0..15
+// only.
+template <int CAP_BITS>
+__device__ __forceinline__ void build_table(HashWarp<CAP_BITS> &W, uint64_t mine, int n, int lane)
+{
+#pragma unroll
+    for (int pass = 0; pass < 3; ++pass) {
+        const int e = lane + 32 * pass;
+        const int c = min(e >> 4, 4), v = e & 15;
+        uint64_t acc = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t sj = __shfl_sync(kFull, mine, 4 * c + j);
+            if (((v >> j) & 1) && 4 * c + j < n) acc |= sj;
+        }
+        if (e < 5 * 16) W.table[e] = acc;
+    }
+}
+
+// a's mask << 32 | b's mask of subset x
+template <int CAP_BITS>
+__device__ __forceinline__ uint64_t lookup(const HashWarp<CAP_BITS> &W, uint32_t x)
+{
+    return W.table[x & 15u] | W.table[16 + ((x >> 4) & 15u)] | W.table[32 + ((x >> 8) & 15u)] |
+           W.table[48 + ((x >> 12) & 15u)] | W.table[64 + ((x >> 16) & 15u)];
+}
+
+// The generation of the next search; the set is cleared when they wrap.
+template <int CAP_BITS>
+__device__ __forceinline__ void next_generation(HashWarp<CAP_BITS> &W, uint32_t &gen, int lane)
+{
+    if (++gen == HashGeom<CAP_BITS>::kGens) {
+        for (int i = lane; i < HashGeom<CAP_BITS>::kCap; i += 32) W.set[i] = 0u;
+        gen = 1;
+        __syncwarp();
+    }
+}
+
+__device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t k, int n)
+{
+    record_result(b, k, n, kLenNonSync);
+    if (b.out_words)
+        for (int c = 0; c < b.word_stride; ++c) b.out_words[(size_t)k * b.word_stride + c] = 0ull;
+    publish_result(b, k);
+}
+
+// The inverse search, for an automaton that the forward search gave up on
+// (lane q < n holds a(q) and b(q)).  A word w synchronizes iff w^-1(q) is the
+// full set for some state q, and (cw)^-1(q) = c^-1(w^-1(q)): so a breadth-first
+// search from the n singletons along preimages reaches the full set first at
+// the length of the shortest word, and the parent chain from there spells the
+// word from its first letter on.  It runs out without the full set iff the
+// automaton is not synchronizing.
+//
+// The slowly synchronizing families (Cerny automata, a permutation plus one
+// merge) have up to 2^n images of the full set but at most n(n-1)+1 preimages
+// of singletons: C_20 is settled by 380 sets over 361 levels (tens of
+// microseconds in one warp; all 2^20 forward subsets took a 1024-thread CTA
+// 1.2 ms).  Their levels hold 1 to n sets; a random automaton whose forward
+// search is wide passes n sets in a level at its fifth or sixth (9,000 random
+// n = 13..28 with over 1536 images: none was settled before that).  So the
+// search stops at the first level wider than n sets, which also keeps every
+// level within one step of the warp.
+//
+// Before giving up, pairs of states settle the wide automata that never
+// synchronize: an automaton synchronizes iff every pair of its states is merged
+// by some word.  Row q (lane q) collects the states that can be merged with q,
+// preimages of the rows of a(q) and b(q), until nothing changes.
+//
+// Takes a fresh generation; returns the sets this lane expanded, with the top
+// bit clear when the automaton is settled and set when it is left to the
+// CTA-wide kernel.
+template <int CAP_BITS>
+__device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n, uint32_t av, uint32_t bv,
+                                                HashWarp<CAP_BITS> &W, uint32_t gen, int lane)
+{
+    using G = HashGeom<CAP_BITS>;
+    uint32_t expanded = 0;
+    const uint32_t full = (1u << n) - 1u;
+    // lane q: the states that a (b) sends to q
+    uint64_t inv = 0;
+    for (int q = 0; q < n; ++q) {
+        const unsigned ia = __ballot_sync(kFull, lane < n && av == (uint32_t)q);
+        const unsigned ib = __ballot_sync(kFull, lane < n && bv == (uint32_t)q);
+        if (lane == q) inv = ((uint64_t)ia << 32) | ib;
+    }
+    build_table<CAP_BITS>(W, inv, n, lane);
+    __syncwarp();
+    if (lane < n) W.queue[lane] = (uint16_t)set_insert<CAP_BITS>(W.set, 1u << lane, gen);
+    __syncwarp();
+    uint32_t head = 0, lvl_end = (uint32_t)n, tail = lvl_end, level = 0;
+    uint32_t found = 0, found_letter = 0;
+    bool hit = false, spent = true;   // spent: no set left to expand
+    while (head < lvl_end) {
+        const uint32_t idx = head + (uint32_t)lane;
+        const bool has = idx < lvl_end;
+        uint32_t ya = 0, yb = 0;
+        if (has) {
+            const uint64_t t = lookup<CAP_BITS>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
+            ya = (uint32_t)(t >> 32);
+            yb = (uint32_t)t;
+        }
+        expanded += has ? 1u : 0u;
+        const unsigned hits = __ballot_sync(kFull, ya == full || yb == full);
+        if (hits) {
+            const int fl = __ffs(hits) - 1;
+            found = head + (uint32_t)fl;
+            found_letter = (uint32_t)__shfl_sync(kFull, ya == full ? 0 : 1, fl);
+            hit = true;
+            break;
+        }
+        const int sa = ya ? set_insert<CAP_BITS>(W.set, ya, gen) : -1;
+        const int sb = yb ? set_insert<CAP_BITS>(W.set, yb, gen) : -1;
+        bool fa = sa >= 0, fb = sb >= 0;
+        const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
+        const uint32_t added = (uint32_t)(__popc(ma) + __popc(mb));
+        if (tail + added > min(G::kLimit, lvl_end + (uint32_t)n)) {
+            spent = false;
+            break;
+        }
+        const unsigned lt = (1u << lane) - 1u;
+        uint32_t p = tail + (uint32_t)(__popc(ma & lt) + __popc(mb & lt));
+        if (!SBFS_CHECK(p + (fa ? 1u : 0u) + (fb ? 1u : 0u) <= G::kLimit, b.error)) fa = fb = false;
+        if (fa) {
+            W.queue[p] = (uint16_t)sa;
+            W.parent[p++] = (uint16_t)idx;
+        }
+        if (fb) {
+            W.queue[p] = (uint16_t)(sb | 0x8000);
+            W.parent[p] = (uint16_t)idx;
+        }
+        tail += added;
+        head = lvl_end;   // a level is one step: at most n sets
+        lvl_end = tail;
+        __syncwarp();
+        if (head < lvl_end) ++level;
+    }
+    if (hit) {
+        __syncwarp();
+        if (lane == 0) {
+            record_result(b, k, n, (int32_t)level + 1);
+            if (b.out_words) {
+                uint64_t *w = b.out_words + (size_t)k * (size_t)b.word_stride;
+                uint64_t acc = found_letter;
+                int c = 0;
+                uint32_t i = found;
+                if (level < 64u * (uint32_t)b.word_stride) {
+                    for (uint32_t d = 1; d <= level; ++d) {
+                        if ((d & 63u) == 0u) {
+                            w[c++] = acc;
+                            acc = 0ull;
+                        }
+                        acc |= (uint64_t)(W.queue[i] >> 15) << (d & 63u);
+                        i = W.parent[i];
+                    }
+                    w[c++] = acc;
+                }
+                for (; c < b.word_stride; ++c) w[c] = 0ull;
+            }
+            publish_result(b, k);
+        }
+        __syncwarp();
+        return expanded;
+    }
+    if (!spent) {
+        uint32_t row = lane < n ? 1u << lane : 0u;
+        while (true) {
+            const uint32_t ra = __shfl_sync(kFull, row, (int)av), rb = __shfl_sync(kFull, row, (int)bv);
+            const uint32_t grown =
+                row | (uint32_t)(lookup<CAP_BITS>(W, ra) >> 32) | (uint32_t)lookup<CAP_BITS>(W, rb);
+            const bool more = lane < n && grown != row;
+            if (lane < n) row = grown;
+            if (!__any_sync(kFull, more)) break;
+        }
+        if (__all_sync(kFull, lane >= n || row == full)) return expanded | kUnsettled;
+    }
+    if (lane == 0) write_not_synchronizing(b, k, n);
+    __syncwarp();
+    return expanded;
+}
+
 template <int CAP_BITS>
 __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
-    k_hash(Batch b, int32_t *heavy_list, unsigned long long *heavy_count, unsigned long long *ticket)
+    k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count, unsigned long long *ticket)
 {
     using G = HashGeom<CAP_BITS>;
     constexpr int kHashCap = G::kCap;
@@ -104,10 +294,12 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
         const int64_t k = automaton_at(order, (int64_t)pos);
         const int n = automaton_n(b, k);
         const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
-        bool bad = n < 1 || n > 20 || n > b.lstride;
+        bool bad = n < 1 || n > G::kMaxN || n > b.lstride;
         uint64_t single = 0;
+        uint32_t av = 0, bv = 0;
         if (!bad && lane < n) {
-            const uint32_t av = rec[lane], bv = rec[b.lstride + lane];
+            av = rec[lane];
+            bv = rec[b.lstride + lane];
             if (av >= (uint32_t)n || bv >= (uint32_t)n)
                 bad = true;
             else
@@ -123,25 +315,8 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
             }
             continue;
         }
-        // nibble tables: 80 entries in three passes that every lane takes (the
-        // shuffles need the whole warp), the third storing lanes 0..15 only
-#pragma unroll
-        for (int pass = 0; pass < 3; ++pass) {
-            const int e = lane + 32 * pass;
-            const int c = min(e >> 4, 4), v = e & 15;
-            uint64_t acc = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint64_t sj = __shfl_sync(kFull, single, 4 * c + j);
-                if (((v >> j) & 1) && 4 * c + j < n) acc |= sj;
-            }
-            if (e < 5 * 16) W.table[e] = acc;
-        }
-        if (++gen == (1u << 12)) {   // generations wrapped: clear once, start again at 1
-            for (int i = lane; i < kHashCap; i += 32) W.set[i] = 0u;
-            gen = 1;
-            __syncwarp();
-        }
+        build_table<CAP_BITS>(W, single, n, lane);
+        next_generation<CAP_BITS>(W, gen, lane);
         const uint32_t full = (1u << n) - 1u;
         if (lane == 0) W.queue[0] = (uint16_t)set_insert<CAP_BITS>(W.set, full, gen);
         __syncwarp();
@@ -155,9 +330,7 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
             const bool has = idx < lvl_end;
             uint32_t ya = 0, yb = 0;
             if (has) {
-                const uint32_t x = W.set[W.queue[idx] & 0x7FFFu] & kSubsetMask;
-                uint64_t t = W.table[x & 15u] | W.table[16 + ((x >> 4) & 15u)] | W.table[32 + ((x >> 8) & 15u)] |
-                             W.table[48 + ((x >> 12) & 15u)] | W.table[64 + ((x >> 16) & 15u)];
+                const uint64_t t = lookup<CAP_BITS>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
                 ya = (uint32_t)(t >> 32);
                 yb = (uint32_t)t;
             }
@@ -205,8 +378,13 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
         }
         __syncwarp();
         if (heavy) {
-            // a long or wide search: the CTA-wide kernel takes it from the start
-            if (lane == 0) heavy_list[atomicAdd(heavy_count, 1ull)] = (int32_t)k;
+            // a long or wide search: backwards from the singletons, and if that is
+            // wide too the CTA-wide kernel takes it from the start
+            next_generation<CAP_BITS>(W, gen, lane);
+            const uint32_t r = inverse_search<CAP_BITS>(b, k, n, av, bv, W, gen, lane);
+            expanded += r & ~kUnsettled;
+            if ((r & kUnsettled) && lane == 0) heavy_list[atomicAdd(heavy_count, 1ull)] = (int32_t)k;
+            __syncwarp();
             continue;
         }
         if (lane == 0) {
