@@ -32,10 +32,12 @@ int cta_max_ctas_per_sm(int nb_max, int threads);
 cudaError_t launch_cta(int nb_max, int threads, int ctas, const Batch &b, uint64_t *queues,
                        unsigned long long *ticket, cudaStream_t st);
 cudaError_t plan_autotune(sbfs_handle *h, Plan &plan);
-int hash_max_ctas_per_sm(int size);
+int hash_max_ctas_per_sm(int size, int max_n);
 cudaError_t launch_sort_handoff(const Batch &b, const int32_t *list, const unsigned long long *count, int32_t *out,
                                 int top_n, unsigned long long *split, cudaStream_t st);
-cudaError_t launch_hash(int size, int ctas, const Batch &b, int32_t *heavy_list, unsigned long long *heavy_count,
+cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
+                        unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st);
+cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
                         unsigned long long *ticket, cudaStream_t st);
 
 cudaError_t DevBuf::reserve(size_t want)
@@ -176,28 +178,29 @@ size_t level_arena_bytes(sbfs_handle *h, int max_n)
     return want;
 }
 
-// Automata with 21 <= n <= 28 run on the device-resident level slots: admit as
-// many as the arena holds, advance them a few levels per launch batch, collect
-// the finished ones, admit more.  Results land in the job's device outputs.
+// Automata that no on-chip kernel settled (n up to 28) run on the device-resident
+// level slots: admit as many as the arena holds, advance them a few levels per
+// launch batch, collect the finished ones, admit more.  Results land in the
+// job's device outputs.  The members are bc.order[range], read back from the
+// device, or the whole uniform job when bc has no range.
 sbfs_status run_level_class(sbfs_handle *h, Lane &L, const Job &j, const Batch &bc, int *launches)
 {
     std::vector<std::pair<int64_t, int>> items;
-    if (!j.ns) {
+    if (!bc.range_dev) {
         items.reserve((size_t)j.count);
         for (int64_t i = 0; i < j.count; ++i) items.push_back({i, j.n_uniform});
     } else {
-        // class-4 members come from the device bucketing: read the range, the order slice and sizes
         unsigned long long range[2] = {0, 0};
         CK(cudaMemcpyAsync(range, bc.range_dev, sizeof(range), cudaMemcpyDeviceToHost, L.stream),
            "reading class range");
-        CK(cudaStreamSynchronize(L.stream), "waiting for bucketing");
+        CK(cudaStreamSynchronize(L.stream), "waiting for class members");
         if (range[1] == 0) return SBFS_OK;
         std::vector<int32_t> idx((size_t)range[1]);
-        std::vector<uint8_t> ns((size_t)j.count);
+        std::vector<uint8_t> ns(j.ns ? (size_t)j.count : 0);
         CK(cudaMemcpy(idx.data(), bc.order + range[0], idx.size() * sizeof(int32_t), cudaMemcpyDeviceToHost),
            "reading class members");
-        CK(cudaMemcpy(ns.data(), j.ns, ns.size(), cudaMemcpyDeviceToHost), "reading sizes");
-        for (int32_t i : idx) items.push_back({i, ns[(size_t)i]});
+        if (j.ns) CK(cudaMemcpy(ns.data(), j.ns, ns.size(), cudaMemcpyDeviceToHost), "reading sizes");
+        for (int32_t i : idx) items.push_back({i, j.ns ? ns[(size_t)i] : j.n_uniform});
     }
     if (items.empty()) return SBFS_OK;
     int max_n = 0;
@@ -338,12 +341,12 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
             } else {
                 // one warp per automaton with a hash set; searches wider than its
                 // set or longer than its level cap go to the CTA-wide kernel, same stream
-                const int hper = hash_max_ctas_per_sm(size);
+                const int hper = hash_max_ctas_per_sm(size, kClassMaxN[c]);
                 if (hper < 1) return fail(h, SBFS_ECUDA, "hash-set kernel does not fit on an SM");
                 // hand-off list | the same sorted by n, largest first (mixed sizes)
                 CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off list");
                 int32_t *list = L.heavy[c].as<int32_t>();
-                CK(launch_hash(size, hper * h->sm_count, bc, list, &ctr->heavy_range[c][1], ticket, cs),
+                CK(launch_hash(size, kClassMaxN[c], hper * h->sm_count, bc, list, &ctr->heavy_range[c][1], ticket, cs),
                    "launching hash-set kernel");
                 Batch bh = bc;
                 bh.order = list;
@@ -416,6 +419,23 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
             CK(L.cta_queue.reserve(cta_queue_entries(nb, ctas) * sizeof(uint64_t)), "allocating CTA queues");
             CK(launch_cta(nb, P.cta.threads, ctas, bc, L.cta_queue.as<uint64_t>(), ticket, st), "launching n<=20 kernel");
         } else {
+            if (!plain && !ticket_override) {
+                // one warp per automaton, then one CTA per automaton, both on chip; the
+                // level slots take what is wider than that (one read-back to see if any is)
+                const int hper = hash_max_ctas_per_sm(2, SBFS_MAX_N);
+                if (hper < 1) return fail(h, SBFS_ECUDA, "hash-set kernel does not fit on an SM");
+                CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off list");
+                int32_t *list = L.heavy[c].as<int32_t>();
+                CK(launch_hash(2, SBFS_MAX_N, hper * h->sm_count, bc, list, &ctr->heavy_range[c][1], ticket, cs),
+                   "launching hash-set kernel");
+                bc.order = list;
+                bc.range_dev = ctr->heavy_range[c];
+                CK(launch_wide(h->sm_count, bc, list + escal_entries, &ctr->wide_range[1], &ctr->heavy_ticket[c], cs),
+                   "launching CTA-wide hash-set kernel");
+                bc.order = list + escal_entries;
+                bc.range_dev = ctr->wide_range;
+                *launches += 2;
+            }
             sbfs_status ls = run_level_class(h, L, j, bc, launches);
             if (ls) return ls;
             continue;
@@ -1320,10 +1340,8 @@ sbfs_status sbfs_destroy(sbfs_handle *h)
             if (L.ev_join[c]) cudaEventDestroy(L.ev_join[c]);
             L.spill_c[c].release();
         }
-        for (int c = 0; c < 4; ++c) {
-            L.heavy[c].release();
-            L.heavy_queue[c].release();
-        }
+        for (DevBuf &d : L.heavy) d.release();
+        for (DevBuf &d : L.heavy_queue) d.release();
         if (L.level_ready) L.level.destroy();
         if (L.stream) cudaStreamDestroy(L.stream);
     }

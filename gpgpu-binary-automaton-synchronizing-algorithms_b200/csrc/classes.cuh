@@ -11,7 +11,9 @@ namespace sbfs {
 // class 1: n <= 12  warp-pooled kernel, 512-byte bitmap
 // class 2: n <= 16  warp-pooled kernel, 8 KiB bitmap
 // class 3: n <= 20  one automaton per CTA, bitmap (<= 128 KiB) in shared memory
-// class 4: n <= 28  level-synchronous, bitmap (<= 32 MiB) and frontier in HBM
+// class 4: n <= 28  one automaton per warp, then per CTA, with a hash set in shared
+//                   memory; what outgrows both: level-synchronous, bitmap (<= 32 MiB)
+//                   and frontier in HBM
 constexpr int kNumClasses = 5;
 constexpr int kClassMaxN[kNumClasses] = {8, 12, 16, 20, 28};
 // Out-of-range n (0 or > 28) is routed to class 0, whose kernel rejects it

@@ -1,5 +1,5 @@
-// k_hash.cu -- power-set BFS of automata with 13..20 states (size classes 2
-// and 3) with one warp per automaton and an open-addressed hash set as the
+// k_hash.cu -- power-set BFS of automata with 13..28 states (size classes 2,
+// 3 and 4) with one warp per automaton and an open-addressed hash set as the
 // visited store.
 //
 // A random automaton of 13..20 states is settled after a few hundred subsets
@@ -8,14 +8,19 @@
 // itself: the CTA's per-level barriers and round trips dominate.  Here each
 // warp keeps in shared memory
 //   * nibble tables: table[c][v] = (a-image << 32) | b-image of the states
-//     4c..4c+3 selected by v, so both images of a subset are 5 loads;
-//   * a hash set of 2^CAP_BITS slots, each holding subset | generation << 20;
-//     the generation changes with every automaton, so a slot from an earlier
-//     automaton reads as empty and the set is cleared once per 4095 automata;
+//     4c..4c+3 selected by v, so both images of a subset are 4, 5 or 7 loads
+//     (instances for n <= 16, 20 and 28: four instead of five at n = 16 is
+//     1.124 -> 1.120 ms per 200K automata);
+//   * a hash set of 2^CAP_BITS slots, each holding subset | generation << MAXN;
+//     the generation changes with every search, so a slot from an earlier one
+//     reads as empty and the set is cleared when the generations (2^(32 - MAXN))
+//     wrap;
 //   * a level-ordered queue of 16-bit entries, set slot | letter-is-b << 15
 //     (a slot keeps its subset for the whole search), with a 16-bit parent
 //     index per entry, retained for the word (GPGPU/CPU/CPU.cs:203-205).
-// 15 KB per warp at 2048 slots: five warps per CTA, three CTAs per SM.
+// 15 KB per warp at 2048 slots: five warps per CTA, three CTAs per SM.  Sizes
+// above 20 take 4096 slots (29 KB, seven warps per SM): at n = 24 5 % of random
+// automata pass 3072 subsets, 25 % would pass 1536.
 // The warp expands 32 subsets of the current level per step (level-
 // synchronous, as GPGPU/CPU/SlimCPUUntweaked.cs:119-184), tests the images
 // against the set (atomicCAS insert), and appends the new ones compacted by
@@ -23,7 +28,7 @@
 // slots or kHashLevelCap levels is tried backwards by the same warp
 // (inverse_search below), which settles the slowly synchronizing families and
 // the automata that never synchronize; what is left -- wide both ways -- goes
-// to the CTA-wide kernel through a list.  Random n = 17..20: 1.7 % of the
+// to the CTA-wide kernel (k_cta, or k_wide above n = 20) through a list.  Random n = 17..20: 1.7 % of the
 // automata pass 1536 subsets, 0.3 % pass 4096.  200K mixed n = 6..20 with 1 %
 // Cerny automata: 3.04 ms with every such automaton on the CTA-wide kernel,
 // 1.20 ms with the inverse search.
@@ -37,20 +42,23 @@ namespace {
 constexpr uint32_t kHashLevelCap = 48;         // random n <= 20: at most ~40 levels
 constexpr uint32_t kUnsettled = 1u << 31;
 
-template <int CAP_BITS>
+template <int CAP_BITS, int MAXN>
 struct HashGeom {
     static constexpr int kCap = 1 << CAP_BITS;                  // hash slots per warp
     static constexpr uint32_t kLimit = 3u * (1u << CAP_BITS) / 4u;   // subsets a warp keeps
-    static constexpr int kWarps = CAP_BITS <= 11 ? 5 : 2;        // warps per CTA (~75 KB)
-    static constexpr int kMaxN = 20;
+    // warps per CTA: 2048 slots 75 KB, three CTAs per SM; 4096 slots 29 KB, seven
+    static constexpr int kWarps = CAP_BITS <= 11 ? 5 : 1;
+    static constexpr int kMaxN = MAXN;
+    static constexpr int kChunks = (MAXN + 3) / 4;               // nibble tables
+    static constexpr int kEntries = 16 * kChunks;
     static constexpr uint32_t kSubsetMask = (1u << kMaxN) - 1u;
     static constexpr uint32_t kGens = 1u << (32 - kMaxN);        // generation 0 marks never-used slots
 };
 
-template <int CAP_BITS>
+template <int CAP_BITS, int MAXN>
 struct __align__(16) HashWarp {
-    using G = HashGeom<CAP_BITS>;
-    uint64_t table[5 * 16];
+    using G = HashGeom<CAP_BITS, MAXN>;
+    uint64_t table[G::kEntries];
     uint32_t set[G::kCap];
     uint16_t queue[G::kLimit];    // set slot | letter-is-b << 15
     uint16_t parent[G::kLimit];
@@ -64,15 +72,15 @@ __device__ __forceinline__ uint32_t hash_slot(uint32_t x)
 
 // Inserts subset x (generation gen); returns its slot when it was not yet in
 // the set, -1 otherwise.
-template <int CAP_BITS>
+template <int CAP_BITS, int MAXN>
 __device__ __forceinline__ int set_insert(uint32_t *set, uint32_t x, uint32_t gen)
 {
     constexpr int kCap = 1 << CAP_BITS;
-    const uint32_t key = x | (gen << 20);
+    const uint32_t key = x | (gen << MAXN);
     uint32_t p = hash_slot<CAP_BITS>(x);
     for (int probe = 0; probe < kCap; ++probe) {
         uint32_t v = set[p];
-        while ((v >> 20) != gen) {   // a slot of an earlier automaton: empty for this one
+        while ((v >> MAXN) != gen) {   // a slot of an earlier automaton: empty for this one
             const uint32_t prev = atomicCAS(&set[p], v, key);
             if (prev == v) return (int)p;
             v = prev;   // someone else took it: look at what is there now
@@ -83,41 +91,43 @@ __device__ __forceinline__ int set_insert(uint32_t *set, uint32_t x, uint32_t ge
     return -1;   // unreachable: the set is never more than ~3/4 full
 }
 
-// Entries of the five nibble tables from one 64-bit mask pair per state (lane q
-// holds state q's, a's mask << 32 | b's): 80 entries in three passes that every
-// lane takes (the shuffles need the whole warp), the third storing lanes 0..15
-// only.
-template <int CAP_BITS>
-__device__ __forceinline__ void build_table(HashWarp<CAP_BITS> &W, uint64_t mine, int n, int lane)
+// Entries of the nibble tables from one 64-bit mask pair per state (lane q
+// holds state q's, a's mask << 32 | b's), in passes of 32 that every lane takes
+// (the shuffles need the whole warp); a last half pass stores lanes 0..15 only.
+template <int CAP_BITS, int MAXN>
+__device__ __forceinline__ void build_table(HashWarp<CAP_BITS, MAXN> &W, uint64_t mine, int n, int lane)
 {
+    using G = HashGeom<CAP_BITS, MAXN>;
 #pragma unroll
-    for (int pass = 0; pass < 3; ++pass) {
+    for (int pass = 0; pass < (G::kEntries + 31) / 32; ++pass) {
         const int e = lane + 32 * pass;
-        const int c = min(e >> 4, 4), v = e & 15;
+        const int c = min(e >> 4, G::kChunks - 1), v = e & 15;
         uint64_t acc = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint64_t sj = __shfl_sync(kFull, mine, 4 * c + j);
             if (((v >> j) & 1) && 4 * c + j < n) acc |= sj;
         }
-        if (e < 5 * 16) W.table[e] = acc;
+        if (e < G::kEntries) W.table[e] = acc;
     }
 }
 
 // a's mask << 32 | b's mask of subset x
-template <int CAP_BITS>
-__device__ __forceinline__ uint64_t lookup(const HashWarp<CAP_BITS> &W, uint32_t x)
+template <int CAP_BITS, int MAXN>
+__device__ __forceinline__ uint64_t lookup(const HashWarp<CAP_BITS, MAXN> &W, uint32_t x)
 {
-    return W.table[x & 15u] | W.table[16 + ((x >> 4) & 15u)] | W.table[32 + ((x >> 8) & 15u)] |
-           W.table[48 + ((x >> 12) & 15u)] | W.table[64 + ((x >> 16) & 15u)];
+    uint64_t t = W.table[x & 15u];
+#pragma unroll
+    for (int c = 1; c < HashGeom<CAP_BITS, MAXN>::kChunks; ++c) t |= W.table[16 * c + ((x >> (4 * c)) & 15u)];
+    return t;
 }
 
 // The generation of the next search; the set is cleared when they wrap.
-template <int CAP_BITS>
-__device__ __forceinline__ void next_generation(HashWarp<CAP_BITS> &W, uint32_t &gen, int lane)
+template <int CAP_BITS, int MAXN>
+__device__ __forceinline__ void next_generation(HashWarp<CAP_BITS, MAXN> &W, uint32_t &gen, int lane)
 {
-    if (++gen == HashGeom<CAP_BITS>::kGens) {
-        for (int i = lane; i < HashGeom<CAP_BITS>::kCap; i += 32) W.set[i] = 0u;
+    if (++gen == HashGeom<CAP_BITS, MAXN>::kGens) {
+        for (int i = lane; i < HashGeom<CAP_BITS, MAXN>::kCap; i += 32) W.set[i] = 0u;
         gen = 1;
         __syncwarp();
     }
@@ -157,11 +167,11 @@ __device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t 
 // Takes a fresh generation; returns the sets this lane expanded, with the top
 // bit clear when the automaton is settled and set when it is left to the
 // CTA-wide kernel.
-template <int CAP_BITS>
+template <int CAP_BITS, int MAXN>
 __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n, uint32_t av, uint32_t bv,
-                                                HashWarp<CAP_BITS> &W, uint32_t gen, int lane)
+                                                HashWarp<CAP_BITS, MAXN> &W, uint32_t gen, int lane)
 {
-    using G = HashGeom<CAP_BITS>;
+    using G = HashGeom<CAP_BITS, MAXN>;
     uint32_t expanded = 0;
     const uint32_t full = (1u << n) - 1u;
     // lane q: the states that a (b) sends to q
@@ -171,9 +181,9 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
         const unsigned ib = __ballot_sync(kFull, lane < n && bv == (uint32_t)q);
         if (lane == q) inv = ((uint64_t)ia << 32) | ib;
     }
-    build_table<CAP_BITS>(W, inv, n, lane);
+    build_table<CAP_BITS, MAXN>(W, inv, n, lane);
     __syncwarp();
-    if (lane < n) W.queue[lane] = (uint16_t)set_insert<CAP_BITS>(W.set, 1u << lane, gen);
+    if (lane < n) W.queue[lane] = (uint16_t)set_insert<CAP_BITS, MAXN>(W.set, 1u << lane, gen);
     __syncwarp();
     uint32_t head = 0, lvl_end = (uint32_t)n, tail = lvl_end, level = 0;
     uint32_t found = 0, found_letter = 0;
@@ -183,7 +193,7 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
         const bool has = idx < lvl_end;
         uint32_t ya = 0, yb = 0;
         if (has) {
-            const uint64_t t = lookup<CAP_BITS>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
+            const uint64_t t = lookup<CAP_BITS, MAXN>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
             ya = (uint32_t)(t >> 32);
             yb = (uint32_t)t;
         }
@@ -196,8 +206,8 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
             hit = true;
             break;
         }
-        const int sa = ya ? set_insert<CAP_BITS>(W.set, ya, gen) : -1;
-        const int sb = yb ? set_insert<CAP_BITS>(W.set, yb, gen) : -1;
+        const int sa = ya ? set_insert<CAP_BITS, MAXN>(W.set, ya, gen) : -1;
+        const int sb = yb ? set_insert<CAP_BITS, MAXN>(W.set, yb, gen) : -1;
         bool fa = sa >= 0, fb = sb >= 0;
         const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
         const uint32_t added = (uint32_t)(__popc(ma) + __popc(mb));
@@ -254,7 +264,7 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
         while (true) {
             const uint32_t ra = __shfl_sync(kFull, row, (int)av), rb = __shfl_sync(kFull, row, (int)bv);
             const uint32_t grown =
-                row | (uint32_t)(lookup<CAP_BITS>(W, ra) >> 32) | (uint32_t)lookup<CAP_BITS>(W, rb);
+                row | (uint32_t)(lookup<CAP_BITS, MAXN>(W, ra) >> 32) | (uint32_t)lookup<CAP_BITS, MAXN>(W, rb);
             const bool more = lane < n && grown != row;
             if (lane < n) row = grown;
             if (!__any_sync(kFull, more)) break;
@@ -266,17 +276,17 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
     return expanded;
 }
 
-template <int CAP_BITS>
-__global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
+template <int CAP_BITS, int MAXN>
+__global__ void __launch_bounds__(HashGeom<CAP_BITS, MAXN>::kWarps * 32)
     k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count, unsigned long long *ticket)
 {
-    using G = HashGeom<CAP_BITS>;
+    using G = HashGeom<CAP_BITS, MAXN>;
     constexpr int kHashCap = G::kCap;
     constexpr uint32_t kHashLimit = G::kLimit;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    HashWarp<CAP_BITS> &W = reinterpret_cast<HashWarp<CAP_BITS> *>(smem_raw)[warp];
+    HashWarp<CAP_BITS, MAXN> &W = reinterpret_cast<HashWarp<CAP_BITS, MAXN> *>(smem_raw)[warp];
     int64_t count;
     const int32_t *order;
     resolve_work(b, count, order);
@@ -315,10 +325,10 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
             }
             continue;
         }
-        build_table<CAP_BITS>(W, single, n, lane);
-        next_generation<CAP_BITS>(W, gen, lane);
+        build_table<CAP_BITS, MAXN>(W, single, n, lane);
+        next_generation<CAP_BITS, MAXN>(W, gen, lane);
         const uint32_t full = (1u << n) - 1u;
-        if (lane == 0) W.queue[0] = (uint16_t)set_insert<CAP_BITS>(W.set, full, gen);
+        if (lane == 0) W.queue[0] = (uint16_t)set_insert<CAP_BITS, MAXN>(W.set, full, gen);
         __syncwarp();
         // n = 1: the visited root is the only singleton, the search generates nothing new
         uint32_t head = 0, lvl_end = n > 1 ? 1u : 0u, tail = lvl_end, level = 0;
@@ -330,7 +340,7 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
             const bool has = idx < lvl_end;
             uint32_t ya = 0, yb = 0;
             if (has) {
-                const uint64_t t = lookup<CAP_BITS>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
+                const uint64_t t = lookup<CAP_BITS, MAXN>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
                 ya = (uint32_t)(t >> 32);
                 yb = (uint32_t)t;
             }
@@ -345,8 +355,8 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
                 len = (int32_t)level + 1;
                 break;
             }
-            const int sa_slot = has ? set_insert<CAP_BITS>(W.set, ya, gen) : -1;
-            const int sb_slot = has ? set_insert<CAP_BITS>(W.set, yb, gen) : -1;
+            const int sa_slot = has ? set_insert<CAP_BITS, MAXN>(W.set, ya, gen) : -1;
+            const int sb_slot = has ? set_insert<CAP_BITS, MAXN>(W.set, yb, gen) : -1;
             bool fa = sa_slot >= 0, fb = sb_slot >= 0;
             const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
             const uint32_t added = (uint32_t)(__popc(ma) + __popc(mb));
@@ -380,8 +390,8 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS>::kWarps * 32)
         if (heavy) {
             // a long or wide search: backwards from the singletons, and if that is
             // wide too the CTA-wide kernel takes it from the start
-            next_generation<CAP_BITS>(W, gen, lane);
-            const uint32_t r = inverse_search<CAP_BITS>(b, k, n, av, bv, W, gen, lane);
+            next_generation<CAP_BITS, MAXN>(W, gen, lane);
+            const uint32_t r = inverse_search<CAP_BITS, MAXN>(b, k, n, av, bv, W, gen, lane);
             expanded += r & ~kUnsettled;
             if ((r & kUnsettled) && lane == 0) heavy_list[atomicAdd(heavy_count, 1ull)] = (int32_t)k;
             __syncwarp();
@@ -470,9 +480,9 @@ int current_device()
 
 // The shared-memory cap and the resident CTAs per SM are set and measured once
 // per device: the enqueue paths ask on every launch.
-template <int CAP_BITS>
+template <int CAP_BITS, int MAXN>
 struct HashLaunch {
-    static size_t smem() { return (size_t)HashGeom<CAP_BITS>::kWarps * sizeof(HashWarp<CAP_BITS>); }
+    static size_t smem() { return (size_t)HashGeom<CAP_BITS, MAXN>::kWarps * sizeof(HashWarp<CAP_BITS, MAXN>); }
     static cudaError_t prepare()
     {
         static std::atomic<int> done[kMaxDevices];
@@ -480,7 +490,7 @@ struct HashLaunch {
         const bool cached = dev >= 0 && dev < kMaxDevices;
         if (cached && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
         const cudaError_t e =
-            cudaFuncSetAttribute(k_hash<CAP_BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
+            cudaFuncSetAttribute(k_hash<CAP_BITS, MAXN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
         if (e == cudaSuccess && cached) done[dev].store(1, std::memory_order_release);
         return e;
     }
@@ -498,7 +508,7 @@ struct HashLaunch {
             return 0;
         }
         int blocks = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_hash<CAP_BITS>, HashGeom<CAP_BITS>::kWarps * 32,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_hash<CAP_BITS, MAXN>, HashGeom<CAP_BITS, MAXN>::kWarps * 32,
                                                           smem()) != cudaSuccess) {
             cudaGetLastError();
             return 0;
@@ -511,17 +521,20 @@ struct HashLaunch {
     {
         cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
-        k_hash<CAP_BITS><<<ctas, HashGeom<CAP_BITS>::kWarps * 32, smem(), st>>>(b, list, count, ticket);
+        k_hash<CAP_BITS, MAXN><<<ctas, HashGeom<CAP_BITS, MAXN>::kWarps * 32, smem(), st>>>(b, list, count, ticket);
         return cudaGetLastError();
     }
 };
 
 }  // namespace
 
-// size 1: 2048 hash slots per warp (1536 subsets), size 2: 4096 (3072 subsets)
-int hash_max_ctas_per_sm(int size)
+// size 1: 2048 hash slots per warp (1536 subsets), size 2: 4096 (3072 subsets);
+// max_n: the largest n of the launch's automata (more than 20 states: size 2 only)
+int hash_max_ctas_per_sm(int size, int max_n)
 {
-    return size == 2 ? HashLaunch<12>::per_sm() : size == 1 ? HashLaunch<11>::per_sm() : 0;
+    if (max_n > 20) return size == 2 ? HashLaunch<12, 28>::per_sm() : 0;
+    if (max_n > 16) return size == 2 ? HashLaunch<12, 20>::per_sm() : size == 1 ? HashLaunch<11, 20>::per_sm() : 0;
+    return size == 2 ? HashLaunch<12, 16>::per_sm() : size == 1 ? HashLaunch<11, 16>::per_sm() : 0;
 }
 
 cudaError_t launch_sort_handoff(const Batch &b, const int32_t *list, const unsigned long long *count, int32_t *out,
@@ -531,12 +544,20 @@ cudaError_t launch_sort_handoff(const Batch &b, const int32_t *list, const unsig
     return cudaGetLastError();
 }
 
-cudaError_t launch_hash(int size, int ctas, const Batch &b, int32_t *heavy_list, unsigned long long *heavy_count,
-                        unsigned long long *ticket, cudaStream_t st)
+cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
+                        unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st)
 {
-    if (ctas < 1 || !heavy_list || !heavy_count) return cudaErrorInvalidValue;
-    if (size == 1) return HashLaunch<11>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
-    if (size == 2) return HashLaunch<12>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+    if (ctas < 1 || !heavy_list || !heavy_count || max_n > SBFS_MAX_N) return cudaErrorInvalidValue;
+    if (max_n > 20)
+        return size == 2 ? HashLaunch<12, 28>::launch(ctas, b, heavy_list, heavy_count, ticket, st)
+                         : cudaErrorInvalidValue;
+    if (max_n > 16) {
+        if (size == 1) return HashLaunch<11, 20>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+        if (size == 2) return HashLaunch<12, 20>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+        return cudaErrorInvalidValue;
+    }
+    if (size == 1) return HashLaunch<11, 16>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+    if (size == 2) return HashLaunch<12, 16>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
     return cudaErrorInvalidValue;
 }
 

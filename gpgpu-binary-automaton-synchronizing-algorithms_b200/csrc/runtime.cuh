@@ -30,10 +30,13 @@ struct DevCounters {
     // escalation list, and claims on it
     unsigned long long escal_count[2];
     unsigned long long escal_claim[2];
-    // classes 0..3 (pooled warps, hash-set warps): automata handed to the
-    // CTA-wide kernel, as {offset 0, count} work ranges, and that kernel's tickets
-    unsigned long long heavy_range[4][2];
-    unsigned long long heavy_ticket[4];
+    // per class (pooled warps, hash-set warps): automata handed to the CTA-wide
+    // kernel (class 4: to k_wide), as {offset 0, count} work ranges, and that
+    // kernel's tickets
+    unsigned long long heavy_range[kNumClasses][2];
+    unsigned long long heavy_ticket[kNumClasses];
+    // class 4: automata k_wide leaves to the level slots
+    unsigned long long wide_range[2];
     // class 3's sorted hand-offs as two work ranges (n = top, n < top) and the
     // second launch's tickets
     unsigned long long heavy_split[4][4];
@@ -100,7 +103,7 @@ struct Lane {
     cudaStream_t aux[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr};
     DevBuf spill_c[3];                         // queue spill of a pooled class, one per class
-    DevBuf heavy[4], heavy_queue[4];           // a class's long searches and their CTA queues
+    DevBuf heavy[kNumClasses], heavy_queue[4]; // a class's long searches and their CTA queues
     DevBuf maps, ns, len, words, spill, order, counters, ranges, cta_queue, hbm_bitmap, hbm_queue,
         escal, tickets;
     LevelEngine level;                         // device-resident slots for n > 20
@@ -129,7 +132,7 @@ struct Lane {
         uint64_t x = 1469598103934665603ull;
         for (const DevBuf *d : {&maps, &ns, &len, &words, &spill, &order, &counters, &ranges, &cta_queue, &escal,
                                 &tickets, &spill_c[0], &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2],
-                                &heavy[3], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3]})
+                                &heavy[3], &heavy[4], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3]})
             x = (x ^ reinterpret_cast<uint64_t>(d->ptr)) * 1099511628211ull;
         for (const HostBuf *b : {&h_counters, &h_maps, &h_ns, &h_len, &h_words})
             x = (x ^ reinterpret_cast<uint64_t>(b->ptr)) * 1099511628211ull;

@@ -47,7 +47,7 @@ def slow_batch(n):
     return np.stack(rows + list(P.uniform_maps(64, n, 5)))
 
 
-@pytest.mark.parametrize("n", [13, 15, 16, 17, 18, 20])
+@pytest.mark.parametrize("n", [13, 15, 16, 17, 18, 20, 21])
 def test_slow_families(engine, oracle_mod, n):
     recs = slow_batch(n)
     # n = 13 and 14 take the per-lane kernel as uniform batches: one member of another size
@@ -72,3 +72,33 @@ def test_generations_wrap_between_searches(engine, oracle_mod):
     recs = np.concatenate([recs] * 160)          # 12,800 automata
     ref = oracle_mod.solve(recs[:80], n=n, words=False, threads=8)["len"]
     np.testing.assert_array_equal(engine.solve(recs, n=n)["len"], np.tile(ref, 160))
+
+
+def test_largest_slow_automaton_and_words(engine, oracle_mod):
+    """C_28: 729 letters in twelve 64-bit words; a word array too narrow for them is left zero."""
+    n = 28
+    recs = np.stack([P.cerny_record(n), _cycle_merge(n, 0, n - 1), P.uniform_maps(1, n, 2)[0]])
+    r = engine.solve(recs, n=n)
+    assert r["len"][0] == (n - 1) ** 2
+    assert oracle_mod.replay(recs, r["len"], r["words"], n=n)[0] == 0
+    short = engine.solve(recs, n=n, word_stride=2)
+    np.testing.assert_array_equal(short["len"], r["len"])
+    assert not short["words"][0].any()
+
+
+@pytest.mark.parametrize("n", [22, 24])
+def test_wide_large_automata(engine, oracle_mod, n):
+    """Random automata past a warp's set (3072 subsets), and two-permutation
+    automata past a CTA's (24,576), beside slow and malformed ones."""
+    rows = [_two_permutations(n, s) for s in range(2)] + [_two_components(n, 7)]
+    recs = np.concatenate([np.stack(rows), P.uniform_maps(400, n, 77)])
+    ns = np.full(len(recs), n, dtype=np.uint8)
+    ns[-1] = 9                                   # mixed sizes: the members come from the bucketing
+    recs[-1] = P.uniform_maps(1, 9, 3)[0]
+    ref = oracle_mod.solve(recs, ns=ns, words=False, threads=8)
+    r = engine.solve(recs, ns=ns)
+    np.testing.assert_array_equal(r["len"], ref["len"])
+    assert oracle_mod.replay(recs, r["len"], r["words"], ns=ns)[0] == 0
+    np.testing.assert_array_equal(engine.solve(recs[:-1], n=n, words=False)["len"], ref["len"][:-1])
+    # lengths that nobody asked for still count for the violation index
+    assert engine.verify(recs, ns=ns, lengths=False)["first_violation"] == -1
