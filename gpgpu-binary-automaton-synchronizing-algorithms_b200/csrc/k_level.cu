@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(kThreads) k_level(LevelSlot *slots, uint64_t *
     for (int q = 0; q < n_init; ++q) {
         const int s = ctl->init_list[q];
         LevelSlot &sl = slots[s];
+        if (sl.state != kSlotInit) continue;   // settled on chip (no CTA of this launch has moved on yet)
         const size_t words4 = sl.n >= 7 ? ((size_t)1 << sl.n) / 128 : 1;
         uint4 *bm4 = reinterpret_cast<uint4 *>(sl.bitmap);
         for (size_t w = gtid; w < words4; w += gthreads) bm4[w] = make_uint4(0u, 0u, 0u, 0u);
@@ -469,7 +470,25 @@ __global__ void __cluster_dims__(kNarrowCluster, 1, 1) __launch_bounds__(kThread
     }
 }
 
+__global__ void k_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n)
+{
+    const int i = threadIdx.x;
+    if (i >= n || t->len[i] == kLenUntried) return;
+    LevelSlot &sl = slots[ctl->init_list[i]];
+    sl.result_len = t->len[i];
+    for (int c = 0; c < kLevelWordU64; ++c) sl.word[c] = t->words[i * kLevelWordU64 + c];
+    sl.state = kSlotDone;
+    atomicAdd(&ctl->finished, 1u);
+}
+
 }  // namespace
+
+cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, cudaStream_t st)
+{
+    if (n < 1 || n > kMaxLevelSlots) return cudaErrorInvalidValue;
+    k_level_settle<<<1, kMaxLevelSlots, 0, st>>>(slots, ctl, t, n);
+    return cudaGetLastError();
+}
 
 int level_max_ctas_per_sm()
 {

@@ -18,6 +18,8 @@ constexpr int kLevelTable = 4 * 256;          // byte tables, entry = a-image <<
 constexpr int kLevelWordU64 = 12;             // 768 bits >= (28-1)^2
 constexpr uint64_t kLevelSubsetMask = 0x0FFFFFFFull;
 
+constexpr int32_t kLenUntried = (int32_t)0x80808080;   // what a cudaMemset of 0x80 leaves
+
 constexpr int kSlotFree = 0, kSlotInit = 1, kSlotRun = 2, kSlotDone = 3, kSlotFail = 4;
 
 struct LevelSlot {
@@ -56,7 +58,24 @@ struct LevelCtl {
     int init_list[kMaxLevelSlots];
 };
 
+// Device and pinned buffers of the on-chip try of freshly admitted slots.
+struct LevelTry {
+    static constexpr int kRec = 64;                  // a[32] | b[32]
+    uint8_t recs[kMaxLevelSlots * kRec];
+    uint8_t ns[kMaxLevelSlots];
+    // device only
+    int32_t len[kMaxLevelSlots];
+    int32_t list[2][kMaxLevelSlots];                 // left by k_hash, left by k_wide
+    uint64_t words[kMaxLevelSlots * kLevelWordU64];
+    unsigned long long ticket[2], range[2][2];       // zeroed before every try
+    unsigned long long first_violation, expanded;
+    int error, pad;
+};
+
 int level_max_ctas_per_sm();
+// Ends the slots init_list[0..n) whose automaton the on-chip kernels settled
+// (t->len[i] is not kLenUntried).
+cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, cudaStream_t st);
 cudaError_t launch_level(int ctas, int parity, LevelSlot *slots, uint64_t *tables, LevelCtl *ctl, const Batch &out,
                          cudaStream_t st);
 cudaError_t launch_level_narrow(int parity, int max_levels, unsigned long long narrow, LevelSlot *slots,
@@ -98,6 +117,12 @@ public:
     void destroy();
     // bytes an automaton with n states needs (bitmap + full-size queue), 256-aligned
     static size_t footprint(int n);
+    // From now on freshly admitted slots (with host maps) are first tried on chip,
+    // one warp and then one CTA each (k_hash.cu, k_wide.cu), in the launch that
+    // admits them; only what is wider than that runs level by level.
+    cudaError_t try_on_chip();
+    // admitted slots that a past launch has not settled: their levels are still to run
+    int running() const { return in_flight_ - (int)pending_init_.size(); }
     // admit one automaton whose record is at d_rec (device); returns slot or -1 (no slot/memory)
     int admit(const uint8_t *d_rec, int lstride, int n, long long tag, const uint8_t *host_a,
               const uint8_t *host_b);
@@ -107,6 +132,7 @@ public:
     // states back
     // (async); results go to `out` when out.out_len is set (batch mode)
     cudaError_t launch(int levels, const Batch &out, int narrow_levels = 0);
+    cudaError_t launch_try(int n);
     // wait for the last launch and collect finished slots (frees their memory)
     struct Finished {
         long long tag;
@@ -148,6 +174,9 @@ private:
     LevelSlot *h_slots_ = nullptr;   // pinned mirror
     LevelCtl *h_ctl_ = nullptr;      // pinned mirror
     int *h_init_ = nullptr;          // pinned: nslots, n_init, init_list[]
+    LevelTry *d_try_ = nullptr;      // set by try_on_chip
+    LevelTry *h_try_ = nullptr;      // pinned: recs and ns
+    int sm_count_ = 0;
     Arena own_;
     Arena *shared_ = nullptr;
     Arena &arena() { return shared_ ? *shared_ : own_; }

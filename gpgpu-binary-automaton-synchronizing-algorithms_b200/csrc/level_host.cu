@@ -1,12 +1,19 @@
 // level_host.cu -- host engine of the device-resident level slots (k_level.cu):
 // a first-fit arena for bitmaps and queues, admission into free slots, level
 // launches and collection of finished automata.
+#include <algorithm>
 #include <climits>
 #include <cstring>
 
 #include "level.cuh"
 
 namespace sbfs {
+
+int hash_max_ctas_per_sm(int size, int max_n);
+cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
+                        unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st);
+cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
+                        unsigned long long *ticket, cudaStream_t st);
 
 cudaError_t Arena::reserve(size_t bytes)
 {
@@ -86,6 +93,7 @@ cudaError_t LevelEngine::init(int sm_count, size_t arena_bytes, cudaStream_t st,
 {
     st_ = st;
     shared_ = shared;
+    sm_count_ = sm_count;
     cudaError_t e;
     const int per_sm = level_max_ctas_per_sm();
     ctas_ = (per_sm > 0 ? per_sm : 1) * sm_count;
@@ -120,8 +128,12 @@ void LevelEngine::destroy()
     if (h_slots_) cudaFreeHost(h_slots_);
     if (h_ctl_) cudaFreeHost(h_ctl_);
     if (h_init_) cudaFreeHost(h_init_);
+    if (d_try_) cudaFree(d_try_);
+    if (h_try_) cudaFreeHost(h_try_);
     if (ev_) cudaEventDestroy(ev_);
     own_.release();
+    d_try_ = nullptr;
+    h_try_ = nullptr;
     d_slots_ = nullptr;
     d_tables_ = nullptr;
     d_ctl_ = nullptr;
@@ -129,6 +141,59 @@ void LevelEngine::destroy()
     h_ctl_ = nullptr;
     h_init_ = nullptr;
     ev_ = nullptr;
+}
+
+cudaError_t LevelEngine::try_on_chip()
+{
+    cudaError_t e = cudaHostAlloc(&h_try_, sizeof(LevelTry), cudaHostAllocDefault);
+    if (e != cudaSuccess) {
+        h_try_ = nullptr;
+        return e;
+    }
+    if ((e = cudaMalloc(&d_try_, sizeof(LevelTry))) != cudaSuccess) d_try_ = nullptr;
+    return e;
+}
+
+// The freshly admitted slots h_init_[2..2+n) through the on-chip kernels, then
+// the settled ones to Done.  Everything on st_, behind the slots' upload.
+cudaError_t LevelEngine::launch_try(int n)
+{
+    cudaError_t e;
+    for (int i = 0; i < n; ++i) {
+        const LevelSlot &sl = h_slots_[h_init_[2 + i]];
+        std::memcpy(h_try_->recs + i * LevelTry::kRec, sl.a, 32);
+        std::memcpy(h_try_->recs + i * LevelTry::kRec + 32, sl.b, 32);
+        h_try_->ns[i] = (uint8_t)sl.n;
+    }
+    if ((e = cudaMemcpyAsync(d_try_->recs, h_try_->recs, (size_t)n * LevelTry::kRec, cudaMemcpyHostToDevice, st_)) !=
+        cudaSuccess)
+        return e;
+    if ((e = cudaMemcpyAsync(d_try_->ns, h_try_->ns, (size_t)n, cudaMemcpyHostToDevice, st_)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(d_try_->len, 0x80, sizeof(int32_t) * (size_t)n, st_)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(d_try_->ticket, 0, sizeof(d_try_->ticket) + sizeof(d_try_->range), st_)) != cudaSuccess)
+        return e;
+    Batch b{};
+    b.maps = d_try_->recs;
+    b.lstride = LevelTry::kRec / 2;
+    b.ns = d_try_->ns;
+    b.count = n;
+    b.out_len = d_try_->len;
+    b.out_words = d_try_->words;
+    b.word_stride = kLevelWordU64;
+    b.first_violation = &d_try_->first_violation;
+    b.expanded = &d_try_->expanded;
+    b.error = &d_try_->error;
+    const int per_sm = hash_max_ctas_per_sm(2, SBFS_MAX_N);
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    if ((e = launch_hash(2, SBFS_MAX_N, std::min(n, per_sm * sm_count_), b, d_try_->list[0], &d_try_->range[0][1],
+                         &d_try_->ticket[0], st_)) != cudaSuccess)
+        return e;
+    b.order = d_try_->list[0];
+    b.range_dev = d_try_->range[0];
+    if ((e = launch_wide(std::min(n, sm_count_), b, d_try_->list[1], &d_try_->range[1][1], &d_try_->ticket[1], st_)) !=
+        cudaSuccess)
+        return e;
+    return launch_level_settle(d_slots_, d_ctl_, d_try_, n, st_);
 }
 
 int LevelEngine::admit(const uint8_t *d_rec, int lstride, int n, long long tag, const uint8_t *host_a,
@@ -174,9 +239,13 @@ cudaError_t LevelEngine::launch(int levels, const Batch &out, int narrow_levels)
     const bool narrow = narrow_levels > 0 && pending_init_.empty() && launches_ > 0 &&
                         h_ctl_->total[parity_ & 1] <= kNarrowLevel;
     // admissions: descriptors of the new slots, then the control block's init list
-    for (int s : pending_init_) {
-        if ((e = cudaMemcpyAsync(d_slots_ + s, h_slots_ + s, sizeof(LevelSlot), cudaMemcpyHostToDevice, st_)) !=
-            cudaSuccess)
+    if (!pending_init_.empty()) {
+        // in one copy from the first to the last of them: the mirror of the slots
+        // between is what the last launch left on the device
+        const auto mm = std::minmax_element(pending_init_.begin(), pending_init_.end());
+        if ((e = cudaMemcpyAsync(d_slots_ + *mm.first, h_slots_ + *mm.first,
+                                 sizeof(LevelSlot) * (size_t)(*mm.second - *mm.first + 1), cudaMemcpyHostToDevice,
+                                 st_)) != cudaSuccess)
             return e;
     }
     // nslots, this launch parity's n_init and init_list are host-owned
@@ -194,6 +263,7 @@ cudaError_t LevelEngine::launch(int levels, const Batch &out, int narrow_levels)
     if (n_init && (e = cudaMemcpyAsync(d_ctl_->init_list, h_init_ + 2, sizeof(int) * n_init,
                                        cudaMemcpyHostToDevice, st_)) != cudaSuccess)
         return e;
+    if (n_init && d_try_ && (e = launch_try(n_init)) != cudaSuccess) return e;
     if (narrow) {
         if ((e = launch_level_narrow((int)(parity_ & 1), narrow_levels, kNarrowLevel, d_slots_, d_tables_, d_ctl_, out,
                                      st_)) != cudaSuccess)

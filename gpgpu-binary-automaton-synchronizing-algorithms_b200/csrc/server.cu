@@ -428,13 +428,16 @@ void run_loop(sbfs_server *s)
                 s->pend_big.pop_front();
             }
             if (E.in_flight() > 0) {
-                const cudaError_t ce = E.launch(s->cfg.max_levels, none, 4 * s->cfg.max_levels);
+                // new requests alone need one level launch, which sets up the few that
+                // the on-chip kernels before it leave
+                const int levels = E.running() > 0 ? s->cfg.max_levels : 1;
+                const cudaError_t ce = E.launch(levels, none, 4 * s->cfg.max_levels);
                 if (ce != cudaSuccess) {
                     cudaGetLastError();
                     fail_all(s, SBFS_ECUDA, std::string("serving level launch: ") + cudaGetErrorString(ce));
                 } else {
                     std::lock_guard<std::mutex> lock(s->mu);
-                    s->st.level_launches += s->cfg.max_levels;
+                    s->st.level_launches += levels;
                 }
                 progress = true;
             }
@@ -522,6 +525,7 @@ sbfs_status sbfs_server_start(const sbfs_server_config *cfg, sbfs_server **out)
     }
     if (e == cudaSuccess && (e = s->arena.reserve((size_t)s->cfg.arena_bytes)) == cudaSuccess)
         e = s->big.init(s->h->sm_count, 0, s->h->lanes[kSmallSlots].stream, &s->arena);
+    if (e == cudaSuccess) e = s->big.try_on_chip();
     if (e == cudaSuccess) e = prime_small(s);
     if (e != cudaSuccess) {
         cudaGetLastError();
