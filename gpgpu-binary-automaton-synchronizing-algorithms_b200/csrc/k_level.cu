@@ -318,7 +318,6 @@ __global__ void __launch_bounds__(kThreads) k_level(LevelSlot *slots, uint64_t *
     for (int q = 0; q < n_init; ++q) {
         const int s = ctl->init_list[q];
         LevelSlot &sl = slots[s];
-        if (sl.state != kSlotInit) continue;   // settled on chip (no CTA of this launch has moved on yet)
         const size_t words4 = sl.n >= 7 ? ((size_t)1 << sl.n) / 128 : 1;
         uint4 *bm4 = reinterpret_cast<uint4 *>(sl.bitmap);
         for (size_t w = gtid; w < words4; w += gthreads) bm4[w] = make_uint4(0u, 0u, 0u, 0u);
@@ -470,23 +469,36 @@ __global__ void __cluster_dims__(kNarrowCluster, 1, 1) __launch_bounds__(kThread
     }
 }
 
-__global__ void k_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n)
+// One thread per fresh slot.  The slots still to be set up move to the front of
+// init_list: each one costs k_level's CTAs two dependent loads before the next.
+__global__ void __launch_bounds__(kMaxLevelSlots) k_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t,
+                                                                 int n, int par)
 {
+    __shared__ int left;
     const int i = threadIdx.x;
-    if (i >= n || t->len[i] == kLenUntried) return;
-    LevelSlot &sl = slots[ctl->init_list[i]];
-    sl.result_len = t->len[i];
-    for (int c = 0; c < kLevelWordU64; ++c) sl.word[c] = t->words[i * kLevelWordU64 + c];
-    sl.state = kSlotDone;
-    atomicAdd(&ctl->finished, 1u);
+    if (i == 0) left = 0;
+    const int s = i < n ? ctl->init_list[i] : -1;
+    const bool settled = i < n && t->len[i] != kLenUntried;
+    __syncthreads();
+    if (settled) {
+        LevelSlot &sl = slots[s];
+        sl.result_len = t->len[i];
+        for (int c = 0; c < kLevelWordU64; ++c) sl.word[c] = t->words[i * kLevelWordU64 + c];
+        sl.state = kSlotDone;
+        atomicAdd(&ctl->finished, 1u);
+    } else if (i < n) {
+        ctl->init_list[atomicAdd(&left, 1)] = s;
+    }
+    __syncthreads();
+    if (i == 0) ctl->n_init[par] = left;
 }
 
 }  // namespace
 
-cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, cudaStream_t st)
+cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, int par, cudaStream_t st)
 {
     if (n < 1 || n > kMaxLevelSlots) return cudaErrorInvalidValue;
-    k_level_settle<<<1, kMaxLevelSlots, 0, st>>>(slots, ctl, t, n);
+    k_level_settle<<<1, kMaxLevelSlots, 0, st>>>(slots, ctl, t, n, par & 1);
     return cudaGetLastError();
 }
 

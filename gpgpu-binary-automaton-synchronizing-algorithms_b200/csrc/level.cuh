@@ -74,8 +74,9 @@ struct LevelTry {
 
 int level_max_ctas_per_sm();
 // Ends the slots init_list[0..n) whose automaton the on-chip kernels settled
-// (t->len[i] is not kLenUntried).
-cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, cudaStream_t st);
+// (t->len[i] is not kLenUntried) and takes them off the list that the launch of
+// parity `par` sets up.
+cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, int par, cudaStream_t st);
 cudaError_t launch_level(int ctas, int parity, LevelSlot *slots, uint64_t *tables, LevelCtl *ctl, const Batch &out,
                          cudaStream_t st);
 cudaError_t launch_level_narrow(int parity, int max_levels, unsigned long long narrow, LevelSlot *slots,

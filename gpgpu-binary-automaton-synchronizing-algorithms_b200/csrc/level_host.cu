@@ -193,7 +193,7 @@ cudaError_t LevelEngine::launch_try(int n)
     if ((e = launch_wide(std::min(n, sm_count_), b, d_try_->list[1], &d_try_->range[1][1], &d_try_->ticket[1], st_)) !=
         cudaSuccess)
         return e;
-    return launch_level_settle(d_slots_, d_ctl_, d_try_, n, st_);
+    return launch_level_settle(d_slots_, d_ctl_, d_try_, n, (int)(parity_ & 1), st_);
 }
 
 int LevelEngine::admit(const uint8_t *d_rec, int lstride, int n, long long tag, const uint8_t *host_a,
