@@ -1,37 +1,41 @@
 // k_hash.cu -- power-set BFS of automata with 13..28 states (size classes 2,
-// 3 and 4) with one warp per automaton and an open-addressed hash set as the
-// visited store.
+// 3 and 4), one warp per automaton with its visited store, queue and image
+// tables in shared memory.
 //
 // A random automaton of 13..20 states is settled after a few hundred subsets
 // over ~11 levels (its shortest word is at most ~36 letters), so neither a
 // 2^n-bit bitmap (128 KiB at n = 20) nor a 1024-thread CTA (k_cta.cu) pays for
-// itself: the CTA's per-level barriers and round trips dominate.  Here each
-// warp keeps in shared memory
+// itself: the CTA's per-level barriers and round trips dominate.  Per warp:
 //   * nibble tables: table[c][v] = (a-image << 32) | b-image of the states
 //     4c..4c+3 selected by v, so both images of a subset are 4, 5 or 7 loads
-//     (instances for n <= 16, 20 and 28: four instead of five at n = 16 is
-//     1.124 -> 1.120 ms per 200K automata);
-//   * a hash set of 2^CAP_BITS slots, each holding subset | generation << MAXN;
-//     the generation changes with every search, so a slot from an earlier one
-//     reads as empty and the set is cleared when the generations (2^(32 - MAXN))
-//     wrap;
-//   * a level-ordered queue of 16-bit entries, set slot | letter-is-b << 15
-//     (a slot keeps its subset for the whole search), with a 16-bit parent
-//     index per entry, retained for the word (GPGPU/CPU/CPU.cs:203-205).
-// 15 KB per warp at 2048 slots: five warps per CTA, three CTAs per SM.  Sizes
-// above 20 take 4096 slots (29 KB, seven warps per SM): at n = 24 5 % of random
-// automata pass 3072 subsets, 25 % would pass 1536.
+//     (instances for n <= 16, 20 and 28);
+//   * the visited store, 4 KB (n <= 16) or 8 KB.  After the first letter every
+//     subset lies in the image of a or of b, so with the states relabelled by
+//     image 2^rank(a) + 2^rank(b) bits tell them apart (ranks average 0.64 n):
+//     a bitmap, one atomicOr per image.  95 % of random n = 20 and nearly all
+//     smaller ones fit; the rest use the store as an open-addressed hash set,
+//     atomicCAS with linear probing, to three quarters full.  With the hash set
+//     for every automaton, whose 32 probe loops a step waits for, 200K n = 16
+//     took 1.120 ms against 0.499 ms, 30K n = 20 0.602 against 0.329 ms;
+//   * a level-ordered queue, retained for the word (GPGPU/CPU/CPU.cs:203-205):
+//     subset, parent index and letter in 32 bits (a separate parent array
+//     where they do not fit).
+// 10.5 KB per warp for n <= 16 (21 warps per SM), 14.6 KB for n <= 20 (15).
+// Sizes above 20 keep 3072 subsets and a 16 KB store (6 warps per SM): at
+// n = 24 5 % of random automata pass that, 25 % would pass 1536.
 // The warp expands 32 subsets of the current level per step (level-
 // synchronous, as GPGPU/CPU/SlimCPUUntweaked.cs:119-184), tests the images
-// against the set (atomicCAS insert), and appends the new ones compacted by
-// ballots in queue order.  An automaton that needs more than 3/4 of the set's
-// slots or kHashLevelCap levels is tried backwards by the same warp
-// (inverse_search below), which settles the slowly synchronizing families and
-// the automata that never synchronize; what is left -- wide both ways -- goes
-// to the CTA-wide kernel (k_cta, or k_wide above n = 20) through a list.  Random n = 17..20: 1.7 % of the
-// automata pass 1536 subsets, 0.3 % pass 4096.  200K mixed n = 6..20 with 1 %
-// Cerny automata: 3.04 ms with every such automaton on the CTA-wide kernel,
-// 1.20 ms with the inverse search.
+// against the store, and appends the new ones compacted by ballots in queue
+// order.  An automaton that needs more than 1536 subsets (or kHashLevelCap
+// levels) is tried backwards by the same warp (inverse_search below), which
+// settles the slowly synchronizing families and the automata that never
+// synchronize; one with a permutation letter and a letter merging at most one
+// pair is tried backwards at once.  What is left -- wide both ways -- goes to
+// the CTA-wide kernel (k_cta, or k_wide above n = 20) through a list.  Random
+// n = 17..20: 1.7 % of the automata pass 1536 subsets, 0.3 % pass 4096.
+// 200K mixed n = 6..20 with 1 % Cerny automata: 3.04 ms with every such
+// automaton on the CTA-wide kernel, 1.17 ms with the inverse search, 0.67 ms
+// with the bitmap store.
 #include <atomic>
 
 #include "common.cuh"
@@ -42,95 +46,113 @@ namespace {
 constexpr uint32_t kHashLevelCap = 48;         // random n <= 20: at most ~40 levels
 constexpr uint32_t kUnsettled = 1u << 31;
 
-template <int CAP_BITS, int MAXN>
+// SIZE 1: 1536 subsets per warp, SIZE 2: 3072.
+template <int MAXN, int SIZE>
 struct HashGeom {
-    static constexpr int kCap = 1 << CAP_BITS;                  // hash slots per warp
-    static constexpr uint32_t kLimit = 3u * (1u << CAP_BITS) / 4u;   // subsets a warp keeps
-    // warps per CTA: 2048 slots 75 KB, three CTAs per SM; 4096 slots 29 KB, seven
-    static constexpr int kWarps = CAP_BITS <= 11 ? 5 : 1;
-    static constexpr int kMaxN = MAXN;
+    static constexpr uint32_t kLimit = 1536u << (SIZE - 1);      // subsets a warp keeps
+    static constexpr int kIdxBits = 10 + SIZE;                   // of a queue index
+    // words of the visited store: 2^15 bits for n <= 16, 2^16 for n <= 20 (twice that at SIZE 2)
+    static constexpr int kWords = (MAXN <= 16 ? 1024 : 2048) << (SIZE - 1);
+    static constexpr uint32_t kBits = 32u * kWords;
+    // as a hash set it is filled to three quarters
+    static constexpr uint32_t kSetLimit = kLimit < 3u * kWords / 4u ? kLimit : 3u * kWords / 4u;
+    static constexpr int kSetShift = 32 - (MAXN <= 16 ? 9 : 10) - SIZE;
+    // a queue entry is subset | parent << MAXN | letter-is-b << 31; sizes that
+    // leave no room for the parent keep it in an array of its own
+    static constexpr bool kPacked = MAXN + kIdxBits + 1 <= 32;
     static constexpr int kChunks = (MAXN + 3) / 4;               // nibble tables
     static constexpr int kEntries = 16 * kChunks;
-    static constexpr uint32_t kSubsetMask = (1u << kMaxN) - 1u;
-    static constexpr uint32_t kGens = 1u << (32 - kMaxN);        // generation 0 marks never-used slots
+    static constexpr uint32_t kMask = (1u << MAXN) - 1u;
+    // warps per CTA: n <= 16 10.5 KB, three CTAs of seven per SM; n <= 20 14.6 KB,
+    // three of five; SIZE 2 single
+    static constexpr int kWarps = SIZE == 2 ? 1 : MAXN <= 16 ? 7 : 5;
 };
 
-template <int CAP_BITS, int MAXN>
+template <int MAXN, int SIZE>
 struct __align__(16) HashWarp {
-    using G = HashGeom<CAP_BITS, MAXN>;
+    using G = HashGeom<MAXN, SIZE>;
+    uint32_t store[G::kWords];    // visited: bitmap or hash set (0 = free slot)
     uint64_t table[G::kEntries];
-    uint32_t set[G::kCap];
-    uint16_t queue[G::kLimit];    // set slot | letter-is-b << 15
-    uint16_t parent[G::kLimit];
+    uint32_t queue[G::kLimit];
+    uint16_t parent[G::kPacked ? 2 : G::kLimit];
+
+    __device__ __forceinline__ uint32_t subset(uint32_t i) const { return queue[i] & G::kMask; }
+    __device__ __forceinline__ uint32_t letter(uint32_t i) const { return queue[i] >> 31; }
+    __device__ __forceinline__ uint32_t parent_of(uint32_t i) const
+    {
+        return G::kPacked ? (queue[i] >> MAXN) & ((1u << G::kIdxBits) - 1u) : parent[i];
+    }
+    __device__ __forceinline__ void push(uint32_t i, uint32_t x, uint32_t par, uint32_t letter)
+    {
+        if (G::kPacked) {
+            queue[i] = x | (par << (MAXN < 32 ? MAXN : 0)) | (letter << 31);
+        } else {
+            queue[i] = x | (letter << 31);
+            parent[i] = (uint16_t)par;
+        }
+    }
 };
 
-template <int CAP_BITS>
-__device__ __forceinline__ uint32_t hash_slot(uint32_t x)
+// Inserts subset x into the store as a hash set; false when it was there.
+template <int MAXN, int SIZE>
+__device__ __forceinline__ bool set_insert(HashWarp<MAXN, SIZE> &W, uint32_t x)
 {
-    return (x * 0x9E3779B1u) >> (32 - CAP_BITS);
-}
-
-// Inserts subset x (generation gen); returns its slot when it was not yet in
-// the set, -1 otherwise.
-template <int CAP_BITS, int MAXN>
-__device__ __forceinline__ int set_insert(uint32_t *set, uint32_t x, uint32_t gen)
-{
-    constexpr int kCap = 1 << CAP_BITS;
-    const uint32_t key = x | (gen << MAXN);
-    uint32_t p = hash_slot<CAP_BITS>(x);
-    for (int probe = 0; probe < kCap; ++probe) {
-        uint32_t v = set[p];
-        while ((v >> MAXN) != gen) {   // a slot of an earlier automaton: empty for this one
-            const uint32_t prev = atomicCAS(&set[p], v, key);
-            if (prev == v) return (int)p;
-            v = prev;   // someone else took it: look at what is there now
+    using G = HashGeom<MAXN, SIZE>;
+    uint32_t p = (x * 0x9E3779B1u) >> G::kSetShift;
+    for (int probe = 0; probe < G::kWords; ++probe) {
+        uint32_t v = W.store[p];
+        if (v == 0u) {
+            v = atomicCAS(&W.store[p], 0u, x);
+            if (v == 0u) return true;
         }
-        if (v == key) return -1;
-        p = (p + 1) & (kCap - 1);
+        if (v == x) return false;
+        p = (p + 1) & (G::kWords - 1);
     }
-    return -1;   // unreachable: the set is never more than ~3/4 full
+    return false;   // unreachable: the set is never more than ~3/4 full
 }
 
-// Entries of the nibble tables from one 64-bit mask pair per state (lane q
-// holds state q's, a's mask << 32 | b's), in passes of 32 that every lane takes
-// (the shuffles need the whole warp); a last half pass stores lanes 0..15 only.
-template <int CAP_BITS, int MAXN>
-__device__ __forceinline__ void build_table(HashWarp<CAP_BITS, MAXN> &W, uint64_t mine, int n, int lane)
+// Zeroes the store's first `bits` bits (rounded up to 128).
+template <int MAXN, int SIZE>
+__device__ __forceinline__ void clear_store(HashWarp<MAXN, SIZE> &W, uint32_t bits, int lane)
 {
-    using G = HashGeom<CAP_BITS, MAXN>;
+    uint4 *s = reinterpret_cast<uint4 *>(W.store);
+    for (uint32_t i = lane; i < (bits + 127u) / 128u; i += 32) s[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Nibble tables of one 64-bit mask pair per state (a's mask << 32 | b's): lane
+// q < 32 passes state `label`'s, zero for labels past the last state.  The
+// store serves as the staging area.
+template <int MAXN, int SIZE>
+__device__ __forceinline__ void build_table(HashWarp<MAXN, SIZE> &W, uint64_t mine, int label, int lane)
+{
+    using G = HashGeom<MAXN, SIZE>;
+    uint64_t *stage = reinterpret_cast<uint64_t *>(W.store);
+    __syncwarp();
+    stage[label] = mine;
+    __syncwarp();
 #pragma unroll
     for (int pass = 0; pass < (G::kEntries + 31) / 32; ++pass) {
         const int e = lane + 32 * pass;
-        const int c = min(e >> 4, G::kChunks - 1), v = e & 15;
-        uint64_t acc = 0;
+        const int c = e >> 4, v = e & 15;
+        if (e < G::kEntries) {
+            uint64_t acc = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint64_t sj = __shfl_sync(kFull, mine, 4 * c + j);
-            if (((v >> j) & 1) && 4 * c + j < n) acc |= sj;
+            for (int j = 0; j < 4; ++j)
+                if ((v >> j) & 1) acc |= stage[4 * c + j];
+            W.table[e] = acc;
         }
-        if (e < G::kEntries) W.table[e] = acc;
     }
+    __syncwarp();
 }
 
 // a's mask << 32 | b's mask of subset x
-template <int CAP_BITS, int MAXN>
-__device__ __forceinline__ uint64_t lookup(const HashWarp<CAP_BITS, MAXN> &W, uint32_t x)
+template <int MAXN, int SIZE>
+__device__ __forceinline__ uint64_t lookup(const HashWarp<MAXN, SIZE> &W, uint32_t x)
 {
     uint64_t t = W.table[x & 15u];
 #pragma unroll
-    for (int c = 1; c < HashGeom<CAP_BITS, MAXN>::kChunks; ++c) t |= W.table[16 * c + ((x >> (4 * c)) & 15u)];
+    for (int c = 1; c < HashGeom<MAXN, SIZE>::kChunks; ++c) t |= W.table[16 * c + ((x >> (4 * c)) & 15u)];
     return t;
-}
-
-// The generation of the next search; the set is cleared when they wrap.
-template <int CAP_BITS, int MAXN>
-__device__ __forceinline__ void next_generation(HashWarp<CAP_BITS, MAXN> &W, uint32_t &gen, int lane)
-{
-    if (++gen == HashGeom<CAP_BITS, MAXN>::kGens) {
-        for (int i = lane; i < HashGeom<CAP_BITS, MAXN>::kCap; i += 32) W.set[i] = 0u;
-        gen = 1;
-        __syncwarp();
-    }
 }
 
 __device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t k, int n)
@@ -141,13 +163,13 @@ __device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t 
     publish_result(b, k);
 }
 
-// The inverse search, for an automaton that the forward search gave up on
-// (lane q < n holds a(q) and b(q)).  A word w synchronizes iff w^-1(q) is the
-// full set for some state q, and (cw)^-1(q) = c^-1(w^-1(q)): so a breadth-first
-// search from the n singletons along preimages reaches the full set first at
-// the length of the shortest word, and the parent chain from there spells the
-// word from its first letter on.  It runs out without the full set iff the
-// automaton is not synchronizing.
+// The inverse search, for an automaton that the forward search gave up on, or
+// that looks slow (lane q < n holds a(q) and b(q)).  A word w synchronizes iff
+// w^-1(q) is the full set for some state q, and (cw)^-1(q) = c^-1(w^-1(q)): so a
+// breadth-first search from the n singletons along preimages reaches the full
+// set first at the length of the shortest word, and the parent chain from there
+// spells the word from its first letter on.  It runs out without the full set
+// iff the automaton is not synchronizing.
 //
 // The slowly synchronizing families (Cerny automata, a permutation plus one
 // merge) have up to 2^n images of the full set but at most n(n-1)+1 preimages
@@ -156,22 +178,25 @@ __device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t 
 // 1.2 ms).  Their levels hold 1 to n sets; a random automaton whose forward
 // search is wide passes n sets in a level at its fifth or sixth (9,000 random
 // n = 13..28 with over 1536 images: none was settled before that).  So the
-// search stops at the first level wider than n sets, which also keeps every
-// level within one step of the warp.
+// search stops at the first level wider than n sets.
+//
+// Hundreds of levels of one or two sets are a serial chain, so a level keeps
+// its sets in registers (lane i: set i) and gives every image a lane of its own
+// -- one hash probe per lane and level.  Sets reach the next level by shuffle
+// when there is one, through the queue otherwise.
 //
 // Before giving up, pairs of states settle the wide automata that never
 // synchronize: an automaton synchronizes iff every pair of its states is merged
 // by some word.  Row q (lane q) collects the states that can be merged with q,
 // preimages of the rows of a(q) and b(q), until nothing changes.
 //
-// Takes a fresh generation; returns the sets this lane expanded, with the top
-// bit clear when the automaton is settled and set when it is left to the
-// CTA-wide kernel.
-template <int CAP_BITS, int MAXN>
+// Returns the images this lane looked up, with the top bit clear when the
+// automaton is settled and set when it is left to the forward searches.
+template <int MAXN, int SIZE>
 __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n, uint32_t av, uint32_t bv,
-                                                HashWarp<CAP_BITS, MAXN> &W, uint32_t gen, int lane)
+                                                HashWarp<MAXN, SIZE> &W, int lane)
 {
-    using G = HashGeom<CAP_BITS, MAXN>;
+    using G = HashGeom<MAXN, SIZE>;
     uint32_t expanded = 0;
     const uint32_t full = (1u << n) - 1u;
     // lane q: the states that a (b) sends to q
@@ -181,59 +206,62 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
         const unsigned ib = __ballot_sync(kFull, lane < n && bv == (uint32_t)q);
         if (lane == q) inv = ((uint64_t)ia << 32) | ib;
     }
-    build_table<CAP_BITS, MAXN>(W, inv, n, lane);
+    build_table(W, inv, lane, lane);
+    clear_store(W, G::kBits, lane);
     __syncwarp();
-    if (lane < n) W.queue[lane] = (uint16_t)set_insert<CAP_BITS, MAXN>(W.set, 1u << lane, gen);
+    uint32_t front = lane < n ? 1u << lane : 0u;   // set `lane` of the level
+    if (front) {
+        set_insert(W, front);
+        W.push((uint32_t)lane, front, 0u, 0u);
+    }
     __syncwarp();
-    uint32_t head = 0, lvl_end = (uint32_t)n, tail = lvl_end, level = 0;
+    uint32_t head = 0, width = (uint32_t)n, tail = width, level = 0;
     uint32_t found = 0, found_letter = 0;
     bool hit = false, spent = true;   // spent: no set left to expand
-    while (head < lvl_end) {
-        const uint32_t idx = head + (uint32_t)lane;
-        const bool has = idx < lvl_end;
-        uint32_t ya = 0, yb = 0;
-        if (has) {
-            const uint64_t t = lookup<CAP_BITS, MAXN>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
-            ya = (uint32_t)(t >> 32);
-            yb = (uint32_t)t;
+    const uint32_t letter = (uint32_t)lane & 1u;
+    while (true) {
+        // image j of the level is letter j & 1 of set j >> 1: 32 images per pass, at most two passes
+        uint32_t added = 0, next = 0;
+        for (uint32_t base = 0; base < 2u * width; base += 32) {
+            const uint32_t set = (base + (uint32_t)lane) >> 1;
+            const uint32_t x = __shfl_sync(kFull, front, (int)set);
+            uint32_t y = 0;
+            if (set < width) {
+                const uint64_t t = lookup(W, x);
+                y = letter ? (uint32_t)t : (uint32_t)(t >> 32);
+            }
+            expanded += set < width ? 1u : 0u;
+            const unsigned hits = __ballot_sync(kFull, y == full);
+            if (hits) {
+                const int fl = __ffs(hits) - 1;
+                found = head + ((base + (uint32_t)fl) >> 1);
+                found_letter = (uint32_t)fl & 1u;
+                hit = true;
+                break;
+            }
+            const bool fresh = y && set_insert(W, y);
+            const unsigned m = __ballot_sync(kFull, fresh);
+            if (m) {
+                const uint32_t p = tail + added + (uint32_t)__popc(m & ((1u << lane) - 1u));
+                if (fresh && p < G::kSetLimit) W.push(p, y, head + set, letter);
+                if (!(m & (m - 1u))) next = __shfl_sync(kFull, y, __ffs(m) - 1);
+                added += (uint32_t)__popc(m);
+            }
         }
-        expanded += has ? 1u : 0u;
-        const unsigned hits = __ballot_sync(kFull, ya == full || yb == full);
-        if (hits) {
-            const int fl = __ffs(hits) - 1;
-            found = head + (uint32_t)fl;
-            found_letter = (uint32_t)__shfl_sync(kFull, ya == full ? 0 : 1, fl);
-            hit = true;
-            break;
-        }
-        const int sa = ya ? set_insert<CAP_BITS, MAXN>(W.set, ya, gen) : -1;
-        const int sb = yb ? set_insert<CAP_BITS, MAXN>(W.set, yb, gen) : -1;
-        bool fa = sa >= 0, fb = sb >= 0;
-        const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
-        const uint32_t added = (uint32_t)(__popc(ma) + __popc(mb));
-        if (tail + added > min(G::kLimit, lvl_end + (uint32_t)n)) {
+        if (hit || added == 0) break;
+        if (added > (uint32_t)n || tail + added > G::kSetLimit) {
             spent = false;
             break;
         }
-        const unsigned lt = (1u << lane) - 1u;
-        uint32_t p = tail + (uint32_t)(__popc(ma & lt) + __popc(mb & lt));
-        if (!SBFS_CHECK(p + (fa ? 1u : 0u) + (fb ? 1u : 0u) <= G::kLimit, b.error)) fa = fb = false;
-        if (fa) {
-            W.queue[p] = (uint16_t)sa;
-            W.parent[p++] = (uint16_t)idx;
-        }
-        if (fb) {
-            W.queue[p] = (uint16_t)(sb | 0x8000);
-            W.parent[p] = (uint16_t)idx;
-        }
+        __syncwarp();
+        front = added == 1 ? next : lane < (int)added ? W.subset(tail + (uint32_t)lane) : 0u;
+        head = tail;
         tail += added;
-        head = lvl_end;   // a level is one step: at most n sets
-        lvl_end = tail;
-        __syncwarp();
-        if (head < lvl_end) ++level;
+        width = added;
+        ++level;
     }
+    __syncwarp();
     if (hit) {
-        __syncwarp();
         if (lane == 0) {
             record_result(b, k, n, (int32_t)level + 1);
             if (b.out_words) {
@@ -247,8 +275,8 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
                             w[c++] = acc;
                             acc = 0ull;
                         }
-                        acc |= (uint64_t)(W.queue[i] >> 15) << (d & 63u);
-                        i = W.parent[i];
+                        acc |= (uint64_t)W.letter(i) << (d & 63u);
+                        i = W.parent_of(i);
                     }
                     w[c++] = acc;
                 }
@@ -263,8 +291,7 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
         uint32_t row = lane < n ? 1u << lane : 0u;
         while (true) {
             const uint32_t ra = __shfl_sync(kFull, row, (int)av), rb = __shfl_sync(kFull, row, (int)bv);
-            const uint32_t grown =
-                row | (uint32_t)(lookup<CAP_BITS, MAXN>(W, ra) >> 32) | (uint32_t)lookup<CAP_BITS, MAXN>(W, rb);
+            const uint32_t grown = row | (uint32_t)(lookup(W, ra) >> 32) | (uint32_t)lookup(W, rb);
             const bool more = lane < n && grown != row;
             if (lane < n) row = grown;
             if (!__any_sync(kFull, more)) break;
@@ -276,24 +303,101 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
     return expanded;
 }
 
-template <int CAP_BITS, int MAXN>
-__global__ void __launch_bounds__(HashGeom<CAP_BITS, MAXN>::kWarps * 32)
-    k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count, unsigned long long *ticket)
+// What the forward search of one automaton ends with.
+struct Forward {
+    bool heavy;              // more subsets or levels than a warp keeps
+    int32_t len;
+    uint32_t level, found, found_letter;
+};
+
+// The warp expands 32 subsets of the current level per step.  BITS: the store
+// is a bitmap, subset y at bit y when y < 2^ra and at base + (y >> shift)
+// otherwise (a-images always are below 2^ra; see the kernel).
+template <int MAXN, int SIZE, bool BITS>
+__device__ __forceinline__ Forward forward_search(const Batch &b, int n, HashWarp<MAXN, SIZE> &W, uint32_t low_end,
+                                                  uint32_t base, uint32_t shift, int lane,
+                                                  unsigned long long &expanded)
 {
-    using G = HashGeom<CAP_BITS, MAXN>;
-    constexpr int kHashCap = G::kCap;
-    constexpr uint32_t kHashLimit = G::kLimit;
+    using G = HashGeom<MAXN, SIZE>;
+    constexpr uint32_t kKeep = BITS ? G::kLimit : G::kSetLimit;
+    Forward r{false, kLenNonSync, 0u, 0u, 0u};
+    // n = 1: the visited root is the only singleton, the search generates nothing new
+    uint32_t head = 0, lvl_end = n > 1 ? 1u : 0u, tail = lvl_end, level = 0;
+    const unsigned lt = (1u << lane) - 1u;
+    while (head < lvl_end) {
+        const uint32_t idx = head + (uint32_t)lane;
+        const bool has = idx < lvl_end;
+        uint32_t ya = 0, yb = 0;
+        if (has) {
+            const uint64_t t = lookup(W, W.subset(idx));
+            ya = (uint32_t)(t >> 32);
+            yb = (uint32_t)t;
+        }
+        expanded += has ? 1u : 0u;
+        const bool sa = has && is_singleton(ya), sb = has && is_singleton(yb);
+        const unsigned smask = __ballot_sync(kFull, sa || sb);
+        if (smask) {
+            // the first singleton in queue order (lowest lane, a before b)
+            const int fl = __ffs(smask) - 1;
+            r.found = head + (uint32_t)fl;
+            r.found_letter = (uint32_t)__shfl_sync(kFull, sa ? 0 : 1, fl);
+            r.len = (int32_t)level + 1;
+            break;
+        }
+        bool fa = false, fb = false;
+        if (has) {
+            if (BITS) {
+                const uint32_t ib = yb < low_end ? yb : base + (yb >> shift);
+                if (SBFS_CHECK(ya < G::kBits && ib < G::kBits, b.error)) {
+                    const uint32_t ma = 1u << (ya & 31u), mb = 1u << (ib & 31u);
+                    const uint32_t oa = atomicOr(&W.store[ya >> 5], ma);
+                    const uint32_t ob = atomicOr(&W.store[ib >> 5], mb);
+                    fa = !(oa & ma);
+                    fb = !(ob & mb);
+                }
+            } else {
+                fa = set_insert(W, ya);
+                fb = set_insert(W, yb);
+            }
+        }
+        const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
+        const uint32_t added = (uint32_t)(__popc(ma) + __popc(mb));
+        if (tail + added > kKeep) {
+            r.heavy = true;
+            break;
+        }
+        uint32_t p = tail + (uint32_t)(__popc(ma & lt) + __popc(mb & lt));
+        if (fa) W.push(p++, ya, idx, 0u);
+        if (fb) W.push(p, yb, idx, 1u);
+        tail += added;
+        head = min(head + 32u, lvl_end);
+        __syncwarp();
+        if (head == lvl_end && tail > lvl_end) {
+            lvl_end = tail;
+            if (++level >= kHashLevelCap) {
+                r.heavy = true;
+                break;
+            }
+        }
+    }
+    __syncwarp();
+    r.level = level;
+    return r;
+}
+
+template <int MAXN, int SIZE>
+__global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32)
+    k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count,
+           unsigned long long *ticket)
+{
+    using G = HashGeom<MAXN, SIZE>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    HashWarp<CAP_BITS, MAXN> &W = reinterpret_cast<HashWarp<CAP_BITS, MAXN> *>(smem_raw)[warp];
+    HashWarp<MAXN, SIZE> &W = reinterpret_cast<HashWarp<MAXN, SIZE> *>(smem_raw)[warp];
     int64_t count;
     const int32_t *order;
     resolve_work(b, count, order);
-    // generation 0 marks never-used slots; each automaton takes the next one
-    for (int i = lane; i < kHashCap; i += 32) W.set[i] = 0u;
-    __syncwarp();
-    uint32_t gen = 0;
     unsigned long long expanded = 0;
 
     while (true) {
@@ -304,16 +408,12 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS, MAXN>::kWarps * 32)
         const int64_t k = automaton_at(order, (int64_t)pos);
         const int n = automaton_n(b, k);
         const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
-        bool bad = n < 1 || n > G::kMaxN || n > b.lstride;
-        uint64_t single = 0;
+        bool bad = n < 1 || n > MAXN || n > b.lstride;
         uint32_t av = 0, bv = 0;
         if (!bad && lane < n) {
             av = rec[lane];
             bv = rec[b.lstride + lane];
-            if (av >= (uint32_t)n || bv >= (uint32_t)n)
-                bad = true;
-            else
-                single = ((uint64_t)(1u << av) << 32) | (1u << bv);
+            if (av >= (uint32_t)n || bv >= (uint32_t)n) bad = true;
         }
         if (__any_sync(kFull, bad)) {
             if (lane == 0) {
@@ -325,90 +425,78 @@ __global__ void __launch_bounds__(HashGeom<CAP_BITS, MAXN>::kWarps * 32)
             }
             continue;
         }
-        build_table<CAP_BITS, MAXN>(W, single, n, lane);
-        next_generation<CAP_BITS, MAXN>(W, gen, lane);
+        // New state labels, image of a first: A \ B | A and B | B \ A | the rest, with
+        // A = a's image and B = b's.  Every subset but the root lies in A or in B:
+        // as a label set it is below 2^ra, or a set of B, whose labels start at
+        // |A \ B|: shifted down by that it is below 2^rb.  So 2^ra + 2^rb bits tell
+        // all reachable subsets apart (n = 20: about 2^13.5 of 2^20, ranks
+        // averaging 12.8).
+        const uint32_t A = __reduce_or_sync(kFull, lane < n ? 1u << av : 0u);
+        const uint32_t B = __reduce_or_sync(kFull, lane < n ? 1u << bv : 0u);
+        const int ra = __popc(A), rb = __popc(B);
+        bool tried = false;
+        if (ra + rb >= 2 * n - 1 && n > 1) {
+            // a permutation and a letter that merges at most one pair: the slow
+            // families, whose forward search would be wide
+            const uint32_t r = inverse_search(b, k, n, av, bv, W, lane);
+            expanded += r & ~kUnsettled;
+            if (!(r & kUnsettled)) continue;
+            tried = true;
+        }
+        const uint32_t below = (1u << lane) - 1u;
+        const bool in_a = (A >> lane) & 1u, in_b = (B >> lane) & 1u;
+        int label = in_a ? (in_b ? __popc(A & ~B) + __popc(A & B & below) : __popc(A & ~B & below))
+                         : (in_b ? ra + __popc(B & ~A & below) : __popc(A | B) + __popc(~(A | B) & below));
+        if (lane >= n) label = lane;
+        const int la = __shfl_sync(kFull, label, (int)av), lb = __shfl_sync(kFull, label, (int)bv);
+        build_table(W, lane < n ? ((uint64_t)(1u << la) << 32) | (1u << lb) : 0ull, label, lane);
         const uint32_t full = (1u << n) - 1u;
-        if (lane == 0) W.queue[0] = (uint16_t)set_insert<CAP_BITS, MAXN>(W.set, full, gen);
+        uint32_t low_end = 1u << ra, base = low_end, shift = (uint32_t)__popc(A & ~B);
+        uint32_t bits = (B & ~A) ? low_end + (1u << rb) : low_end;
+        if (bits > 1u << n) {   // a full-rank b beside a smaller a: the plain index is shorter
+            base = shift = 0u;
+            bits = 1u << n;
+        }
+        const bool fits = bits <= G::kBits;
+        clear_store(W, fits ? bits : G::kBits, lane);
         __syncwarp();
-        // n = 1: the visited root is the only singleton, the search generates nothing new
-        uint32_t head = 0, lvl_end = n > 1 ? 1u : 0u, tail = lvl_end, level = 0;
-        int32_t len = kLenNonSync;
-        uint32_t found = 0, found_letter = 0;
-        bool heavy = false;
-        while (head < lvl_end) {
-            const uint32_t idx = head + (uint32_t)lane;
-            const bool has = idx < lvl_end;
-            uint32_t ya = 0, yb = 0;
-            if (has) {
-                const uint64_t t = lookup<CAP_BITS, MAXN>(W, W.set[W.queue[idx] & 0x7FFFu] & G::kSubsetMask);
-                ya = (uint32_t)(t >> 32);
-                yb = (uint32_t)t;
-            }
-            expanded += has ? 1u : 0u;
-            const bool sa = has && is_singleton(ya), sb = has && is_singleton(yb);
-            const unsigned smask = __ballot_sync(kFull, sa || sb);
-            if (smask) {
-                // the first singleton in queue order (lowest lane, a before b)
-                const int fl = __ffs(smask) - 1;
-                found = head + (uint32_t)fl;
-                found_letter = (uint32_t)__shfl_sync(kFull, sa ? 0 : 1, fl);
-                len = (int32_t)level + 1;
-                break;
-            }
-            const int sa_slot = has ? set_insert<CAP_BITS, MAXN>(W.set, ya, gen) : -1;
-            const int sb_slot = has ? set_insert<CAP_BITS, MAXN>(W.set, yb, gen) : -1;
-            bool fa = sa_slot >= 0, fb = sb_slot >= 0;
-            const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
-            const uint32_t added = (uint32_t)(__popc(ma) + __popc(mb));
-            if (tail + added > kHashLimit) {
-                heavy = true;
-                break;
-            }
-            const unsigned lt = (1u << lane) - 1u;
-            uint32_t p = tail + (uint32_t)(__popc(ma & lt) + __popc(mb & lt));
-            if (!SBFS_CHECK(p + (fa ? 1u : 0u) + (fb ? 1u : 0u) <= kHashLimit, b.error)) fa = fb = false;
-            if (fa) {
-                W.queue[p] = (uint16_t)sa_slot;
-                W.parent[p++] = (uint16_t)idx;
-            }
-            if (fb) {
-                W.queue[p] = (uint16_t)(sb_slot | 0x8000);
-                W.parent[p] = (uint16_t)idx;
-            }
-            tail += added;
-            head = min(head + 32u, lvl_end);
-            __syncwarp();
-            if (head == lvl_end && tail > lvl_end) {
-                lvl_end = tail;
-                if (++level >= kHashLevelCap) {
-                    heavy = true;
-                    break;
-                }
+        if (lane == 0) {
+            W.push(0u, full, 0u, 0u);
+            // the root comes back only through a permutation
+            if (!fits) {
+                set_insert(W, full);
+            } else if (ra == n || rb == n) {
+                const uint32_t i = full < low_end ? full : base + (full >> shift);
+                W.store[i >> 5] = 1u << (i & 31u);
             }
         }
         __syncwarp();
-        if (heavy) {
+        const Forward f = fits ? forward_search<MAXN, SIZE, true>(b, n, W, low_end, base, shift, lane, expanded)
+                               : forward_search<MAXN, SIZE, false>(b, n, W, 0u, 0u, 0u, lane, expanded);
+        if (f.heavy) {
             // a long or wide search: backwards from the singletons, and if that is
             // wide too the CTA-wide kernel takes it from the start
-            next_generation<CAP_BITS, MAXN>(W, gen, lane);
-            const uint32_t r = inverse_search<CAP_BITS, MAXN>(b, k, n, av, bv, W, gen, lane);
-            expanded += r & ~kUnsettled;
+            uint32_t r = kUnsettled;
+            if (!tried) {
+                r = inverse_search(b, k, n, av, bv, W, lane);
+                expanded += r & ~kUnsettled;
+            }
             if ((r & kUnsettled) && lane == 0) heavy_list[atomicAdd(heavy_count, 1ull)] = (int32_t)k;
             __syncwarp();
             continue;
         }
         if (lane == 0) {
-            record_result(b, k, n, len);
+            record_result(b, k, n, f.len);
             if (b.out_words) {
                 // letters from the root: the entry at depth d + 1 holds letter d
                 // (a word here has at most kHashLevelCap <= 64 letters)
                 uint64_t w0 = 0;
-                if (len > 0) {
-                    if (found_letter) w0 |= 1ull << level;
-                    uint32_t i = found;
-                    for (int d = (int)level - 1; d >= 0; --d) {
-                        if (W.queue[i] >> 15) w0 |= 1ull << d;
-                        i = W.parent[i];
+                if (f.len > 0) {
+                    if (f.found_letter) w0 |= 1ull << f.level;
+                    uint32_t i = f.found;
+                    for (int d = (int)f.level - 1; d >= 0; --d) {
+                        w0 |= (uint64_t)W.letter(i) << d;
+                        i = W.parent_of(i);
                     }
                 }
                 uint64_t *w = b.out_words + (size_t)k * (size_t)b.word_stride;
@@ -480,9 +568,9 @@ int current_device()
 
 // The shared-memory cap and the resident CTAs per SM are set and measured once
 // per device: the enqueue paths ask on every launch.
-template <int CAP_BITS, int MAXN>
+template <int MAXN, int SIZE>
 struct HashLaunch {
-    static size_t smem() { return (size_t)HashGeom<CAP_BITS, MAXN>::kWarps * sizeof(HashWarp<CAP_BITS, MAXN>); }
+    static size_t smem() { return (size_t)HashGeom<MAXN, SIZE>::kWarps * sizeof(HashWarp<MAXN, SIZE>); }
     static cudaError_t prepare()
     {
         static std::atomic<int> done[kMaxDevices];
@@ -490,7 +578,7 @@ struct HashLaunch {
         const bool cached = dev >= 0 && dev < kMaxDevices;
         if (cached && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
         const cudaError_t e =
-            cudaFuncSetAttribute(k_hash<CAP_BITS, MAXN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
+            cudaFuncSetAttribute(k_hash<MAXN, SIZE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
         if (e == cudaSuccess && cached) done[dev].store(1, std::memory_order_release);
         return e;
     }
@@ -508,7 +596,7 @@ struct HashLaunch {
             return 0;
         }
         int blocks = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_hash<CAP_BITS, MAXN>, HashGeom<CAP_BITS, MAXN>::kWarps * 32,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_hash<MAXN, SIZE>, HashGeom<MAXN, SIZE>::kWarps * 32,
                                                           smem()) != cudaSuccess) {
             cudaGetLastError();
             return 0;
@@ -521,7 +609,7 @@ struct HashLaunch {
     {
         cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
-        k_hash<CAP_BITS, MAXN><<<ctas, HashGeom<CAP_BITS, MAXN>::kWarps * 32, smem(), st>>>(b, list, count, ticket);
+        k_hash<MAXN, SIZE><<<ctas, HashGeom<MAXN, SIZE>::kWarps * 32, smem(), st>>>(b, list, count, ticket);
         return cudaGetLastError();
     }
 };
@@ -532,9 +620,9 @@ struct HashLaunch {
 // max_n: the largest n of the launch's automata (more than 20 states: size 2 only)
 int hash_max_ctas_per_sm(int size, int max_n)
 {
-    if (max_n > 20) return size == 2 ? HashLaunch<12, 28>::per_sm() : 0;
-    if (max_n > 16) return size == 2 ? HashLaunch<12, 20>::per_sm() : size == 1 ? HashLaunch<11, 20>::per_sm() : 0;
-    return size == 2 ? HashLaunch<12, 16>::per_sm() : size == 1 ? HashLaunch<11, 16>::per_sm() : 0;
+    if (max_n > 20) return size == 2 ? HashLaunch<28, 2>::per_sm() : 0;
+    if (max_n > 16) return size == 2 ? HashLaunch<20, 2>::per_sm() : size == 1 ? HashLaunch<20, 1>::per_sm() : 0;
+    return size == 2 ? HashLaunch<16, 2>::per_sm() : size == 1 ? HashLaunch<16, 1>::per_sm() : 0;
 }
 
 cudaError_t launch_sort_handoff(const Batch &b, const int32_t *list, const unsigned long long *count, int32_t *out,
@@ -549,15 +637,15 @@ cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *
 {
     if (ctas < 1 || !heavy_list || !heavy_count || max_n > SBFS_MAX_N) return cudaErrorInvalidValue;
     if (max_n > 20)
-        return size == 2 ? HashLaunch<12, 28>::launch(ctas, b, heavy_list, heavy_count, ticket, st)
+        return size == 2 ? HashLaunch<28, 2>::launch(ctas, b, heavy_list, heavy_count, ticket, st)
                          : cudaErrorInvalidValue;
     if (max_n > 16) {
-        if (size == 1) return HashLaunch<11, 20>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
-        if (size == 2) return HashLaunch<12, 20>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+        if (size == 1) return HashLaunch<20, 1>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+        if (size == 2) return HashLaunch<20, 2>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
         return cudaErrorInvalidValue;
     }
-    if (size == 1) return HashLaunch<11, 16>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
-    if (size == 2) return HashLaunch<12, 16>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+    if (size == 1) return HashLaunch<16, 1>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+    if (size == 2) return HashLaunch<16, 2>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
     return cudaErrorInvalidValue;
 }
 
