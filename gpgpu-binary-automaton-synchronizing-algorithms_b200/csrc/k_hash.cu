@@ -66,6 +66,7 @@ struct HashGeom {
     // warps per CTA: n <= 16 10.5 KB, three CTAs of seven per SM; n <= 20 14.6 KB,
     // three of five; SIZE 2 single
     static constexpr int kWarps = SIZE == 2 ? 1 : MAXN <= 16 ? 7 : 5;
+    static constexpr int kCtas = SIZE == 2 ? 6 : 3;
 };
 
 template <int MAXN, int SIZE>
@@ -109,6 +110,22 @@ __device__ __forceinline__ bool set_insert(HashWarp<MAXN, SIZE> &W, uint32_t x)
         p = (p + 1) & (G::kWords - 1);
     }
     return false;   // unreachable: the set is never more than ~3/4 full
+}
+
+// The free slot where subset x would go, or -1 when it is in the set: every
+// lane of the warp looks up the same x.
+template <int MAXN, int SIZE>
+__device__ __forceinline__ int set_find(const HashWarp<MAXN, SIZE> &W, uint32_t x)
+{
+    using G = HashGeom<MAXN, SIZE>;
+    uint32_t p = (x * 0x9E3779B1u) >> G::kSetShift;
+    for (int probe = 0; probe < G::kWords; ++probe) {
+        const uint32_t v = W.store[p];
+        if (v == 0u) return (int)p;
+        if (v == x) return -1;
+        p = (p + 1) & (G::kWords - 1);
+    }
+    return -1;
 }
 
 // Zeroes the store's first `bits` bits (rounded up to 128).
@@ -180,10 +197,12 @@ __device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t 
 // n = 13..28 with over 1536 images: none was settled before that).  So the
 // search stops at the first level wider than n sets.
 //
-// Hundreds of levels of one or two sets are a serial chain, so a level keeps
-// its sets in registers (lane i: set i) and gives every image a lane of its own
-// -- one hash probe per lane and level.  Sets reach the next level by shuffle
-// when there is one, through the queue otherwise.
+// Hundreds of levels of one to n sets are a serial chain.  A level of one set
+// (every level of a Cerny automaton but the first) is run by all lanes alike on
+// the same set: both preimages and both hash probes in registers, no ballot,
+// shuffle or atomic on the way to the next level.  Wider levels keep set i in
+// lane i and give every image a lane of its own, one hash probe per lane.  C_28
+// (729 levels): 0.40 ms with every level on the lane-per-image form.
 //
 // Before giving up, pairs of states settle the wide automata that never
 // synchronize: an automaton synchronizes iff every pair of its states is merged
@@ -220,6 +239,48 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
     bool hit = false, spent = true;   // spent: no set left to expand
     const uint32_t letter = (uint32_t)lane & 1u;
     while (true) {
+        while (width == 1) {
+            const uint32_t x = __shfl_sync(kFull, front, 0);
+            const uint64_t t = lookup(W, x);
+            const uint32_t ya = (uint32_t)(t >> 32), yb = (uint32_t)t;
+            expanded += lane < 2 ? 1u : 0u;
+            if (ya == full || yb == full) {
+                found = head;
+                found_letter = ya == full ? 0u : 1u;
+                hit = true;
+                break;
+            }
+            const int pa = ya ? set_find(W, ya) : -1, pb = yb && yb != ya ? set_find(W, yb) : -1;
+            if (pa < 0 && pb < 0) {
+                width = 0;
+                break;
+            }
+            if (tail + 2u > G::kSetLimit) {
+                spent = false;
+                break;
+            }
+            const uint32_t both = pa >= 0 && pb >= 0 ? 1u : 0u;
+            if (pa == pb) {   // two new sets for one free slot
+                if (lane == 0) {
+                    set_insert(W, ya);
+                    set_insert(W, yb);
+                }
+            } else {
+                if (lane == 0 && pa >= 0) W.store[pa] = ya;
+                if (lane == 0 && pb >= 0) W.store[pb] = yb;
+            }
+            if (lane == 0) {
+                if (pa >= 0) W.push(tail, ya, head, 0u);
+                if (pb >= 0) W.push(tail + both, yb, head, 1u);
+            }
+            __syncwarp();
+            front = both ? (lane == 0 ? ya : lane == 1 ? yb : 0u) : pa >= 0 ? ya : yb;
+            head = tail;
+            width = 1u + both;
+            tail += width;
+            ++level;
+        }
+        if (hit || !spent || width == 0) break;
         // image j of the level is letter j & 1 of set j >> 1: 32 images per pass, at most two passes
         uint32_t added = 0, next = 0;
         for (uint32_t base = 0; base < 2u * width; base += 32) {
@@ -386,7 +447,7 @@ __device__ __forceinline__ Forward forward_search(const Batch &b, int n, HashWar
 }
 
 template <int MAXN, int SIZE>
-__global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32)
+__global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32, HashGeom<MAXN, SIZE>::kCtas)
     k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count,
            unsigned long long *ticket)
 {
