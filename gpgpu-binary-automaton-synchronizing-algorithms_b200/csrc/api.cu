@@ -489,27 +489,27 @@ sbfs_status ensure_plan(sbfs_handle *h)
     for (int c = 0; c < 2; ++c) {
         LaneShape &ls = P.lane[c];
         ls.nmax = kClassMaxN[c];
-        ls.warps = h->cfg.lane_warps > 0 ? h->cfg.lane_warps : lane_defaults[c][0];
         ls.ring = h->cfg.lane_ring > 0 ? h->cfg.lane_ring : lane_defaults[c][1];
+        ls.warps = h->cfg.lane_warps > 0 ? h->cfg.lane_warps : lane_defaults[c][0];
         ls.refill_k = h->cfg.lane_refill > 0 ? h->cfg.lane_refill : lane_defaults[c][2];
         ls.tail_k = h->cfg.lane_tail > 0 ? std::min(h->cfg.lane_tail, 32) : h->cfg.lane_tail < 0 ? 0 : lane_defaults[c][3];
         if (lane_max_ctas_per_sm(ls.nmax, ls.warps, ls.ring) < 1) {
-            ls.warps = lane_defaults[c][0];
             ls.ring = lane_defaults[c][1];
+            ls.warps = lane_defaults[c][0];
         }
         const int per_sm = lane_max_ctas_per_sm(ls.nmax, ls.warps, ls.ring);
         if (per_sm < 1) return fail(h, SBFS_EINVAL, "per-lane kernel shape does not fit in shared memory");
         ls.ctas = per_sm * sms;
     }
     {
-        // uniform n = 13: 1 KB of bitmap per lane and a 128-entry ring, four
-        // one-warp CTAs per SM.  2^21 automata: ring 32 3.47 ms, 64 2.48 ms,
-        // 128 2.03 ms, 256 2.60 ms, 512 3.84 ms -- a small ring escalates more
+        // uniform n = 13: a 128-entry ring, six one-warp CTAs per SM.  2^21
+        // automata with a 1 KB bitmap per lane: ring 32 3.47 ms, 64 2.48 ms, 128
+        // 2.03 ms, 256 2.60 ms, 512 3.84 ms -- a small ring escalates more
         // searches to the whole-warp path, a large one costs resident warps
         LaneShape &ls = P.lane13;
         ls.nmax = 13;
-        ls.warps = 1;
         ls.ring = 128;
+        ls.warps = 1;
         ls.refill_k = 16;
         ls.tail_k = 4;
         const int per_sm = lane_max_ctas_per_sm(13, ls.warps, ls.ring);
@@ -517,13 +517,13 @@ sbfs_status ensure_plan(sbfs_handle *h)
         P.use_lane13 = per_sm > 0 && h->cfg.small_kernel != 2 ? 1 : 0;
     }
     {
-        // uniform n = 14: 2 KB of bitmap per lane and a 256-entry ring, two
-        // one-warp CTAs per SM.  2^21 automata: 4.83 ms (k_hash: 7.80 ms; ring
-        // 128: 5.19 ms; ring 512, one CTA per SM: 9.48 ms)
+        // uniform n = 14: a 256-entry ring, three one-warp CTAs per SM.  2^21
+        // automata with a 2 KB bitmap per lane: 4.83 ms (ring 128: 5.19 ms; ring
+        // 512, one CTA per SM: 9.48 ms)
         LaneShape &ls = P.lane14;
         ls.nmax = 14;
-        ls.warps = 1;
         ls.ring = 256;
+        ls.warps = 1;
         ls.refill_k = 16;
         ls.tail_k = 4;
         const int per_sm = lane_max_ctas_per_sm(14, ls.warps, ls.ring);
@@ -913,7 +913,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
             return fail(h, SBFS_ETIMEOUT, "streamed solve: no progress for 600 s");
         std::this_thread::yield();
     }
-    CK(cudaEventSynchronize(S.ev_kdone), "waiting for the kernel");
+    if (next < nch) CK(cudaEventSynchronize(S.ev_kdone), "waiting for the kernel");
     for (; next < nch; ++next)
         if ((st = copy_chunk_out(next))) return st;
     // escalated automata finish after their chunk may have been copied: store
@@ -926,20 +926,23 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     if (mapped && dst_words && cudaHostGetDevicePointer((void **)&map_words, dst_words, 0) != cudaSuccess)
         mapped = false;
     cudaGetLastError();
+    mapped &= out_len || out_words;
+    if (mapped) {
+        // behind the kernel and the last chunk's copy, without a trip to the host
+        CK(cudaStreamWaitEvent(S.copy_out, L.ev_k1, 0), "ordering streams");
+        CK(launch_escal_patch(S.escal_out.as<EscalResult>(), &ctr->escal_count[lc], map_len, map_words, ws, h->sm_count,
+                              S.copy_out),
+           "launching result patch");
+        o.launches += 1;
+    }
+    CK(cudaEventSynchronize(S.ev_kdone), "waiting for the kernel");
     const DevCounters *hc = L.h_counters.as<DevCounters>();
     const int64_t esc = (int64_t)hc->escal_count[lc];
-    if (esc > 0 && (out_len || out_words)) {
-        if (mapped) {
-            CK(launch_escal_patch(S.escal_out.as<EscalResult>(), &ctr->escal_count[lc], map_len, map_words, ws,
-                                  h->sm_count, S.copy_out),
-               "launching result patch");
-            o.launches += 1;
-        } else {
-            CK(S.h_escal.reserve((size_t)esc * sizeof(EscalResult)), "allocating escalated results");
-            CK(cudaMemcpyAsync(S.h_escal.ptr, S.escal_out.ptr, (size_t)esc * sizeof(EscalResult),
-                               cudaMemcpyDeviceToHost, S.copy_out),
-               "copying escalated results");
-        }
+    if (esc > 0 && (out_len || out_words) && !mapped) {
+        CK(S.h_escal.reserve((size_t)esc * sizeof(EscalResult)), "allocating escalated results");
+        CK(cudaMemcpyAsync(S.h_escal.ptr, S.escal_out.ptr, (size_t)esc * sizeof(EscalResult), cudaMemcpyDeviceToHost,
+                           S.copy_out),
+           "copying escalated results");
     }
     CK(cudaStreamSynchronize(S.copy_out), "copying results");
     if (!pin_out) {
@@ -952,11 +955,12 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
         std::atomic<bool> corrupt{false};
         h->copy_pool().parallel_for((size_t)esc, 2048, [&](size_t i0, size_t i1) {
             for (size_t i = i0; i < i1; ++i) {
-                if (i + 16 < i1) {   // the stores miss the cache: keep several in flight
+                if (i + 16 < i1 && r[i + 16].k >= 0) {   // the stores miss the cache: keep several in flight
                     if (out_len) __builtin_prefetch(out_len + r[i + 16].k, 1);
                     if (out_words) __builtin_prefetch(out_words + (size_t)r[i + 16].k * ws, 1);
                 }
                 const int64_t k = r[i].k;
+                if (k == kEscalInChunk) continue;
                 if (k < 0 || k >= cnt) {
                     corrupt.store(true, std::memory_order_relaxed);
                     continue;

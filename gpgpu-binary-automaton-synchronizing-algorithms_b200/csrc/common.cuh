@@ -130,13 +130,13 @@ cudaError_t launch_pool(const PoolShape &s, const Batch &b, uint32_t *spill,
                                                                                                         nullptr});
 int pool_max_ctas_per_sm(const PoolShape &s);
 
-size_t lane_smem_bytes(int nmax, int warps, int ring);
 int lane_max_ctas_per_sm(int nmax, int warps, int ring);
 // Streaming form of the per-lane kernel (host path, uniform batch in
 // order): records arrive chunk by chunk while the kernel runs, and results
 // leave chunk by chunk.  All pointers null = everything resident, no tracking.
+constexpr int64_t kEscalInChunk = -1;
 struct EscalResult {
-    int64_t k;          // automaton
+    int64_t k;          // automaton, or kEscalInChunk: its chunk's copy has the result
     int32_t len;
     int32_t pad;
     uint64_t word[3];   // n <= 13: at most 144 letters
@@ -152,7 +152,11 @@ struct LaneStream {
     // start sooner (whole 128-byte lines of records too)
     int64_t first;
 
-    __host__ __device__ int64_t chunk_of(int64_t k) const { return k < first ? 0 : 1 + (k - first) / chunk; }
+    // (a job's automata, 2^24 at most, are divided in 32 bits)
+    __host__ __device__ int64_t chunk_of(int64_t k) const
+    {
+        return k < first ? 0 : 1 + (int64_t)((uint32_t)(k - first) / (uint32_t)chunk);
+    }
     __host__ __device__ int64_t chunk_begin(int64_t c) const { return c == 0 ? 0 : first + (c - 1) * chunk; }
     // chunks of a batch of `count` automata, and the size of chunk c
     __host__ __device__ int64_t chunks(int64_t count) const

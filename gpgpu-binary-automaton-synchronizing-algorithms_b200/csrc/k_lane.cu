@@ -10,7 +10,23 @@
 //
 // Shared memory is lane-interleaved: element e of lane l's bitmap, table and
 // queue lives at [e][l], so every lane-private access of a warp touches 32
-// different banks.  The queue is a ring of R entries holding only the live
+// different banks.
+//
+// Shared memory bounds the resident warps, and those the speed (1M n = 12:
+// 0.71 ms at 6 warps per SM, 0.58 at 8, 0.51 at 10 of the same kernel), so the
+// bitmap is kept small (n > 8).  After the first letter every subset lies in the
+// image of a or of b.  With the states relabelled A \ B, A and B, B \ A, the rest
+// (A, B the images), a subset of A is a number below 2^rank(a), and one of B is,
+// shifted down by |A \ B|, one below 2^rank(b): 2^rank(a) + 2^rank(b) bits tell
+// all of them apart.  Ranks average 0.65 n; 1536 bits serve 98 % of random n = 12
+// (512 B of one bit per subset became 192 B, 7 warps per SM became 10), 3072 and
+// 6400 bits over 99 % at n = 13 and 14 (4 became 6, 2 became 3).  The other
+// automata take bitmaps from a pool of the warp's, in the order in which they came.
+// Relabelling changes neither the order of the search nor its words.  1M n = 12
+// device-resident: 0.592 -> 0.472 ms; 500K n = 14: 1.158 -> 0.760 ms; a Verify call
+// on 2^21 n = 13: 2.25 -> 1.95 ms.
+//
+// The queue is a ring of R entries holding only the live
 // frontier (current level remainder + next level); with words requested each
 // entry carries the letters of the word that reaches it (bit NMAX + d =
 // letter d, 1 = b), so a word needs no parent pointers or retained history.
@@ -19,7 +35,8 @@
 // looks up their eight images: more independent work per step hides the
 // shared-memory latencies that one warp's dependent chain exposes at 7 warps
 // per SM (2 -> 4 subsets: 0.64 -> 0.56 ms per 10^6 automata at n = 12; 6 and 8
-// were slower again).  A singleton among them ends the search (no singleton
+// were slower again; at ten warps per SM two take 0.556, three 0.521 and four
+// 0.515 ms).  A singleton among them ends the search (no singleton
 // is visited before the first one is generated, so it needs no bitmap test).
 // Otherwise the eight images are test-and-set with shared-memory atomicOr, issued
 // back to back and kept in program order by the hardware for a repeated
@@ -45,16 +62,22 @@
 // runs with many lanes active instead of one.
 //
 // Instances: NMAX = 8 and 12 for size classes 0 and 1; 13 and 14 for uniform
-// batches of that n (a fourth nibble chunk, 1 or 2 KB of bitmap per lane, and
-// words of up to (NMAX - 1)^2 = 144 or 169 letters -- three 64-bit words -- in
+// batches of that n (a fourth nibble chunk, and words of up to (NMAX - 1)^2 =
+// 144 or 169 letters -- three 64-bit words -- in
 // the whole-warp search).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sbfs {
 namespace {
 
-constexpr int kActive = 0, kDone = 1, kEscalate = 2, kIdle = 3, kHeld = 4;
+constexpr int kActive = 0, kDone = 1, kEscalate = 2, kIdle = 3, kHeld = 4, kWaiting = 5;
 constexpr int kStep = 4;   // subsets a lane expands per step (their 2 * kStep images are tested together)
+// Warps of a launched CTA when `warps` are asked for (n > 8: one, see kOneWarp),
+// and CTAs of that many that the registers must allow for
+__host__ __device__ constexpr int lane_cta_warps(int nmax, int warps) { return nmax <= 8 ? warps : 1; }
+__host__ __device__ constexpr int lane_min_ctas(int nmax) { return nmax <= 8 ? 4 : 11; }
 // At n = 13 and 14 fewer warps fit on an SM (four, two), and six subsets per
 // step hide more of each warp's latency: 2^21 automata at n = 14 4.83 -> 4.64 ms,
 // the n = 13 streamed kernel 2.19 -> 2.09 ms (eight: no better than six)
@@ -67,7 +90,27 @@ __host__ __device__ constexpr int low_bit4(int v)
 
 template <int NMAX>
 struct LaneGeom {
-    static constexpr int kBitmapWords = (1 << NMAX) / 32;
+    static constexpr int kBitmapWords = (1 << NMAX) / 32;   // whole-warp search: one bit per subset
+    // Per-lane search: words of a lane's visited bitmap, and the pool of
+    // bitmaps that serves the warp's lanes whose automaton needs more (half of one
+    // bit per subset, or a pair of such halves).  The pool takes what the resident
+    // warps leave of shared memory (10, 6 and 3 per SM at n = 12, 13 and 14): with
+    // one bitmap at n = 12 the automata that need it, the longer searches among
+    // them, queued up.
+    static constexpr bool kRelabel = NMAX > 8;
+    static constexpr int kLaneWords = NMAX <= 8 ? 8 : NMAX <= 12 ? 48 : NMAX == 13 ? 96 : 200;
+    static constexpr int kHalfWords = kRelabel ? kBitmapWords / 2 : 0;
+    static constexpr int kHalves = NMAX <= 8 ? 0 : NMAX <= 12 ? 6 : NMAX == 13 ? 2 : 8;
+    static constexpr int kPoolWords = kHalves * kHalfWords;
+    static constexpr uint32_t kAllHalves = (1u << kHalves) - 1u;
+    // One warp per CTA, so that its region starts at a constant address and every
+    // access of a step is a lane's offset plus an immediate (1M n = 12: 0.514 ->
+    // 0.490 ms at ten warps per SM).  n <= 8 keeps more warps than that allows.
+    static constexpr bool kOneWarp = NMAX > 8;
+    // Steps between two looks at the lanes' states while automata are left to hand
+    // out.  A look costs three ballots and their branches: 1M n = 12 0.507 ms with
+    // one step, 0.471 with two, three or four alike.
+    static constexpr int kRounds = NMAX > 8 ? 2 : 1;
     static constexpr int kChunks = (NMAX + 3) / 4;
     static constexpr int kTable = kChunks * 16;
     static constexpr uint32_t kMask = (1u << NMAX) - 1u;
@@ -80,8 +123,9 @@ __device__ __forceinline__ uint32_t lane_image(const uint32_t *tb, uint32_t x)
 {
     uint32_t t = tb[(x & 15u) * 32];
     if (LaneGeom<NMAX>::kChunks > 1) t |= tb[(16 + ((x >> 4) & 15u)) * 32];
+    // (x carries a word's letters from bit NMAX on)
     if (LaneGeom<NMAX>::kChunks > 2) t |= tb[(32 + ((x >> 8) & 15u)) * 32];
-    if (LaneGeom<NMAX>::kChunks > 3) t |= tb[(48 + ((x >> 12) & 15u)) * 32];
+    if (LaneGeom<NMAX>::kChunks > 3) t |= tb[(48 + ((x >> 12) & ((1u << (NMAX > 12 ? NMAX - 12 : 0)) - 1u))) * 32];
     return t;
 }
 
@@ -100,6 +144,73 @@ __device__ __forceinline__ uint32_t table_entry(const uint8_t *rec, int lstride,
     return t;
 }
 
+// v << (c & 31)
+__device__ __forceinline__ uint32_t shl_wrap(uint32_t v, uint32_t c) { return __funnelshift_l(0u, v, c); }
+
+// The bytes of a word that hold the first `left` of its four states (all when
+// left >= 4, none when left <= 0).
+__device__ __forceinline__ uint32_t keep_bytes(int left)
+{
+    return left >= 4 ? ~0u : left <= 0 ? 0u : (1u << (8 * left)) - 1u;
+}
+
+// Every byte of w (0..15) replaced by byte w of the table L.
+__device__ __forceinline__ uint32_t map_bytes(uint32_t w, const uint32_t (&L)[4])
+{
+    const uint32_t t = w & 0x07070707u;
+    const uint32_t sel = __byte_perm(t | (t >> 4), 0u, 0x4420);
+    const uint32_t low = __byte_perm(L[0], L[1], sel), high = __byte_perm(L[2], L[3], sel);
+    uint32_t m;   // 0xFF where bit 3 is set (selector bit 3: the sign of the byte, spread)
+    asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(m) : "r"(w << 4));
+    return (high & m) | (low & ~m);
+}
+
+// Four-byte pieces of one map of n states at p (any alignment); bytes past the
+// map are whatever follows it.
+template <int CHUNKS>
+__device__ __forceinline__ void load_map(const uint8_t *p, int n, uint32_t (&w)[CHUNKS])
+{
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);
+    const uint32_t *q = reinterpret_cast<const uint32_t *>(p - off);
+    uint32_t v[CHUNKS + 1];
+#pragma unroll
+    for (int c = 0; c <= CHUNKS; ++c) v[c] = 4 * c < n + (int)off ? __ldg(q + c) : 0u;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) w[c] = __funnelshift_r(v[c], v[c + 1], 8u * off);
+}
+
+// Automaton k's maps, four images per word.  Aligned words whatever the record
+// stride: a first or last record whose words would reach outside the batch is
+// read byte by byte.
+template <int NMAX>
+__device__ __forceinline__ void load_maps(const Batch &b, int64_t k, int n, int64_t count, bool valid,
+                                          uint32_t (&aw)[(NMAX + 3) / 4], uint32_t (&bw)[(NMAX + 3) / 4])
+{
+    constexpr int CH = (NMAX + 3) / 4;
+    const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) aw[c] = bw[c] = 0u;
+    if (!valid) return;
+    // an order array may point anywhere in the batch: only its own record is known to be there
+    const uint8_t *first = b.order ? rec : b.maps;
+    const uint8_t *end = b.order ? rec + 2 * b.lstride : b.maps + (size_t)count * 2u * (size_t)b.lstride;
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(rec) & ~(uintptr_t)3;
+    const uintptr_t hi = (reinterpret_cast<uintptr_t>(rec + b.lstride + n) + 3) & ~(uintptr_t)3;
+    if (lo >= reinterpret_cast<uintptr_t>(first) && hi <= reinterpret_cast<uintptr_t>(end)) {
+        load_map<CH>(rec, n, aw);
+        load_map<CH>(rec + b.lstride, n, bw);
+        return;
+    }
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (4 * c + j < n) {
+                aw[c] |= (uint32_t)__ldg(rec + 4 * c + j) << (8 * j);
+                bw[c] |= (uint32_t)__ldg(rec + b.lstride + 4 * c + j) << (8 * j);
+            }
+}
+
 // Claims the next escalated automaton of the launch for a warp with no lane
 // work left, or returns -1.  A claim is one atomicAdd on the claim counter and
 // one atomicCAS on the claimed slot, raced against the slot's writer (which
@@ -116,27 +227,15 @@ __device__ int64_t claim_escalated(int32_t *list, unsigned long long capacity, u
     return prev >= 0 ? (int64_t)prev : -1;
 }
 
-// Waits (bounded: `polls` polls about 0.2 us apart) until the streamed records
-// of chunk c are on the device; false when the wait ran out.
-__device__ bool wait_chunk(const unsigned int *ready, int64_t c, int polls)
-{
-    for (int it = 0; it < polls; ++it) {
-        if (*(volatile const unsigned int *)(ready + c)) {
-            __threadfence();
-            return true;
-        }
-        __nanosleep(200);
-    }
-    return false;
-}
-
 // One automaton (n <= NMAX) solved by the whole warp inside its region of
 // `region_words` shared words (>= 2^NMAX / 32 + 2^NMAX).  Queue entry:
-// subset | parent index << NMAX | letter << 2*NMAX (letter 1 = b).
+// subset | parent index << NMAX | letter << 2*NMAX (letter 1 = b).  Returns the
+// subsets this lane expanded.
 template <int NMAX, bool WORDS, bool STREAM>
-__device__ void warp_solve(const Batch &b, int64_t k, uint32_t *region, int lane, unsigned long long &expanded,
-                           const LaneStream &ls, unsigned long long slot)
+__device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, uint32_t *region, int lane,
+                                            const LaneStream &ls, unsigned long long slot)
 {
+    uint32_t expanded = 0;
     using G = LaneGeom<NMAX>;
     constexpr int BW = G::kBitmapWords;
     uint32_t *bm = region;        // linear bitmap
@@ -234,8 +333,13 @@ __device__ void warp_solve(const Batch &b, int64_t k, uint32_t *region, int lane
         }
         if (STREAM && ls.escal_out) {
             // streamed batches: the host patches escalated automata from here
+            // (if the chunk still had searches out after these results were stored, its
+            // copy, which comes after the last of them, takes them along)
+            __threadfence();
+            const int64_t c = ls.chunk_of(k);
+            const bool early = *(volatile unsigned int *)(ls.chunk_done + c) < (unsigned)ls.chunk_size(c, b.count);
             EscalResult r;
-            r.k = k;
+            r.k = early ? kEscalInChunk : k;
             r.len = len;
             r.pad = 0;
             r.word[0] = w0;
@@ -246,24 +350,53 @@ __device__ void warp_solve(const Batch &b, int64_t k, uint32_t *region, int lane
         publish_result(b, k);
     }
     __syncwarp();
+    return expanded;
+}
+
+// (a call of its own in the streamed kernel, which has three places for it)
+template <int NMAX, bool WORDS>
+__device__ __noinline__ uint32_t warp_solve_call(const Batch &b, int64_t k, uint32_t *region, int lane,
+                                                 const LaneStream &ls, unsigned long long slot)
+{
+    return warp_solve_body<NMAX, WORDS, true>(b, k, region, lane, ls, slot);
 }
 
 template <int NMAX, bool WORDS, bool STREAM>
-__global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, int tail_k, int32_t *escal_list,
-                                              unsigned long long escal_capacity, unsigned long long *escal_count,
-                                              unsigned long long *escal_claim, unsigned long long *ticket,
-                                              LaneStream ls)
+__device__ __forceinline__ uint32_t warp_solve(const Batch &b, int64_t k, uint32_t *region, int lane,
+                                               const LaneStream &ls, unsigned long long slot)
+{
+    return STREAM ? warp_solve_call<NMAX, WORDS>(b, k, region, lane, ls, slot)
+                  : warp_solve_body<NMAX, WORDS, false>(b, k, region, lane, ls, slot);
+}
+
+// Words of a warp's shared-memory region: the lanes' bitmaps, tables and rings
+// and the pool, or the whole-warp search's bitmap and queue.
+template <int NMAX>
+__host__ __device__ constexpr size_t region_words(int ring)
 {
     using G = LaneGeom<NMAX>;
-    constexpr int BW = G::kBitmapWords;
+    const size_t lanes = (size_t)(G::kLaneWords + G::kTable + ring) * 32 + G::kPoolWords;
+    const size_t whole = (size_t)G::kBitmapWords + ((size_t)1 << NMAX);
+    return lanes > whole ? lanes : whole;
+}
+
+template <int NMAX, bool WORDS, bool STREAM>
+__global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NMAX))
+    k_lane(const __grid_constant__ Batch b, int ring, int refill_k, int tail_k, int32_t *escal_list,
+           unsigned long long escal_capacity, unsigned long long *escal_count, unsigned long long *escal_claim,
+           unsigned long long *ticket, const __grid_constant__ LaneStream ls)
+{
+    using G = LaneGeom<NMAX>;
+    constexpr int LW = G::kLaneWords;
     constexpr int T = G::kTable;
     extern __shared__ __align__(16) uint32_t smem[];
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    uint32_t *base = smem + (size_t)warp * (BW + T + ring) * 32;
-    uint32_t *bm = base + lane;                  // bm[w * 32]
-    uint32_t *tb = base + BW * 32 + lane;        // tb[e * 32]
-    uint32_t *rq = base + (BW + T) * 32 + lane;  // rq[i * 32]
+    const int warp = G::kOneWarp ? 0 : threadIdx.x >> 5;
+    uint32_t *base = smem + (size_t)warp * region_words<NMAX>(ring);
+    uint32_t *const own = base + lane;           // the lane's bitmap, own[w * 32]
+    uint32_t *tb = base + LW * 32 + lane;        // tb[e * 32]
+    uint32_t *rq = base + (LW + T) * 32 + lane;  // rq[i * 32]
+    uint32_t *const pool = base + (LW + T + ring) * 32;
     const uint32_t rmask = (uint32_t)ring - 1u;
 
     int64_t count;
@@ -277,9 +410,18 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
     int32_t res_len = kLenNonSync;
     uint32_t res_word = 0;
     bool more = true;
-    unsigned long long expanded = 0;
+    unsigned long long expanded = 0;   // whole-warp searches
+    uint32_t steps_expanded = 0;       // this lane's own searches
     unsigned long long hslot = 0;   // escalation slot of a held automaton
-    int64_t ready_upto = -1;        // streamed chunks known to be on the device
+    // The lane's visited bitmap: bit y of subset y below low_end, bit index0 +
+    // (y >> shift) of the others (b-images only), word w at bm[w * stride].
+    uint32_t *bm = own;
+    uint32_t stride = 32, low_end = 1u << NMAX, index0 = 0, shift = 0;
+    uint32_t held = 0;              // halves of the pool this lane's bitmap is in
+    uint32_t pool_free = G::kAllHalves;   // halves nobody holds (alike in every lane)
+    uint32_t pass = 0, since = 0;   // passes that asked for the pool; the one this lane came in
+    uint32_t checks = 0;
+    int ready_upto = -1;            // streamed chunks known to be on the device
 
     while (true) {
         // ---- phase: finish waiting lanes, load new automata -----------------
@@ -291,8 +433,11 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
             if (state == kActive && __popc(active) <= tail_k) state = kEscalate;
         }
         const unsigned not_active = __ballot_sync(kFull, state != kActive);
-        if (not_active == kFull ||
-            (__popc(not_active) >= refill_k && (more || __any_sync(kFull, state == kDone || state == kEscalate)))) {
+        // (streamed: lanes that wait for records ask for a look at the chunk flags,
+        // one trip to L2, at every eighth check only)
+        const unsigned served = STREAM ? not_active & ~__ballot_sync(kFull, state == kWaiting) : not_active;
+        if (not_active == kFull || (STREAM && served != not_active && (++checks & 7u) == 0u) ||
+            (__popc(served) >= refill_k && (more || __any_sync(kFull, state == kDone || state == kEscalate)))) {
             const bool outcome = state == kDone || state == kEscalate;
             if (state == kDone) {
                 record_result(b, k, n, res_len);
@@ -338,61 +483,135 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
                     }
                 }
             }
-            if (state != kActive && state != kHeld) state = kIdle;
+            if (state != kActive && state != kHeld && state != kWaiting) state = kIdle;
+            if (G::kRelabel) {
+                if (state != kActive) held = 0;
+                pool_free = G::kAllHalves & ~__reduce_or_sync(kFull, held);
+            }
             const unsigned idle = __ballot_sync(kFull, state == kIdle);
+            bool fresh = false;   // the lane just received an automaton
             if (more && idle) {
                 unsigned long long got = 0;
                 const int leader = __ffs(idle) - 1;
                 if (lane == leader) got = atomicAdd(ticket, (unsigned long long)__popc(idle));
                 got = __shfl_sync(kFull, got, leader);
                 if (got + __popc(idle) >= (unsigned long long)count) more = false;
-                if (STREAM && got < (unsigned long long)count) {
-                    // streamed batch: the records handed out must have arrived
-                    const int64_t last = (int64_t)min(got + (unsigned long long)__popc(idle),
-                                                      (unsigned long long)count) - 1;
-                    const int64_t c_last = ls.chunk_of(last);
-                    if (c_last > ready_upto) {
-                        bool ok = true;
-                        if (lane == 0) ok = wait_chunk(ls.chunk_ready, c_last, ls.wait_polls);
-                        ok = __shfl_sync(kFull, ok, 0);
-                        if (!ok && lane == 0) atomicOr(b.error, kErrWait);
-                        ready_upto = c_last;
-                        __syncwarp();
-                    }
-                }
                 if (state == kIdle) {
                     const unsigned long long pos = got + __popc(idle & ((1u << lane) - 1u));
                     if (pos < (unsigned long long)count) {
                         k = automaton_at(order, (int64_t)pos);
                         n = automaton_n(b, k);
                         state = kActive;
+                        fresh = true;
+                        since = 0;
                     }
                 }
-                // every lane that just received an automaton sets it up
-                if (state == kActive && (idle & (1u << lane))) {
-                    bool bad = (n < 1 || n > NMAX || n > b.lstride);
-                    const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
-                    uint32_t aw[G::kChunks] = {}, bw[G::kChunks] = {};
-                    if (!bad) {
-                        if ((b.lstride & 3) == 0) {
-                            const uint32_t *ra = reinterpret_cast<const uint32_t *>(rec);
-                            const uint32_t *rb = reinterpret_cast<const uint32_t *>(rec + b.lstride);
-#pragma unroll
-                            for (int c = 0; c < G::kChunks; ++c) {
-                                aw[c] = 4 * c < n ? __ldg(ra + c) : 0u;
-                                bw[c] = 4 * c < n ? __ldg(rb + c) : 0u;
-                            }
+            }
+            // every lane that just received an automaton sets it up, and so does one
+            // that waited (for the pool, or for its records)
+            bool setup = fresh || state == kWaiting;
+            if (STREAM) {
+                // Streamed batch: the records handed out must have arrived.  A warp with
+                // other lanes still searching does not wait for them: stopping those
+                // would hold back the results of the chunk before (1M n = 12 end to
+                // end: 1.17 ms with every such wait blocking, now that the kernel is
+                // faster than the link).
+                const int c = setup ? (int)ls.chunk_of(k) : -1;
+                const int c_last = (int)__reduce_max_sync(kFull, (unsigned)(c + 1)) - 1;
+                if (c_last > ready_upto) {
+                    const int c_first = (int)__reduce_min_sync(kFull, setup ? (unsigned)c : ~0u);
+                    const bool busy = __any_sync(kFull, state == kActive && !fresh);
+                    // With nothing to search the warp waits (bounded: wait_polls polls
+                    // about 0.2 us apart), solving escalated automata meanwhile
+                    for (int polls = 0;;) {
+                        if (lane == 0)
+                            while (ready_upto < c_last &&
+                                   *(volatile const unsigned int *)(ls.chunk_ready + ready_upto + 1))
+                                ++ready_upto;
+                        ready_upto = __shfl_sync(kFull, ready_upto, 0);
+                        if (busy || ready_upto >= c_first) break;
+                        if (polls >= ls.wait_polls) {
+                            if (lane == 0) atomicOr(b.error, kErrWait);
+                            ready_upto = c_last;
+                            break;
+                        }
+                        int64_t e = -1;
+                        unsigned long long slot = 0;
+                        if (lane == 0 && *(volatile unsigned long long *)escal_claim <
+                                             *(volatile unsigned long long *)escal_count)
+                            e = claim_escalated(escal_list, escal_capacity, escal_claim, slot);
+                        e = __shfl_sync(kFull, e, 0);
+                        slot = __shfl_sync(kFull, slot, 0);
+                        if (e >= 0) {
+                            expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
                         } else {
+                            ++polls;
+                            __nanosleep(200);
+                        }
+                    }
+                    __threadfence();
+                }
+                if (setup && c > ready_upto) {
+                    setup = fresh = false;
+                    state = kWaiting;
+                }
+            }
+            if (__any_sync(kFull, setup)) {
+                uint32_t words = 0, halves = 0;   // bitmap words, and pool halves they take
+                if (setup) {
+                    state = kActive;
+                    bool bad = (n < 1 || n > NMAX || n > b.lstride);
+                    const int nn = bad ? 1 : n;
+                    uint32_t aw[G::kChunks], bw[G::kChunks];   // four images each, 15 past the last state
+                    load_maps<NMAX>(b, k, nn, count, !bad, aw, bw);
+                    {
+                        uint32_t high = 0;   // top bits: an image that is no state
+                        const uint32_t over = (0x80u - (uint32_t)nn) * 0x01010101u;
 #pragma unroll
-                            for (int c = 0; c < G::kChunks; ++c) {
+                        for (int c = 0; c < G::kChunks; ++c) {
+                            const uint32_t keep = keep_bytes(nn - 4 * c);
+                            aw[c] &= keep;
+                            bw[c] &= keep;
+                            high |= aw[c] | (aw[c] + over) | bw[c] | (bw[c] + over);
+                            aw[c] |= 0x0F0F0F0Fu & ~keep;
+                            bw[c] |= 0x0F0F0F0Fu & ~keep;
+                        }
+                        bad |= (high & 0x80808080u) != 0u;
+                    }
+                    uint32_t ra = 0, rb = 0, a_only = 0;
+                    bool b_only = false;
+                    if (G::kRelabel) {
+                        // bit 2q: q is an image of a, bit 2q + 1: of b
+                        uint32_t z = 0;
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    if (4 * c + j < n) {
-                                        aw[c] |= (uint32_t)__ldg(rec + 4 * c + j) << (8 * j);
-                                        bw[c] |= (uint32_t)__ldg(rec + b.lstride + 4 * c + j) << (8 * j);
-                                    }
-                                }
-                            }
+                        for (int c = 0; c < G::kChunks; ++c)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                z |= shl_wrap(1u, (aw[c] * 2u) >> (8 * j)) | shl_wrap(2u, (bw[c] * 2u) >> (8 * j));
+                        z &= (1u << (2 * nn)) - 1u;
+                        const uint32_t za = z & 0x55555555u, zb = (z >> 1) & 0x55555555u;
+                        ra = (uint32_t)__popc(za);
+                        rb = (uint32_t)__popc(zb);
+                        a_only = (uint32_t)__popc(za & ~zb);
+                        b_only = (zb & ~za) != 0u;
+                        // new labels, a byte per state: A \ B | A and B | B \ A | the rest.  One
+                        // counter per group, at byte (in A) + 2 * (in B) of `next`
+                        uint32_t next = (a_only + rb) | (ra << 16) | (a_only << 24);
+                        uint32_t L[4] = {0u, 0u, 0u, 16u << 24};   // 16: the label of image 15, none
+#pragma unroll
+                        for (int st = 0; st < NMAX; ++st) {
+                            const uint32_t at = (st < 2 ? z << (3 - 2 * st) : z >> (2 * st - 3)) & 24u;
+                            L[st / 4] = __byte_perm(L[st / 4], next >> at, 0x3210 ^ ((st & 3 ^ 4) << (4 * (st & 3))));
+                            next += 1u << at;
+                        }
+#pragma unroll
+                        for (int c = 0; c < G::kChunks; ++c) {
+                            const uint32_t la = map_bytes(aw[c], L), lb = map_bytes(bw[c], L);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (4 * c + j < NMAX)
+                                    own[((L[c] >> (8 * j)) & 0xFFu) * 32u] =
+                                        shl_wrap(0x10000u, la >> (8 * j)) | (shl_wrap(1u, lb >> (8 * j)) & 0xFFFFu);
                         }
                     }
 #pragma unroll
@@ -401,10 +620,12 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const int st = 4 * c + j;
-                            const uint32_t av = (aw[c] >> (8 * j)) & 0xFFu, bv = (bw[c] >> (8 * j)) & 0xFFu;
-                            const bool in = !bad && st < n;
-                            if (in && (av >= (uint32_t)n || bv >= (uint32_t)n)) bad = true;
-                            s[j] = in ? ((1u << ((av & 15u) + 16)) | (1u << (bv & 15u))) : 0u;
+                            if (G::kRelabel) {
+                                s[j] = st < NMAX ? own[st * 32] : 0u;
+                            } else {
+                                const uint32_t av = (aw[c] >> (8 * j)) & 15u, bv = (bw[c] >> (8 * j)) & 15u;
+                                s[j] = st < nn ? (1u << (av + 16)) | (1u << bv) : 0u;
+                            }
                         }
                         // table[c*16 + v] = OR of s[j] over the set bits j of v
                         uint32_t t[16];
@@ -430,16 +651,72 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
                         res_len = kLenNonSync;
                         res_word = 0;
                     } else {
-#pragma unroll 16
-                        for (int w = 0; w < BW; ++w) bm[w * 32] = 0u;
-                        const uint32_t full = (1u << n) - 1u;
-                        bm[(full >> 5) * 32] = 1u << (full & 31u);
-                        rq[0] = full;
-                        head = 0;
-                        tail = 1;
-                        lvl_end = 1;
-                        level = 0;
+                        uint32_t bits = 1u << n;
+                        index0 = shift = 0;
+                        low_end = 1u << NMAX;
+                        if (G::kRelabel) {
+                            const uint32_t need = (1u << ra) + (b_only ? 1u << rb : 0u);
+                            if (need < bits) {
+                                bits = need;
+                                low_end = index0 = 1u << ra;
+                                shift = a_only;
+                            }
+                        }
+                        words = (bits + 31u) / 32u;
+                        halves = words <= (uint32_t)LW ? 0u : words <= (uint32_t)G::kHalfWords ? 1u : 2u;
+                        bm = own;
+                        stride = 32;
                     }
+                }
+                if (G::kRelabel) {
+                    // The pool goes to the lanes that need it, in the order in which they
+                    // came; the others wait.  (Out of order, a lane could wait until the
+                    // end of the batch: a streamed batch's first chunk was then complete
+                    // only with its last.)
+                    unsigned want = __ballot_sync(kFull, halves != 0u);
+                    if (want) ++pass;
+                    if (halves != 0u && since == 0u) since = pass;
+                    for (; want; ) {
+                        const uint32_t first = __reduce_min_sync(kFull, (want >> lane) & 1u ? since : ~0u);
+                        const int l = __ffs(__ballot_sync(kFull, ((want >> lane) & 1u) && since == first)) - 1;
+                        const uint32_t pairs = pool_free & (pool_free >> 1) & 0x55555555u;
+                        const bool two = __shfl_sync(kFull, halves, l) == 2u;
+                        // one half: of a broken pair if there is one
+                        const uint32_t lone = pool_free & ~(pairs * 3u);
+                        const uint32_t from = two ? pairs : lone ? lone : pool_free;
+                        if (!from) break;
+                        const int at = __ffs(from) - 1;
+                        const uint32_t take = (two ? 3u : 1u) << at;
+                        want &= ~(1u << l);
+                        pool_free &= ~take;
+                        uint32_t *const part = pool + at * G::kHalfWords;
+                        for (int w = lane; w < (two ? 2 : 1) * G::kHalfWords; w += 32) part[w] = 0u;
+                        __syncwarp();
+                        if (lane == l) {
+                            bm = part;
+                            stride = 1;
+                            held = take;
+                        }
+                    }
+                    if (halves != 0u) {
+                        words = 0;
+                        if (!held) state = kWaiting;
+                    }
+                }
+                const uint32_t most = __reduce_max_sync(kFull, words);
+#pragma unroll 8
+                for (uint32_t w = 0; w < most; ++w)
+                    if (setup) own[w * 32] = 0u;
+                if (setup && state == kActive) {
+                    const uint32_t full = (1u << n) - 1u;
+                    // the root comes back only through a permutation, and then every
+                    // subset keeps its plain index
+                    if (index0 == 0) bm[(full >> 5) * (G::kRelabel ? stride : 32u)] = 1u << (full & 31u);
+                    rq[0] = full;
+                    head = 0;
+                    tail = 1;
+                    lvl_end = 1;
+                    level = 0;
                 }
             }
             if (__ballot_sync(kFull, state == kActive) == 0u) {
@@ -448,7 +725,7 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
                 for (unsigned held = __ballot_sync(kFull, state == kHeld); held; held &= held - 1u) {
                     const int64_t e = __shfl_sync(kFull, k, __ffs(held) - 1);
                     const unsigned long long slot = __shfl_sync(kFull, hslot, __ffs(held) - 1);
-                    warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, expanded, ls, slot);
+                    expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
                 }
                 if (state == kHeld) state = kIdle;
                 if (!more) {
@@ -463,7 +740,7 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
                         e = __shfl_sync(kFull, e, 0);
                         slot = __shfl_sync(kFull, slot, 0);
                         if (e < 0) break;
-                        warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, expanded, ls, slot);
+                        expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
                     }
                     break;
                 }
@@ -472,79 +749,92 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
         }
 
         // ---- up to kStep expansions per active lane ----------------------------
-        if (state == kActive) {
-            // a lane with fewer than kStep subsets left in the level expands its
-            // first one again in the spare places: those copies' images are
-            // already visited by the time they are tested
-            constexpr int P = NMAX >= 13 ? kStepWide : kStep;
-            const uint32_t take = min(lvl_end - head, (uint32_t)P);
-            uint32_t e[P];
+        // (kRounds of them between two looks at the lanes while new automata are
+        // left; in the tail one, so that the few lanes left are seen at once)
+#pragma unroll 1
+        for (int round = 0; round < G::kRounds; ++round) {
+            if (state == kActive && (round == 0 || more)) {
+                // a lane with fewer than kStep subsets left in the level expands its
+                // first one again in the spare places: those copies' images are
+                // already visited by the time they are tested
+                constexpr int P = NMAX >= 13 ? kStepWide : kStep;
+                const uint32_t take = min(lvl_end - head, (uint32_t)P);
+                uint32_t e[P];
 #pragma unroll
-            for (int i = 0; i < P; ++i)
-                e[i] = (i == 0 || (uint32_t)i < take) ? rq[((head + (uint32_t)i) & rmask) * 32] : e[0];
-            head += take;
-            expanded += take;
-            uint32_t y[2 * P], hi[2 * P];
-            // entries carry the word that reaches them: the parent's letters,
-            // plus letter `level` = b for the b-images (an entry holds 32 - NMAX
-            // letters; at level >= 32 - NMAX a fresh image escalates instead)
-            const uint32_t lb = (WORDS && level < (uint32_t)G::kWordMax) ? 1u << (level + NMAX) : 0u;
+                for (int i = 0; i < P; ++i)
+                    e[i] = (i == 0 || (uint32_t)i < take) ? rq[((head + (uint32_t)i) & rmask) * 32] : e[0];
+                head += take;
+                steps_expanded += take;
+                uint32_t y[2 * P], hi[2 * P];
+                // entries carry the word that reaches them: the parent's letters,
+                // plus letter `level` = b for the b-images (an entry holds 32 - NMAX
+                // letters; at level >= 32 - NMAX a fresh image escalates instead)
+                const uint32_t lb = (WORDS && level < (uint32_t)G::kWordMax) ? 1u << (level + NMAX) : 0u;
 #pragma unroll
-            for (int i = 0; i < P; ++i) {
-                const uint32_t t = lane_image<NMAX>(tb, e[i] & G::kMask);
-                y[2 * i] = t >> 16;
-                y[2 * i + 1] = t & 0xFFFFu;
-                hi[2 * i] = WORDS ? (e[i] & ~G::kMask) : 0u;
-                hi[2 * i + 1] = WORDS ? ((e[i] & ~G::kMask) | lb) : 0u;
-            }
-            // no singleton is ever visited (the search stops at the first one), so
-            // a singleton image ends the search without a bitmap test
-            int sc = -1;
+                for (int i = 0; i < P; ++i) {
+                    const uint32_t t = lane_image<NMAX>(tb, e[i]);
+                    y[2 * i] = t >> 16;
+                    y[2 * i + 1] = t & 0xFFFFu;
+                    hi[2 * i] = e[i];
+                    hi[2 * i + 1] = e[i] | lb;
+                }
+                // no singleton is ever visited (the search stops at the first one), so
+                // a singleton image ends the search without a bitmap test
+                bool hit = false;
 #pragma unroll
-            for (int c = 2 * P - 1; c >= 0; --c)
-                if (is_singleton(y[c])) sc = c;
-            if (sc >= 0) {
-                state = kDone;
-                res_len = (int32_t)level + 1;
-                uint32_t es = e[0];
+                for (int c = 0; c < 2 * P; ++c) hit |= is_singleton(y[c]);
+                if (hit) {
+                    int sc = 0;   // the first one in queue order
 #pragma unroll
-                for (int i = 1; i < P; ++i)
-                    if ((sc >> 1) == i) es = e[i];
-                res_word = WORDS ? ((es >> NMAX) | ((uint32_t)(sc & 1) << level)) : 0u;
-            } else {
-                // test-and-set in queue order: a subset met twice in this step is
-                // fresh only the first time (same-address atomics keep program order)
-                uint32_t old[2 * P];
+                    for (int c = 2 * P - 1; c >= 0; --c)
+                        if (is_singleton(y[c])) sc = c;
+                    state = kDone;
+                    res_len = (int32_t)level + 1;
+                    uint32_t es = e[0];
 #pragma unroll
-                for (int c = 0; c < 2 * P; ++c)
-                    old[c] = SBFS_CHECK((y[c] >> 5) < (uint32_t)BW, b.error)
-                                 ? atomicOr(&bm[(y[c] >> 5) * 32], 1u << (y[c] & 31u))
-                                 : ~0u;
-                bool any = false;
+                    for (int i = 1; i < P; ++i)
+                        if ((sc >> 1) == i) es = e[i];
+                    res_word = WORDS ? ((es >> NMAX) | ((uint32_t)(sc & 1) << level)) : 0u;
+                } else {
+                    // test-and-set in queue order: a subset met twice in this step is
+                    // fresh only the first time (same-address atomics keep program order)
+                    uint32_t old[2 * P], at[2 * P];
 #pragma unroll
-                for (int c = 0; c < 2 * P; ++c) {
-                    if (!(old[c] & (1u << (y[c] & 31u)))) {
-                        rq[(tail & rmask) * 32] = y[c] | hi[c];
-                        ++tail;
-                        any = true;
+                    for (int c = 0; c < 2 * P; ++c) {
+                        // an a-image is always below low_end
+                        at[c] = !G::kRelabel || (c & 1) == 0 || y[c] < low_end ? y[c] : index0 + (y[c] >> shift);
+                        old[c] = SBFS_CHECK((at[c] >> 5) < (held ? 2u * (uint32_t)G::kHalfWords : (uint32_t)LW), b.error)
+                                     ? atomicOr(&bm[(at[c] >> 5) * (G::kRelabel ? stride : 32u)], 1u << (at[c] & 31u))
+                                     : ~0u;
+                    }
+                    bool any = false;
+#pragma unroll
+                    for (int c = 0; c < 2 * P; ++c) {
+                        if (!(old[c] & (1u << (at[c] & 31u)))) {
+                            rq[(tail & rmask) * 32] = WORDS ? y[c] | (hi[c] & ~G::kMask) : y[c];
+                            ++tail;
+                            any = true;
+                        }
+                    }
+                    // more live entries than ring slots (the oldest were overwritten), or
+                    // a word longer than an entry carries: the whole-warp search takes over
+                    if (tail - head > (uint32_t)ring || (WORDS && any && level >= (uint32_t)G::kWordMax)) {
+                        state = kEscalate;
+                    } else if (head == lvl_end) {
+                        if (tail == lvl_end) {
+                            state = kDone;
+                            res_len = kLenNonSync;
+                        } else {
+                            lvl_end = tail;
+                            ++level;
+                        }
                     }
                 }
-                // more live entries than ring slots (the oldest were overwritten), or
-                // a word longer than an entry carries: the whole-warp search takes over
-                if (tail - head > (uint32_t)ring || (WORDS && any && level >= (uint32_t)G::kWordMax)) {
-                    state = kEscalate;
-                } else if (head == lvl_end) {
-                    if (tail == lvl_end) {
-                        state = kDone;
-                        res_len = kLenNonSync;
-                    } else {
-                        lvl_end = tail;
-                        ++level;
-                    }
-                }
             }
+            __syncwarp();
         }
     }
+    expanded += steps_expanded;
     for (int o = 16; o; o >>= 1) expanded += __shfl_down_sync(kFull, expanded, o);
     if (lane == 0 && b.expanded) atomicAdd(b.expanded, expanded);
 }
@@ -552,8 +842,7 @@ __global__ void __launch_bounds__(256) k_lane(Batch b, int ring, int refill_k, i
 template <int NMAX>
 size_t smem_for(int warps, int ring)
 {
-    using G = LaneGeom<NMAX>;
-    return (size_t)warps * (G::kBitmapWords + G::kTable + ring) * 32 * sizeof(uint32_t);
+    return (size_t)warps * region_words<NMAX>(ring) * sizeof(uint32_t);
 }
 
 template <int NMAX, bool WORDS>
@@ -562,48 +851,43 @@ cudaError_t launch_t(int warps, int ring, int refill_k, int tail_k, int ctas, co
                      unsigned long long *escal_claim, unsigned long long *ticket, const LaneStream &ls,
                      cudaStream_t st)
 {
-    using G = LaneGeom<NMAX>;
-    // the warp-cooperative search needs the bitmap and 2^NMAX queue entries in one region
-    if ((size_t)G::kBitmapWords + ((size_t)1 << NMAX) > (size_t)(G::kBitmapWords + G::kTable + ring) * 32)
-        return cudaErrorInvalidValue;
-    const size_t smem = smem_for<NMAX>(warps, ring);
+    // a grid of `ctas` CTAs of `warps` warps, as CTAs of one warp where the kernel wants those
+    const int w = lane_cta_warps(NMAX, warps);
+    const size_t smem = smem_for<NMAX>(w, ring);
     // the streamed form's bookkeeping is compiled out of the resident-batch kernel
     auto kernel = ls.chunk_done ? k_lane<NMAX, WORDS, true> : k_lane<NMAX, WORDS, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kernel<<<ctas, warps * 32, smem, st>>>(b, ring, refill_k, tail_k, escal_list, escal_capacity, escal_count,
-                                           escal_claim, ticket, ls);
+    kernel<<<ctas * (warps / w), w * 32, smem, st>>>(b, ring, refill_k, tail_k, escal_list, escal_capacity,
+                                                     escal_count, escal_claim, ticket, ls);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t lane_smem_bytes(int nmax, int warps, int ring)
-{
-    return nmax <= 8    ? smem_for<8>(warps, ring)
-           : nmax <= 12 ? smem_for<12>(warps, ring)
-           : nmax == 13 ? smem_for<13>(warps, ring)
-                        : smem_for<14>(warps, ring);
-}
-
+// CTAs of `warps` warps that an SM holds (n > 8: groups of that many one-warp CTAs).
 int lane_max_ctas_per_sm(int nmax, int warps, int ring)
 {
-    if (nmax > 14) return 0;
+    if (nmax > 14 || warps < 1) return 0;
     const void *k = nmax <= 8    ? (const void *)k_lane<8, true, false>
                     : nmax <= 12 ? (const void *)k_lane<12, true, false>
                     : nmax == 13 ? (const void *)k_lane<13, true, false>
                                  : (const void *)k_lane<14, true, false>;
-    const size_t smem = lane_smem_bytes(nmax, warps, ring);
+    const int w = lane_cta_warps(nmax, warps);
+    const size_t smem = nmax <= 8    ? smem_for<8>(w, ring)
+                        : nmax <= 12 ? smem_for<12>(w, ring)
+                        : nmax == 13 ? smem_for<13>(w, ring)
+                                     : smem_for<14>(w, ring);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, warps * 32, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, w * 32, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    return blocks;
+    return blocks * w / warps;
 }
 
 // Streamed batches: after the chunk copies, the escalated automata's results
@@ -615,6 +899,7 @@ __global__ void k_escal_patch(const EscalResult *r, const unsigned long long *co
     const int64_t n = (int64_t)*count;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const EscalResult e = r[i];
+        if (e.k == kEscalInChunk) continue;
         if (len) len[e.k] = e.len;
         if (words) {
             uint64_t *w = words + (size_t)e.k * (size_t)ws;

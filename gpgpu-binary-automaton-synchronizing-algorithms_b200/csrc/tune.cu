@@ -96,7 +96,7 @@ std::string device_key(sbfs_handle *h)
     cudaDeviceProp p;
     cudaGetDeviceProperties(&p, h->device);
     char buf[320];
-    std::snprintf(buf, sizeof buf, "%s|sm%d|abi%d|v10", p.name, h->sm_count, SBFS_ABI_VERSION);
+    std::snprintf(buf, sizeof buf, "%s|sm%d|abi%d|v11", p.name, h->sm_count, SBFS_ABI_VERSION);
     for (char *c = buf; *c; ++c)
         if (*c == ' ') *c = '_';
     return buf;
@@ -206,7 +206,7 @@ cudaError_t plan_autotune(sbfs_handle *h, Plan &plan)
         if ((e = prepare(b, n, count)) != cudaSuccess) break;
         Plan best = P;
         double best_ms = 1e30;
-        const int warps_c[2][3] = {{2, 4, 8}, {1, 2, 0}};
+        const int warps_c[2][3] = {{2, 4, 8}, {1, 0, 0}};   // n > 8 runs one-warp CTAs
         for (int w : warps_c[c])
             for (int ring : {16, 32, 64})
                 for (int rk : {8, 16})
