@@ -33,10 +33,11 @@ cudaError_t launch_cta(int nb_max, int threads, int ctas, const Batch &b, uint64
                        unsigned long long *ticket, cudaStream_t st);
 cudaError_t plan_autotune(sbfs_handle *h, Plan &plan);
 int hash_max_ctas_per_sm(int size, int max_n);
-cudaError_t launch_sort_handoff(const Batch &b, const int32_t *list, const unsigned long long *count, int32_t *out,
-                                int top_n, unsigned long long *split, cudaStream_t st);
 cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
                         unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st);
+size_t mid_spill_entries(int sm_count);
+cudaError_t launch_mid(int sm_count, const Batch &b, uint64_t *spill, int32_t *left_list,
+                       unsigned long long *left_count, unsigned long long *ticket, cudaStream_t st);
 cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
                         unsigned long long *ticket, cudaStream_t st);
 
@@ -103,7 +104,6 @@ constexpr int kDefaultLanes = 4;
 // CTA-wide kernel: random automata with n <= 20 stay below 40 (max 36 in 20K
 // samples at n = 20), a Cerny automaton needs (n-1)^2
 constexpr int kPoolLevelCap = 48;
-constexpr int kHandoffThreads16 = 256;   // CTA width of the CTA-wide kernel on n <= 16 hand-offs
 constexpr int64_t kDefaultChunk = 1 << 18;
 
 sbfs_status fail(sbfs_handle *h, sbfs_status st, const std::string &msg)
@@ -327,59 +327,40 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                    (c == 3 && P.class3_hash && !P.class3_level)) {
             const int size = c == 2 ? P.class2_hash : P.class3_hash;
             const int nb = c == 2 ? kClassMaxN[2] : std::min(20, std::max(j.ns ? j.max_n : j.n_uniform, 17));
-            // class 2's hand-offs (Cerny C_13..C_16: a few hundred subsets per level)
-            // run 256-thread CTAs, several per SM; class 3 keeps the tuned width
-            const int threads = c == 2 && !plain && !ticket_override ? std::min(P.cta.threads, kHandoffThreads16)
-                                                                     : P.cta.threads;
+            const int threads = P.cta.threads;
             const int per_sm = cta_max_ctas_per_sm(nb, threads);
             if (per_sm < 1) return fail(h, SBFS_ECUDA, "CTA-wide kernel does not fit on an SM");
             const int ctas = std::min(P.cta.ctas, per_sm * h->sm_count);
-            CK(L.heavy_queue[c].reserve(cta_queue_entries(nb, ctas) * sizeof(uint64_t)), "allocating CTA queues");
-            if (plain || ticket_override) {
+            const bool direct = plain || ticket_override;
+            if (direct || c == 3)
+                CK(L.heavy_queue[c].reserve(cta_queue_entries(nb, ctas) * sizeof(uint64_t)), "allocating CTA queues");
+            if (direct) {
                 CK(launch_cta(nb, threads, ctas, bc, L.heavy_queue[c].as<uint64_t>(), ticket, cs),
                    "launching CTA-wide kernel");
             } else {
-                // one warp per automaton with a hash set; searches wider than its
-                // set or longer than its level cap go to the CTA-wide kernel, same stream
+                // one warp per automaton; what is wide both ways goes on to k_mid, and
+                // class 3's largest ranks from there to the CTA-wide kernel, on the same stream
                 const int hper = hash_max_ctas_per_sm(size, kClassMaxN[c]);
                 if (hper < 1) return fail(h, SBFS_ECUDA, "hash-set kernel does not fit on an SM");
-                // hand-off list | the same sorted by n, largest first (mixed sizes)
-                CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off list");
+                // left by k_hash | left by k_mid
+                CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off lists");
                 int32_t *list = L.heavy[c].as<int32_t>();
                 CK(launch_hash(size, kClassMaxN[c], hper * h->sm_count, bc, list, &ctr->heavy_range[c][1], ticket, cs),
                    "launching hash-set kernel");
                 Batch bh = bc;
                 bh.order = list;
                 bh.range_dev = ctr->heavy_range[c];
-                // class 3, mixed sizes: the hand-offs below the class's top n run in a
-                // second launch sized for n - 1, whose halved bitmap fits two CTAs per SM
-                const bool split = j.ns && c == 3 && nb >= 18;
-                if (j.ns) {
-                    CK(launch_sort_handoff(bc, list, &ctr->heavy_range[c][1], list + escal_entries, nb,
-                                           split ? ctr->heavy_split[c] : nullptr, cs),
-                       "launching hand-off sort");
+                DevBuf &spill = L.mid_spill[c - 2];
+                CK(spill.reserve(mid_spill_entries(h->sm_count) * sizeof(uint64_t)), "allocating queue spill");
+                CK(launch_mid(h->sm_count, bh, spill.as<uint64_t>(), list + escal_entries, &ctr->left_range[c][1],
+                              &ctr->heavy_ticket[c], cs),
+                   "launching hand-off kernel");
+                *launches += 1;
+                if (c == 3) {
                     bh.order = list + escal_entries;
-                    *launches += 1;
-                }
-                if (split) {
-                    const int nb2 = nb - 1;
-                    const int per_sm2 = cta_max_ctas_per_sm(nb2, threads);
-                    if (per_sm2 < 1) return fail(h, SBFS_ECUDA, "CTA-wide kernel does not fit on an SM");
-                    const int ctas2 = std::min(P.cta.ctas, per_sm2 * h->sm_count);
-                    CK(L.heavy_queue[c].reserve(std::max(cta_queue_entries(nb, ctas), cta_queue_entries(nb2, ctas2)) *
-                                                sizeof(uint64_t)),
-                       "allocating CTA queues");
-                    bh.range_dev = ctr->heavy_split[c];
-                    CK(launch_cta(nb, threads, ctas, bh, L.heavy_queue[c].as<uint64_t>(), &ctr->heavy_ticket[c], cs),
-                       "launching hand-off kernel");
-                    bh.range_dev = ctr->heavy_split[c] + 2;
-                    CK(launch_cta(nb2, threads, ctas2, bh, L.heavy_queue[c].as<uint64_t>(), &ctr->heavy_ticket2[c],
-                                  cs),
-                       "launching hand-off kernel");
-                    *launches += 2;
-                } else {
-                    CK(launch_cta(nb, threads, ctas, bh, L.heavy_queue[c].as<uint64_t>(), &ctr->heavy_ticket[c], cs),
-                       "launching hand-off kernel");
+                    bh.range_dev = ctr->left_range[c];
+                    CK(launch_cta(nb, threads, ctas, bh, L.heavy_queue[c].as<uint64_t>(), &ctr->left_ticket[c], cs),
+                       "launching CTA-wide kernel");
                     *launches += 1;
                 }
             }
@@ -430,10 +411,11 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                    "launching hash-set kernel");
                 bc.order = list;
                 bc.range_dev = ctr->heavy_range[c];
-                CK(launch_wide(h->sm_count, bc, list + escal_entries, &ctr->wide_range[1], &ctr->heavy_ticket[c], cs),
+                CK(launch_wide(h->sm_count, bc, list + escal_entries, &ctr->left_range[c][1], &ctr->heavy_ticket[c],
+                               cs),
                    "launching CTA-wide hash-set kernel");
                 bc.order = list + escal_entries;
-                bc.range_dev = ctr->wide_range;
+                bc.range_dev = ctr->left_range[c];
                 *launches += 2;
             }
             sbfs_status ls = run_level_class(h, L, j, bc, launches);
@@ -1346,6 +1328,7 @@ sbfs_status sbfs_destroy(sbfs_handle *h)
         }
         for (DevBuf &d : L.heavy) d.release();
         for (DevBuf &d : L.heavy_queue) d.release();
+        for (DevBuf &d : L.mid_spill) d.release();
         if (L.level_ready) L.level.destroy();
         if (L.stream) cudaStreamDestroy(L.stream);
     }

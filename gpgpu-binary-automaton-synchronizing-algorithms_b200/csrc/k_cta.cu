@@ -1,4 +1,6 @@
-// k_cta.cu -- power-set BFS with one automaton per CTA (n <= 20).
+// k_cta.cu -- power-set BFS with one automaton per CTA (n <= 20): the searches of
+// n = 17..20 that k_hash and k_mid leave, the pooled kernel's long ones, and the
+// plain form.
 //
 // The visited bitmap (2^n bits, up to 128 KiB at n = 20) lives in shared
 // memory; the level-ordered queue lives in a per-CTA global area of 2^n

@@ -31,7 +31,7 @@
 // settles the slowly synchronizing families and the automata that never
 // synchronize; one with a permutation letter and a letter merging at most one
 // pair is tried backwards at once.  What is left -- wide both ways -- goes to
-// the CTA-wide kernel (k_cta, or k_wide above n = 20) through a list.  Random
+// one CTA per automaton (k_mid, or k_wide above n = 20) through a list.  Random
 // n = 17..20: 1.7 % of the automata pass 1536 subsets, 0.3 % pass 4096.
 // 200K mixed n = 6..20 with 1 % Cerny automata: 3.04 ms with every such
 // automaton on the CTA-wide kernel, 1.17 ms with the inverse search, 0.67 ms
@@ -572,49 +572,6 @@ __global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32, HashGeom<MA
     if (lane == 0 && b.expanded && expanded) atomicAdd(b.expanded, expanded);
 }
 
-// Counting sort of a hand-off list by n, largest first (one CTA): the
-// persistent CTA-wide kernel then takes the longest searches first, and the
-// short ones fill the SMs that free up (longest-processing-time order).
-// With split, the sorted list is also described as two work ranges,
-// {0, entries with n >= top_n} and {that, the rest}, so the entries below
-// top_n can run in a launch sized for top_n - 1.
-__global__ void __launch_bounds__(1024) k_sort_handoff(Batch b, const int32_t *list,
-                                                       const unsigned long long *count, int32_t *out,
-                                                       int top_n, unsigned long long *split)
-{
-    __shared__ unsigned int hist[SBFS_MAX_N + 2];
-    const int tid = threadIdx.x;
-    const int64_t cnt = (int64_t)*count;
-    for (int i = tid; i < SBFS_MAX_N + 2; i += blockDim.x) hist[i] = 0u;
-    __syncthreads();
-    for (int64_t i = tid; i < cnt; i += blockDim.x) {
-        const int n = min(max(automaton_n(b, list[i]), 0), SBFS_MAX_N + 1);
-        atomicAdd(&hist[n], 1u);
-    }
-    __syncthreads();
-    if (tid == 0) {
-        unsigned int off = 0, top = 0;
-        for (int n = SBFS_MAX_N + 1; n >= 0; --n) {
-            const unsigned int c = hist[n];
-            hist[n] = off;
-            off += c;
-            if (n == top_n) top = off;   // entries with n >= top_n
-        }
-        if (split) {
-            split[0] = 0ull;
-            split[1] = top;
-            split[2] = top;
-            split[3] = (unsigned long long)cnt - top;
-        }
-    }
-    __syncthreads();
-    for (int64_t i = tid; i < cnt; i += blockDim.x) {
-        const int32_t k = list[i];
-        const int n = min(max(automaton_n(b, k), 0), SBFS_MAX_N + 1);
-        out[atomicAdd(&hist[n], 1u)] = k;
-    }
-}
-
 constexpr int kMaxDevices = 16;
 
 int current_device()
@@ -684,13 +641,6 @@ int hash_max_ctas_per_sm(int size, int max_n)
     if (max_n > 20) return size == 2 ? HashLaunch<28, 2>::per_sm() : 0;
     if (max_n > 16) return size == 2 ? HashLaunch<20, 2>::per_sm() : size == 1 ? HashLaunch<20, 1>::per_sm() : 0;
     return size == 2 ? HashLaunch<16, 2>::per_sm() : size == 1 ? HashLaunch<16, 1>::per_sm() : 0;
-}
-
-cudaError_t launch_sort_handoff(const Batch &b, const int32_t *list, const unsigned long long *count, int32_t *out,
-                                int top_n, unsigned long long *split, cudaStream_t st)
-{
-    k_sort_handoff<<<1, 1024, 0, st>>>(b, list, count, out, top_n, split);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,

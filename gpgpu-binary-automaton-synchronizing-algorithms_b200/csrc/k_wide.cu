@@ -214,7 +214,249 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     if (lane == 0 && b.expanded && expanded) atomicAdd(b.expanded, expanded);
 }
 
+// ---- n <= 20 -----------------------------------------------------------------
+// The automata of 13..20 states that outgrow a warp (k_hash.cu: 1536 subsets;
+// 0.4 % of random automata at n = 16, 4 % at n = 20).  Same search with the
+// bitmap of k_hash.cu as its visited store -- states relabelled by image,
+// 2^rank(a) + 2^rank(b) bits, 2^17 at most -- and a queue whose first 8192
+// subsets stay on chip: 65 KB, so three CTAs per SM instead of the one that
+// k_cta.cu's 2^20-bit bitmap allows, and no trips to global memory but for the
+// widest searches.  Those continue in a spill of 2^17 entries per CTA, which no
+// search can outgrow: its subsets have different bits.  Ranks that need more bits
+// (n > 16 only) are left to k_cta.  The widest search of a batch bounds the
+// launch, hence 512 threads: 30K random n = 20 took 0.330 ms with k_cta alone,
+// 0.334 with 256 threads here, 0.315 with 512, 0.326 with 1024 (two CTAs per SM);
+// 200K mixed n = 6..20 0.611, 0.599, 0.591 and 0.611 ms.
+constexpr int kMidThreads = 512;
+constexpr uint32_t kMidLimit = 8192;
+constexpr uint32_t kMidSpill = 1u << 17;
+constexpr int kMidWords = 4096;
+constexpr int kMidChunks = 5;
+
+struct MidSmem {
+    uint32_t store[kMidWords];
+    uint64_t table[16 * kMidChunks];
+    uint32_t queue[kMidLimit];      // subset | letter-is-b << 31
+    uint16_t parent[kMidLimit];
+};
+
+struct MidCtl {
+    int64_t k;
+    int n;
+    uint32_t low_end, index0, shift, bits;
+    uint32_t found[2], cnt[3];            // as in WideCtl
+    uint64_t single[32];                  // a's << 32 | b's image of the state with that label
+};
+
+__global__ void __launch_bounds__(kMidThreads, 3)
+    k_mid(const __grid_constant__ Batch b, uint2 *spill_base, int32_t *left_list, unsigned long long *left_count,
+          unsigned long long *ticket)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    MidSmem &S = *reinterpret_cast<MidSmem *>(smem_raw);
+    __shared__ MidCtl ctl;
+    // {subset | letter-is-b << 31, parent} of the queue entries from kMidLimit on
+    uint2 *const spill = spill_base + (size_t)blockIdx.x * kMidSpill;
+    const int tid = threadIdx.x;
+    const int lane = tid & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    int64_t count;
+    const int32_t *order;
+    resolve_work(b, count, order);
+    unsigned long long expanded = 0;
+
+    while (true) {
+        if (tid < 32) {
+            unsigned long long pos = 0;
+            if (lane == 0) pos = atomicAdd(ticket, 1ull);
+            pos = __shfl_sync(kFull, pos, 0);
+            const int64_t k = pos < (unsigned long long)count ? automaton_at(order, (int64_t)pos) : -1;
+            int n = 0;
+            uint32_t av = 0, bv = 0;
+            if (k >= 0) {
+                // the record was checked by the kernel that handed the automaton on
+                n = automaton_n(b, k);
+                const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
+                if (lane < n) {
+                    av = rec[lane] & 31u;
+                    bv = rec[b.lstride + lane] & 31u;
+                }
+            }
+            const uint32_t A = __reduce_or_sync(kFull, lane < n ? 1u << av : 0u);
+            const uint32_t B = __reduce_or_sync(kFull, lane < n ? 1u << bv : 0u);
+            const int ra = __popc(A), rb = __popc(B);
+            const bool in_a = (A >> lane) & 1u, in_b = (B >> lane) & 1u;
+            int label = in_a ? (in_b ? __popc(A & ~B) + __popc(A & B & lt) : __popc(A & ~B & lt))
+                             : (in_b ? ra + __popc(B & ~A & lt) : __popc(A | B) + __popc(~(A | B) & lt));
+            if (lane >= n) label = lane;
+            const int la = __shfl_sync(kFull, label, (int)av), lb = __shfl_sync(kFull, label, (int)bv);
+            ctl.single[label] = lane < n ? ((uint64_t)(1u << la) << 32) | (1u << lb) : 0ull;
+            if (lane == 0) {
+                ctl.k = k;
+                ctl.n = n;
+                uint32_t bits = (1u << ra) + ((B & ~A) ? 1u << rb : 0u);
+                ctl.low_end = ctl.index0 = 1u << ra;
+                ctl.shift = (uint32_t)__popc(A & ~B);
+                if (bits > 1u << n) {
+                    bits = 1u << n;
+                    ctl.index0 = ctl.shift = 0u;
+                }
+                ctl.bits = bits;
+                ctl.found[0] = ctl.found[1] = ~0u;
+                ctl.cnt[0] = ctl.cnt[1] = ctl.cnt[2] = 0u;
+            }
+        }
+        __syncthreads();
+        const int64_t k = ctl.k;
+        if (k < 0) break;
+        const int n = ctl.n;
+        const uint32_t low_end = ctl.low_end, index0 = ctl.index0, shift = ctl.shift, bits = ctl.bits;
+        if (bits > 32u * kMidWords) {
+            if (tid == 0) left_list[atomicAdd(left_count, 1ull)] = (int32_t)k;
+            __syncthreads();   // every thread has read ctl
+            continue;
+        }
+        if (tid < 16 * kMidChunks) {
+            const int c = tid >> 4, v = tid & 15;
+            uint64_t acc = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if ((v >> j) & 1) acc |= ctl.single[4 * c + j];
+            S.table[tid] = acc;
+        }
+        uint4 *store4 = reinterpret_cast<uint4 *>(S.store);
+        for (uint32_t i = tid; i < (bits + 127u) / 128u; i += kMidThreads) store4[i] = make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t full = (1u << n) - 1u;
+        if (tid == 0) S.queue[0] = full;
+        __syncthreads();
+        // the root comes back only through a permutation, and then the index is plain:
+        // the first level sets its bit before any other thread reads the store
+        uint32_t ls = 0, le = n > 1 ? 1u : 0u, level = 0;
+        if (tid == 0 && (index0 == 0u || low_end > full)) S.store[full >> 5] |= 1u << (full & 31u);
+        while (true) {
+            uint32_t *cnt = &ctl.cnt[level % 3];
+            uint32_t *found = &ctl.found[level & 1];
+            if (tid == 0) ctl.cnt[(level + 1) % 3] = 0u;
+            for (uint32_t base = ls + (tid & ~31); base < le; base += kMidThreads) {
+                const uint32_t i = base + lane;
+                uint32_t ya = 0, yb = 0;
+                bool fa = false, fb = false;
+                if (i < le) {
+                    const uint32_t x = (i < kMidLimit ? S.queue[i] : spill[i - kMidLimit].x) & 0x7FFFFFFFu;
+                    uint64_t t = S.table[x & 15u];
+#pragma unroll
+                    for (int c = 1; c < kMidChunks; ++c) t |= S.table[16 * c + ((x >> (4 * c)) & 15u)];
+                    ya = (uint32_t)(t >> 32);
+                    yb = (uint32_t)t;
+                    ++expanded;
+                    // no singleton is visited before the first one is generated
+                    const bool sa = is_singleton(ya), sb = is_singleton(yb);
+                    if (sa || sb) atomicMin(found, (i << 1) | (sa ? 0u : 1u));
+                    const uint32_t ib = yb < low_end ? yb : index0 + (yb >> shift);
+                    if (SBFS_CHECK(ya < 32u * kMidWords && ib < 32u * kMidWords, b.error)) {
+                        const uint32_t ma = 1u << (ya & 31u), mb = 1u << (ib & 31u);
+                        const uint32_t oa = atomicOr(&S.store[ya >> 5], ma);
+                        const uint32_t ob = atomicOr(&S.store[ib >> 5], mb);
+                        fa = !(oa & ma);
+                        fb = !(ob & mb);
+                    }
+                }
+                const unsigned ma = __ballot_sync(kFull, fa), mb = __ballot_sync(kFull, fb);
+                const uint32_t c = (uint32_t)(__popc(ma) + __popc(mb));
+                if (!c) continue;
+                uint32_t pos = 0;
+                if (lane == 0) pos = le + atomicAdd(cnt, c);
+                pos = __shfl_sync(kFull, pos, 0) + __popc(ma & lt) + __popc(mb & lt);
+                // (a parent below kMidLimit fits 16 bits; one past it pushes past it)
+                auto push = [&](uint32_t p, uint32_t e) {
+                    if (p < kMidLimit) {
+                        S.queue[p] = e;
+                        S.parent[p] = (uint16_t)i;
+                    } else if (SBFS_CHECK(p - kMidLimit < kMidSpill, b.error)) {
+                        spill[p - kMidLimit] = make_uint2(e, i);
+                    }
+                };
+                if (fa) push(pos++, ya);
+                if (fb) push(pos, yb | 0x80000000u);
+            }
+            __syncthreads();
+            const uint32_t f = *found, added = *cnt;
+            if (f != ~0u) {
+                if (tid == 0) {
+                    record_result(b, k, n, (int32_t)level + 1);
+                    if (b.out_words) {
+                        uint64_t *w = b.out_words + (size_t)k * (size_t)b.word_stride;
+                        for (int c = 0; c < b.word_stride; ++c) w[c] = 0ull;
+                        if (level < 64u * (uint32_t)b.word_stride) {
+                            w[level >> 6] |= (uint64_t)(f & 1u) << (level & 63u);
+                            uint32_t i = f >> 1;
+                            for (int d = (int)level - 1; d >= 0; --d) {
+                                const uint2 e = i < kMidLimit ? make_uint2(S.queue[i], S.parent[i])
+                                                              : spill[i - kMidLimit];
+                                w[d >> 6] |= (uint64_t)(e.x >> 31) << (d & 63);
+                                i = e.y;
+                            }
+                        }
+                    }
+                    publish_result(b, k);
+                }
+                break;
+            }
+            if (added == 0) {
+                if (tid == 0) {
+                    record_result(b, k, n, kLenNonSync);
+                    if (b.out_words)
+                        for (int c = 0; c < b.word_stride; ++c) b.out_words[(size_t)k * b.word_stride + c] = 0ull;
+                    publish_result(b, k);
+                }
+                break;
+            }
+            ls = le;
+            le += added;
+            ++level;
+        }
+        __syncthreads();
+    }
+    for (int o = 16; o; o >>= 1) expanded += __shfl_down_sync(kFull, expanded, o);
+    if (lane == 0 && b.expanded && expanded) atomicAdd(b.expanded, expanded);
+}
+
+// Dynamic shared memory of a kernel, set once per device: the enqueue paths ask
+// on every launch.
+template <class F>
+cudaError_t allow_smem(F *kernel, size_t bytes, std::atomic<int> (&done)[16])
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool cached = dev >= 0 && dev < 16;
+    if (cached && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && cached) done[dev].store(1, std::memory_order_release);
+    return e;
+}
+
 }  // namespace
+
+// uint64 entries of the spill that launch_mid takes
+size_t mid_spill_entries(int sm_count)
+{
+    return 3 * (size_t)sm_count * kMidSpill;
+}
+
+// Solves the automata of b (n <= 20, three CTAs per SM); those whose ranks need
+// more than 2^17 bits (n > 16) are appended to left_list.
+cudaError_t launch_mid(int sm_count, const Batch &b, uint64_t *spill, int32_t *left_list,
+                       unsigned long long *left_count, unsigned long long *ticket, cudaStream_t st)
+{
+    if (sm_count < 1 || !left_list || !left_count) return cudaErrorInvalidValue;
+    static std::atomic<int> done[16];
+    const cudaError_t e = allow_smem(k_mid, sizeof(MidSmem), done);
+    if (e != cudaSuccess) return e;
+    k_mid<<<3 * sm_count, kMidThreads, sizeof(MidSmem), st>>>(b, reinterpret_cast<uint2 *>(spill), left_list,
+                                                              left_count, ticket);
+    return cudaGetLastError();
+}
 
 // Solves the automata of b (n <= 28, one CTA per SM); those that need more
 // than kWideLimit subsets are appended to left_list.
@@ -222,18 +464,9 @@ cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsign
                         unsigned long long *ticket, cudaStream_t st)
 {
     if (sm_count < 1 || !left_list || !left_count) return cudaErrorInvalidValue;
-    // set once per device: the enqueue paths ask on every launch
-    constexpr int kMaxDevices = 16;
-    static std::atomic<int> done[kMaxDevices];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static std::atomic<int> done[16];
+    const cudaError_t e = allow_smem(k_wide, sizeof(WideSmem), done);
     if (e != cudaSuccess) return e;
-    const bool cached = dev >= 0 && dev < kMaxDevices;
-    if (!cached || !done[dev].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(k_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WideSmem));
-        if (e != cudaSuccess) return e;
-        if (cached) done[dev].store(1, std::memory_order_release);
-    }
     k_wide<<<sm_count, kWideThreads, sizeof(WideSmem), st>>>(b, left_list, left_count, ticket);
     return cudaGetLastError();
 }

@@ -30,17 +30,14 @@ struct DevCounters {
     // escalation list, and claims on it
     unsigned long long escal_count[2];
     unsigned long long escal_claim[2];
-    // per class (pooled warps, hash-set warps): automata handed to the CTA-wide
-    // kernel (class 4: to k_wide), as {offset 0, count} work ranges, and that
-    // kernel's tickets
+    // per class: automata that the warps (pooled, or k_hash) hand on, as
+    // {offset 0, count} work ranges, and the tickets of the kernel that takes them
     unsigned long long heavy_range[kNumClasses][2];
     unsigned long long heavy_ticket[kNumClasses];
-    // class 4: automata k_wide leaves to the level slots
-    unsigned long long wide_range[2];
-    // class 3's sorted hand-offs as two work ranges (n = top, n < top) and the
-    // second launch's tickets
-    unsigned long long heavy_split[4][4];
-    unsigned long long heavy_ticket2[4];
+    // what k_mid (classes 2 and 3) or k_wide (class 4) hands on in turn, to k_cta
+    // or the level slots, and k_cta's tickets
+    unsigned long long left_range[kNumClasses][2];
+    unsigned long long left_ticket[kNumClasses];
     int error;
     int pad;
     unsigned long long synchronizing;             // lengths >= 0 written by this job
@@ -103,7 +100,8 @@ struct Lane {
     cudaStream_t aux[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr};
     DevBuf spill_c[3];                         // queue spill of a pooled class, one per class
-    DevBuf heavy[kNumClasses], heavy_queue[4]; // a class's long searches and their CTA queues
+    // a class's hand-off lists, their CTA queues, and k_mid's spill (classes 2, 3)
+    DevBuf heavy[kNumClasses], heavy_queue[4], mid_spill[2];
     DevBuf maps, ns, len, words, spill, order, counters, ranges, cta_queue, hbm_bitmap, hbm_queue,
         escal, tickets;
     LevelEngine level;                         // device-resident slots for n > 20
@@ -132,7 +130,7 @@ struct Lane {
         uint64_t x = 1469598103934665603ull;
         for (const DevBuf *d : {&maps, &ns, &len, &words, &spill, &order, &counters, &ranges, &cta_queue, &escal,
                                 &tickets, &spill_c[0], &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2],
-                                &heavy[3], &heavy[4], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3]})
+                                &heavy[3], &heavy[4], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3], &mid_spill[0], &mid_spill[1]})
             x = (x ^ reinterpret_cast<uint64_t>(d->ptr)) * 1099511628211ull;
         for (const HostBuf *b : {&h_counters, &h_maps, &h_ns, &h_len, &h_words})
             x = (x ^ reinterpret_cast<uint64_t>(b->ptr)) * 1099511628211ull;
