@@ -94,7 +94,7 @@ namespace {
 
 __global__ void finalize_violation(const DevCounters *c, int64_t *out)
 {
-    *out = c->first_violation == ULLONG_MAX ? -1ll : (int64_t)c->first_violation;
+    *out = (int64_t)~c->first_violation;   // ~0 = -1: none
 }
 
 thread_local std::string g_create_error;
@@ -257,8 +257,23 @@ const LaneShape *uniform_lane(const sbfs_handle *h, const uint8_t *ns, int32_t n
     return nullptr;
 }
 
+int32_t *escal_list(Lane &L)
+{
+    return reinterpret_cast<int32_t *>(L.counters.as<char>() + kCounterBytes);
+}
+
+// Entries of the escalation lists that a job's per-lane kernels need.
+size_t escal_list_entries(const sbfs_handle *h, const Job &j)
+{
+    if (!j.ns)
+        return class_of_n(j.n_uniform) < 2 || uniform_lane(h, j.ns, j.n_uniform)
+                   ? (size_t)std::max<int64_t>(j.count, 1)
+                   : 0;
+    return 2 * (size_t)std::max<int64_t>(j.count, 1);
+}
+
 // Reserve the lane's work buffers for a job and enqueue its kernels on the lane's
-// stream.  Counters must already be reset.
+// stream.  Counters and escalation lists must already be reset.
 sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches, bool plain = false,
                             unsigned long long *ticket_override = nullptr)
 {
@@ -278,6 +293,7 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
     b.word_stride = j.word_stride;
     b.slack = h->cfg.slack;
     b.first_violation = &ctr->first_violation;
+    if (!plain && j.len && !j.done_flag) b.synchronizing = &ctr->synchronizing;
     b.expanded = &ctr->expanded;
     b.error = &ctr->error;
     b.done_flag = j.done_flag;
@@ -289,20 +305,21 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
     const bool fork = j.ns && !plain && __builtin_popcount((unsigned)present) > 1 && L.aux[0];
     bool joined[3] = {false, false, false};
     if (j.ns) {
-        CK(L.order.reserve((size_t)j.count * sizeof(int32_t)), "allocating order array");
-        // hist[K] | ranges[2K] | cursor[K]
-        CK(L.ranges.reserve(4 * kNumClasses * sizeof(unsigned long long)), "allocating class ranges");
-        unsigned long long *r = L.ranges.as<unsigned long long>();
-        ClassScratch sc{r, r + kNumClasses, r + 3 * kNumClasses, L.order.as<int32_t>()};
-        CK(launch_classify(j.ns, j.count, sc, h->sm_count, st), "launching size-class bucketing");
-        *launches += 3;
-        b.order = sc.order;
+        CK(L.order.reserve(kNumClasses * (size_t)j.count * sizeof(int32_t)), "allocating order array");
+        CK(launch_classify(j.ns, j.count, ctr->class_range[0], L.order.as<int32_t>(), h->sm_count, st),
+           "launching size-class bucketing");
+        *launches += 1;
+        b.order = L.order.as<int32_t>();
         if (fork) CK(cudaEventRecord(L.ev_fork, st), "recording event");
     }
-    for (int c = 0; c < kNumClasses; ++c) {
+    // A mixed batch's classes share the SMs, and each kernel's grid fills them: the
+    // largest sizes, whose searches are the longest, go first (with the stream
+    // priorities, see sbfs_create) and the small ones fill in behind them.  200K
+  
+    for (const int c : {3, 2, 1, 0, 4}) {
         if (!(present & (1 << c))) continue;
         Batch bc = b;
-        if (j.ns) bc.range_dev = L.ranges.as<unsigned long long>() + kNumClasses + 2 * c;
+        if (j.ns) bc.range_dev = ctr->class_range[c];
         unsigned long long *ticket = ticket_override ? ticket_override : &ctr->ticket[c];
         cudaStream_t cs = st;
         if (fork && c < 3) {
@@ -314,12 +331,10 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
         const bool lane13 = ul != nullptr;
         if ((c < 2 && !plain && !P.use_pool[c]) || lane13) {
             const LaneShape &ls = lane13 ? *ul : P.lane[c];
-            // one escalation list per lane class (a uniform n = 13 batch has no
-            // class 1 and takes its list and counters); entries read as -1 until stored
+            // one escalation list per lane class, behind the counters and reset with
+            // them (a uniform n = 13 batch has no class 1 and takes its counters)
             const int lc = lane13 ? 1 : c;
-            CK(L.escal.reserve(2 * escal_entries * sizeof(int32_t)), "allocating escalation list");
-            int32_t *list = L.escal.as<int32_t>() + (size_t)lc * escal_entries;
-            CK(cudaMemsetAsync(list, 0xFF, escal_entries * sizeof(int32_t), cs), "resetting escalation list");
+            int32_t *list = escal_list(L) + (j.ns ? (size_t)lc * escal_entries : 0);
             CK(launch_lane(ls.nmax, ls.warps, ls.ring, ls.refill_k, ls.tail_k, ls.ctas, bc, list, escal_entries,
                            &ctr->escal_count[lc], &ctr->escal_claim[lc], ticket, LaneStream{}, cs),
                "launching per-lane kernel");
@@ -427,10 +442,6 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
     }
     for (int c = 0; c < 3; ++c)
         if (joined[c]) CK(cudaStreamWaitEvent(st, L.ev_join[c], 0), "ordering streams");
-    if (!plain && j.len && j.count > 0 && !j.done_flag) {
-        CK(launch_count_sync(j.len, j.count, &ctr->synchronizing, h->sm_count, st), "launching result count");
-        *launches += 1;
-    }
     return SBFS_OK;
 }
 
@@ -556,14 +567,13 @@ sbfs_status check_records(sbfs_handle *h, const uint8_t *maps, int32_t lstride, 
     return SBFS_OK;
 }
 
-sbfs_status reset_counters(sbfs_handle *h, Lane &L)
+// Counters and `entries` escalation-list entries to zero.
+sbfs_status reset_counters(sbfs_handle *h, Lane &L, size_t entries)
 {
-    CK(L.counters.reserve(sizeof(DevCounters)), "allocating counters");
-    CK(cudaMemsetAsync(L.counters.ptr, 0, sizeof(DevCounters), L.stream), "resetting counters");
+    const size_t bytes = kCounterBytes + entries * sizeof(int32_t);
+    CK(L.counters.reserve(bytes), "allocating counters");
+    CK(cudaMemsetAsync(L.counters.ptr, 0, bytes, L.stream), "resetting counters");
     L.level_expanded = 0;
-    CK(cudaMemsetAsync(&L.counters.as<DevCounters>()->first_violation, 0xFF, sizeof(unsigned long long),
-                       L.stream),
-       "resetting counters");
     return SBFS_OK;
 }
 
@@ -586,8 +596,8 @@ sbfs_status finish_lane(sbfs_handle *h, Lane &L, Totals &t)
     t.expanded += (int64_t)(c->expanded + L.level_expanded);
     t.escalated += (int64_t)(c->escal_count[0] + c->escal_count[1]);
     t.synchronizing += (int64_t)c->synchronizing;
-    if (c->first_violation != ULLONG_MAX) {
-        const int64_t g = L.begin + (int64_t)c->first_violation;
+    if (c->first_violation) {
+        const int64_t g = L.begin + (int64_t)~c->first_violation;
         if (t.first_violation < 0 || g < t.first_violation) t.first_violation = g;
     }
     float ms = 0;
@@ -725,9 +735,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     CK(L.maps.reserve(cnt * rec), "allocating records");
     if (out_len) CK(L.len.reserve(cnt * sizeof(int32_t)), "allocating lengths");
     if (out_words) CK(L.words.reserve((size_t)cnt * ws * sizeof(uint64_t)), "allocating words");
-    CK(L.counters.reserve(sizeof(DevCounters)), "allocating counters");
     CK(L.h_counters.reserve(sizeof(DevCounters)), "allocating pinned counters");
-    CK(L.escal.reserve((size_t)cnt * sizeof(int32_t)), "allocating escalation list");
     CK(S.flags.reserve(2 * (size_t)nch * sizeof(unsigned int)), "allocating chunk flags");
     CK(S.escal_out.reserve((size_t)cnt * sizeof(EscalResult)), "allocating escalated results");
     CK(S.h_flags.reserve(3 * (size_t)nch * sizeof(unsigned int)), "allocating host chunk flags");
@@ -789,11 +797,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     CK(cudaEventRecord(S.ev_in0, h->copy_in), "recording event");
     // the kernel, behind chunk 0
     CK(cudaStreamWaitEvent(L.stream, S.ev_in0, 0), "ordering streams");
-    CK(cudaMemsetAsync(L.counters.ptr, 0, sizeof(DevCounters), L.stream), "resetting counters");
-    L.level_expanded = 0;
-    CK(cudaMemsetAsync(&L.counters.as<DevCounters>()->first_violation, 0xFF, sizeof(unsigned long long), L.stream),
-       "resetting counters");
-    CK(cudaMemsetAsync(L.escal.ptr, 0xFF, (size_t)cnt * sizeof(int32_t), L.stream), "resetting escalation list");
+    if ((st = reset_counters(h, L, (size_t)cnt))) return st;
     CK(cudaMemsetAsync(done, 0, nch * sizeof(unsigned int), L.stream), "resetting chunk counts");
     DevCounters *ctr = L.counters.as<DevCounters>();
     Batch b{};
@@ -806,6 +810,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     b.word_stride = out_words ? ws : 0;
     b.slack = h->cfg.slack;
     b.first_violation = &ctr->first_violation;
+    if (out_len) b.synchronizing = &ctr->synchronizing;
     b.expanded = &ctr->expanded;
     b.error = &ctr->error;
     LaneStream lsd = geo;
@@ -815,7 +820,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     lsd.escal_out = S.escal_out.as<EscalResult>();
     lsd.wait_polls = h->cfg.wait_polls > 0 ? h->cfg.wait_polls : (1 << 24);
     CK(cudaEventRecord(L.ev_k0, L.stream), "recording event");
-    CK(launch_lane(ls.nmax, ls.warps, ls.ring, ls.refill_k, ls.tail_k, ls.ctas, b, L.escal.as<int32_t>(),
+    CK(launch_lane(ls.nmax, ls.warps, ls.ring, ls.refill_k, ls.tail_k, ls.ctas, b, escal_list(L),
                    (unsigned long long)cnt, &ctr->escal_count[lc], &ctr->escal_claim[lc], &ctr->ticket[c], lsd,
                    L.stream),
        "launching per-lane kernel");
@@ -869,10 +874,6 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     for (int64_t ci = 1; ci < nch; ++ci) {
         if ((st = poll_out())) return st;
         if ((st = copy_chunk_in(ci))) return st;
-    }
-    if (out_len) {
-        CK(launch_count_sync(b.out_len, cnt, &ctr->synchronizing, h->sm_count, L.stream), "launching result count");
-        o.launches += 1;
     }
     CK(cudaMemcpyAsync(L.h_counters.ptr, L.counters.ptr, sizeof(DevCounters), cudaMemcpyDeviceToHost, L.stream),
        "copying counters");
@@ -960,7 +961,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     o.escalated += esc;
     o.synchronizing += (int64_t)hc->synchronizing;
     o.error |= hc->error;
-    if (hc->first_violation != ULLONG_MAX && o.first_violation < 0) o.first_violation = (int64_t)hc->first_violation;
+    if (hc->first_violation && o.first_violation < 0) o.first_violation = (int64_t)~hc->first_violation;
     float ms = 0;
     if (cudaEventElapsedTime(&ms, L.ev_k0, L.ev_k1) == cudaSuccess) o.kernel_ms += ms;
     cudaGetLastError();
@@ -1095,7 +1096,7 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
         if (!plain) {
             // one chunk: counters, bucketing, class kernels, copies out
             auto body = [&]() -> sbfs_status {
-                sbfs_status bs = reset_counters(h, L);
+                sbfs_status bs = reset_counters(h, L, escal_list_entries(h, j));
                 if (bs) return bs;
                 if ((bs = enqueue_kernels(h, L, j, &launches))) return bs;
                 if (out_len)
@@ -1117,7 +1118,7 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
         } else {
             CK(cudaMemcpyAsync(L.maps.ptr, src_maps, cnt * rec, cudaMemcpyHostToDevice, L.stream), "copying records");
             if (ns) CK(cudaMemcpyAsync(L.ns.ptr, src_ns, cnt, cudaMemcpyHostToDevice, L.stream), "copying sizes");
-            if ((s = reset_counters(h, L))) return s;
+            if ((s = reset_counters(h, L, 0))) return s;
             // one launch per automaton, same kernels, one-CTA grid
             Plan saved = h->plan;
             for (int c = 0; c < 3; ++c) h->plan.pool[c].ctas = 1;
@@ -1198,9 +1199,9 @@ sbfs_status engine_enqueue(sbfs_handle *h, Lane &L, const uint8_t *d_maps, int32
 {
     sbfs_status s = ensure_plan(h);
     if (s) return s;
-    if ((s = reset_counters(h, L))) return s;
     Job j{d_maps, lstride, d_ns, n_uniform, max_n, count, d_len, d_words, d_words ? word_stride : 0, done_flag,
           done_tag};
+    if ((s = reset_counters(h, L, escal_list_entries(h, j)))) return s;
     return enqueue_kernels(h, L, j, launches);
 }
 
@@ -1293,7 +1294,9 @@ sbfs_status sbfs_create(const sbfs_config *cfg, sbfs_handle **out)
             return cuda_fail(nullptr, e, "creating streams");
         }
         for (int c = 0; c < 3; ++c)
-            if ((e = cudaStreamCreateWithPriority(&L.aux[c], cudaStreamNonBlocking, prio)) != cudaSuccess ||
+            // (class 3 runs on the lane's own stream; smaller classes come after it)
+            if ((e = cudaStreamCreateWithPriority(&L.aux[c], cudaStreamNonBlocking,
+                                                  std::min(prio_least, prio + 3 - c))) != cudaSuccess ||
                 (e = cudaEventCreateWithFlags(&L.ev_join[c], cudaEventDisableTiming)) != cudaSuccess) {
                 sbfs_destroy(h);
                 return cuda_fail(nullptr, e, "creating streams");
@@ -1312,8 +1315,8 @@ sbfs_status sbfs_destroy(sbfs_handle *h)
         for (cudaStream_t a : L.aux)
             if (a) cudaStreamSynchronize(a);
         L.drop_graphs();
-        for (DevBuf *d : {&L.maps, &L.ns, &L.len, &L.words, &L.spill, &L.order, &L.counters, &L.ranges,
-                          &L.cta_queue, &L.hbm_bitmap, &L.hbm_queue, &L.escal, &L.tickets})
+        for (DevBuf *d : {&L.maps, &L.ns, &L.len, &L.words, &L.spill, &L.order, &L.counters,
+                          &L.cta_queue, &L.hbm_bitmap, &L.hbm_queue, &L.tickets})
             d->release();
         for (HostBuf *b : {&L.h_counters, &L.h_maps, &L.h_ns, &L.h_len, &L.h_words}) b->release();
         if (L.ev_k0) cudaEventDestroy(L.ev_k0);
@@ -1434,7 +1437,7 @@ sbfs_status sbfs_solve_batch_device(sbfs_handle *h, const uint8_t *d_maps, int32
     int launches = 0;
     // counters, bucketing, class kernels, the violation index, counters back to the host
     auto body = [&]() -> sbfs_status {
-        sbfs_status bs = reset_counters(h, L);
+        sbfs_status bs = reset_counters(h, L, escal_list_entries(h, j));
         if (bs) return bs;
         if (count > 0 && (bs = enqueue_kernels(h, L, j, &launches))) return bs;
         launches += 1;

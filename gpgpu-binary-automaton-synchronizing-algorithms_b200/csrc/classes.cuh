@@ -24,17 +24,9 @@ __host__ __device__ __forceinline__ int class_of_n(int n)
     return (n >= 1 && n <= 8) ? 0 : n <= 12 ? 1 : n <= 16 ? 2 : n <= 20 ? 3 : n <= 28 ? 4 : 0;
 }
 
-struct ClassScratch {
-    unsigned long long *hist;     // kNumClasses
-    unsigned long long *ranges;   // 2 * kNumClasses: {offset, count}
-    unsigned long long *cursor;   // kNumClasses
-    int32_t *order;               // count entries
-};
-
-// Adds the number of non-negative lengths in len[0..count) to *out.
-cudaError_t launch_count_sync(const int32_t *d_len, int64_t count, unsigned long long *out, int sm_count,
-                              cudaStream_t st);
-cudaError_t launch_classify(const uint8_t *d_ns, int64_t count, ClassScratch sc, int sm_count,
-                            cudaStream_t st);
+// Buckets d_ns[0..count): ranges[2 * c], ranges[2 * c + 1] = class c's offset into
+// order (kNumClasses * count entries) and its members.  The counts start at 0.
+cudaError_t launch_classify(const uint8_t *d_ns, int64_t count, unsigned long long *ranges, int32_t *order,
+                            int sm_count, cudaStream_t st);
 
 }  // namespace sbfs

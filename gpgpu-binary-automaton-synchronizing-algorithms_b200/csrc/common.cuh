@@ -46,7 +46,10 @@ struct Batch {
     uint64_t *out_words;        // nullable
     int32_t word_stride;
     int32_t slack;
-    unsigned long long *first_violation;   // atomicMin target, starts at ULLONG_MAX
+    // complement of the smallest violating index: an atomicMax target that starts
+    // at 0, so that one memset resets every counter
+    unsigned long long *first_violation;
+    unsigned long long *synchronizing;     // stats counter: results with a length >= 0 (nullable)
     unsigned long long *expanded;          // stats counter (nullable)
     int *error;                            // error bits
     // Per-automaton completion (serving): after an automaton's length and
@@ -101,8 +104,8 @@ __device__ __forceinline__ void publish_result(const Batch &b, int64_t k)
 __device__ __forceinline__ void record_result(const Batch &b, int64_t k, int n, int32_t len)
 {
     if (b.out_len) b.out_len[k] = len;
-    if (len > cerny_bound(n, b.slack))
-        atomicMin(b.first_violation, (unsigned long long)k);
+    if (len >= 0 && b.synchronizing) atomicAdd(b.synchronizing, 1ull);
+    if (len > cerny_bound(n, b.slack)) atomicMax(b.first_violation, ~(unsigned long long)k);
 }
 
 // Host-side launch helpers implemented in the kernel translation units.
@@ -176,7 +179,8 @@ cudaError_t launch_escal_patch(const EscalResult *r, const unsigned long long *c
                                int ws, int sm_count, cudaStream_t st);
 
 // escal_list holds escal_capacity entries (>= the automata of the launch), all
-// -1; escal_count and escal_claim start at 0.
+// 0 (an entry: automaton + 1, or -1 when given up on); escal_count and
+// escal_claim start at 0.
 // tail_k: once the batch is handed out, lanes of a warp with at most tail_k
 // lanes still searching give their automata to the whole-warp search (0 = off).
 cudaError_t launch_lane(int nmax, int warps, int ring, int refill_k, int tail_k, int ctas, const Batch &b,

@@ -214,8 +214,8 @@ __device__ __forceinline__ void load_maps(const Batch &b, int64_t k, int n, int6
 // Claims the next escalated automaton of the launch for a warp with no lane
 // work left, or returns -1.  A claim is one atomicAdd on the claim counter and
 // one atomicCAS on the claimed slot, raced against the slot's writer (which
-// stores with atomicCAS too): if the slot is still empty the claimer marks it
-// abandoned (-2) and stops, and the writer, finding it abandoned, keeps the
+// stores with atomicCAS too): if the slot is still empty (0) the claimer marks it
+// abandoned (-1) and stops, and the writer, finding it abandoned, keeps the
 // automaton and solves it itself once it runs out of lane work.  Nothing ever
 // waits for another warp.
 __device__ int64_t claim_escalated(int32_t *list, unsigned long long capacity, unsigned long long *claim,
@@ -223,8 +223,8 @@ __device__ int64_t claim_escalated(int32_t *list, unsigned long long capacity, u
 {
     slot = atomicAdd(claim, 1ull);
     if (slot >= capacity) return -1;
-    const int32_t prev = atomicCAS(list + slot, -1, -2);
-    return prev >= 0 ? (int64_t)prev : -1;
+    const int32_t prev = atomicCAS(list + slot, 0, -1);
+    return (int64_t)prev - 1;   // an empty slot: -1
 }
 
 // One automaton (n <= NMAX) solved by the whole warp inside its region of
@@ -458,9 +458,9 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     // a slot a drained warp already gave up on: solve this one ourselves later
                     const unsigned long long slot = pos + __popc(esc & ((1u << lane) - 1u));
                     const int32_t prev = SBFS_CHECK(slot < escal_capacity, b.error)
-                                             ? atomicCAS(escal_list + slot, -1, (int32_t)k)
-                                             : -2;
-                    state = prev == -1 ? kIdle : kHeld;
+                                             ? atomicCAS(escal_list + slot, 0, (int32_t)k + 1)
+                                             : -1;
+                    state = prev == 0 ? kIdle : kHeld;
                     hslot = slot;
                 }
             }

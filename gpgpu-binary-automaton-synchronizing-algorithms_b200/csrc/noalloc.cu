@@ -37,7 +37,7 @@ constexpr size_t kHeaderBytes = 256;
 
 struct NoAllocHeader {
     unsigned long long ticket;
-    unsigned long long first_violation;
+    unsigned long long first_violation;   // complement of the index, 0 = none
     unsigned long long expanded;
     int error;
 };
@@ -54,7 +54,7 @@ constexpr int kCtas = (int)((kScratchBytes - kHeaderBytes) / (kSpillPerSlot * 4 
 
 __global__ void finalize(const NoAllocHeader *hdr, int64_t *out)
 {
-    *out = hdr->first_violation == ~0ull ? -1ll : (int64_t)hdr->first_violation;
+    *out = (int64_t)~hdr->first_violation;   // ~0 = -1: none
 }
 
 // Device address of g_scratch in the current device's context.  In host code
@@ -92,8 +92,7 @@ extern "C" sbfs_status sbfs_solve_small_noalloc(const uint8_t *d_maps, int32_t l
     NoAllocHeader *hdr = reinterpret_cast<NoAllocHeader *>(scratch);
     uint32_t *spill = reinterpret_cast<uint32_t *>(scratch + kHeaderBytes);
     // the array keeps the previous call's contents: reset the counters
-    if (cudaMemsetAsync(hdr, 0, sizeof(NoAllocHeader), st) != cudaSuccess ||
-        cudaMemsetAsync(&hdr->first_violation, 0xFF, sizeof(unsigned long long), st) != cudaSuccess) {
+    if (cudaMemsetAsync(hdr, 0, sizeof(NoAllocHeader), st) != cudaSuccess) {
         cudaGetLastError();
         return SBFS_ECUDA;
     }

@@ -24,7 +24,8 @@ namespace sbfs {
 // Counters one launch sequence reads and writes on the device.
 struct DevCounters {
     unsigned long long ticket[kNumClasses + 1];   // per-class work tickets (last one spare)
-    unsigned long long first_violation;
+    unsigned long long class_range[kNumClasses][2];   // a mixed batch's classes: {offset, count} of the order array
+    unsigned long long first_violation;   // complement of the index, 0 = none
     unsigned long long expanded;
     // per-lane kernels of classes 0 and 1: automata appended to the class's
     // escalation list, and claims on it
@@ -42,6 +43,9 @@ struct DevCounters {
     int pad;
     unsigned long long synchronizing;             // lengths >= 0 written by this job
 };
+
+// A lane's counters, and the escalation lists behind them: one memset resets both.
+constexpr size_t kCounterBytes = (sizeof(DevCounters) + 255) & ~(size_t)255;
 
 // Grow-only device allocation.
 struct DevBuf {
@@ -102,8 +106,8 @@ struct Lane {
     DevBuf spill_c[3];                         // queue spill of a pooled class, one per class
     // a class's hand-off lists, their CTA queues, and k_mid's spill (classes 2, 3)
     DevBuf heavy[kNumClasses], heavy_queue[4], mid_spill[2];
-    DevBuf maps, ns, len, words, spill, order, counters, ranges, cta_queue, hbm_bitmap, hbm_queue,
-        escal, tickets;
+    DevBuf maps, ns, len, words, spill, order, counters, cta_queue, hbm_bitmap, hbm_queue,
+        tickets;
     LevelEngine level;                         // device-resident slots for n > 20
     bool level_ready = false;
     unsigned long long level_expanded = 0;     // subsets the level slots expanded for the current job
@@ -128,8 +132,8 @@ struct Lane {
     uint64_t signature() const
     {
         uint64_t x = 1469598103934665603ull;
-        for (const DevBuf *d : {&maps, &ns, &len, &words, &spill, &order, &counters, &ranges, &cta_queue, &escal,
-                                &tickets, &spill_c[0], &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2],
+        for (const DevBuf *d : {&maps, &ns, &len, &words, &spill, &order, &counters, &cta_queue, &tickets,
+                                &spill_c[0], &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2],
                                 &heavy[3], &heavy[4], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3], &mid_spill[0], &mid_spill[1]})
             x = (x ^ reinterpret_cast<uint64_t>(d->ptr)) * 1099511628211ull;
         for (const HostBuf *b : {&h_counters, &h_maps, &h_ns, &h_len, &h_words})
