@@ -251,6 +251,7 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
                 break;
             }
             const int pa = ya ? set_find(W, ya) : -1, pb = yb && yb != ya ? set_find(W, yb) : -1;
+            __syncwarp();   // every lane has probed before lane 0 writes
             if (pa < 0 && pb < 0) {
                 width = 0;
                 break;
