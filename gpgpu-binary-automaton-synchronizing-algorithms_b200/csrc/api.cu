@@ -105,6 +105,10 @@ constexpr int kDefaultLanes = 4;
 // samples at n = 20), a Cerny automaton needs (n-1)^2
 constexpr int kPoolLevelCap = 48;
 constexpr int64_t kDefaultChunk = 1 << 18;
+// A pageable caller's single chunk whose results fit this many bytes has them
+// behind its counters on the device, reset with one memset and read back with
+// one copy: each of the three it replaces costs a small batch 2 to 3 us.
+constexpr size_t kFusedBytes = 1 << 20;
 
 sbfs_status fail(sbfs_handle *h, sbfs_status st, const std::string &msg)
 {
@@ -259,7 +263,21 @@ const LaneShape *uniform_lane(const sbfs_handle *h, const uint8_t *ns, int32_t n
 
 int32_t *escal_list(Lane &L)
 {
-    return reinterpret_cast<int32_t *>(L.counters.as<char>() + kCounterBytes);
+    return reinterpret_cast<int32_t *>(L.counters.as<char>() + L.list_off);
+}
+
+// CTAs and warps per CTA of a per-lane kernel for `count` automata: of a small
+// batch only as many warps as have automata, spread over the SMs.  Warps without
+// any would only give up escalation slots ahead of the warps that fill them,
+// which then keep those automata to themselves (10,000 n = 8: 1252 of them).
+void lane_grid(const LaneShape &ls, int64_t count, int sm_count, int &warps, int &ctas)
+{
+    warps = ls.warps;
+    ctas = ls.ctas;
+    const int64_t need = std::max<int64_t>(1, (count + 31) / 32);
+    if (need >= (int64_t)warps * ctas) return;
+    while (warps > 1 && need <= (int64_t)warps * sm_count) warps /= 2;
+    ctas = (int)std::min<int64_t>((int64_t)ctas * ls.warps / warps, (need + warps - 1) / warps);
 }
 
 // Entries of the escalation lists that a job's per-lane kernels need.
@@ -335,7 +353,9 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
             // them (a uniform n = 13 batch has no class 1 and takes its counters)
             const int lc = lane13 ? 1 : c;
             int32_t *list = escal_list(L) + (j.ns ? (size_t)lc * escal_entries : 0);
-            CK(launch_lane(ls.nmax, ls.warps, ls.ring, ls.refill_k, ls.tail_k, ls.ctas, bc, list, escal_entries,
+            int warps, ctas;
+            lane_grid(ls, j.count, h->sm_count, warps, ctas);
+            CK(launch_lane(ls.nmax, warps, ls.ring, ls.refill_k, ls.tail_k, ctas, bc, list, escal_entries,
                            &ctr->escal_count[lc], &ctr->escal_claim[lc], ticket, LaneStream{}, cs),
                "launching per-lane kernel");
         } else if ((c == 2 && P.class2_hash && !plain && !ticket_override) ||
@@ -360,7 +380,8 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                 // left by k_hash | left by k_mid
                 CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off lists");
                 int32_t *list = L.heavy[c].as<int32_t>();
-                CK(launch_hash(size, kClassMaxN[c], hper * h->sm_count, bc, list, &ctr->heavy_range[c][1], ticket, cs),
+                const int hctas = (int)std::min<int64_t>(hper * h->sm_count, std::max<int64_t>(j.count, 1));
+                CK(launch_hash(size, kClassMaxN[c], hctas, bc, list, &ctr->heavy_range[c][1], ticket, cs),
                    "launching hash-set kernel");
                 Batch bh = bc;
                 bh.order = list;
@@ -422,7 +443,8 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                 if (hper < 1) return fail(h, SBFS_ECUDA, "hash-set kernel does not fit on an SM");
                 CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off list");
                 int32_t *list = L.heavy[c].as<int32_t>();
-                CK(launch_hash(2, SBFS_MAX_N, hper * h->sm_count, bc, list, &ctr->heavy_range[c][1], ticket, cs),
+                const int hctas = (int)std::min<int64_t>(hper * h->sm_count, std::max<int64_t>(j.count, 1));
+                CK(launch_hash(2, SBFS_MAX_N, hctas, bc, list, &ctr->heavy_range[c][1], ticket, cs),
                    "launching hash-set kernel");
                 bc.order = list;
                 bc.range_dev = ctr->heavy_range[c];
@@ -567,10 +589,12 @@ sbfs_status check_records(sbfs_handle *h, const uint8_t *maps, int32_t lstride, 
     return SBFS_OK;
 }
 
-// Counters and `entries` escalation-list entries to zero.
-sbfs_status reset_counters(sbfs_handle *h, Lane &L, size_t entries)
+// Counters, `between` bytes of results behind them and `entries` escalation-list
+// entries to zero.
+sbfs_status reset_counters(sbfs_handle *h, Lane &L, size_t entries, size_t between = 0)
 {
-    const size_t bytes = kCounterBytes + entries * sizeof(int32_t);
+    L.list_off = kCounterBytes + between;
+    const size_t bytes = L.list_off + entries * sizeof(int32_t);
     CK(L.counters.reserve(bytes), "allocating counters");
     CK(cudaMemsetAsync(L.counters.ptr, 0, bytes, L.stream), "resetting counters");
     L.level_expanded = 0;
@@ -590,7 +614,7 @@ sbfs_status finish_lane(sbfs_handle *h, Lane &L, Totals &t)
 {
     if (!L.busy) return SBFS_OK;
     L.busy = false;
-    CK(cudaEventSynchronize(L.ev_done), "waiting for a chunk");
+    CK(cudaEventSynchronize(L.ev_end), "waiting for a chunk");
     const DevCounters *c = L.h_counters.as<DevCounters>();
     t.error |= c->error;
     t.expanded += (int64_t)(c->expanded + L.level_expanded);
@@ -603,11 +627,12 @@ sbfs_status finish_lane(sbfs_handle *h, Lane &L, Totals &t)
     float ms = 0;
     if (cudaEventElapsedTime(&ms, L.ev_k0, L.ev_k1) == cudaSuccess) t.kernel_ms += ms;
     cudaGetLastError();
-    if (L.staged_out) {
+    if (L.staged_len || L.staged_words) {
         CopyPool::Group g;
-        if (L.user_len) h->copy_pool().copy(L.user_len + L.begin, L.h_len.ptr, (size_t)L.count * sizeof(int32_t), g);
-        if (L.user_words)
-            h->copy_pool().copy(L.user_words + (size_t)L.begin * L.word_stride, L.h_words.ptr,
+        if (L.staged_len)
+            h->copy_pool().copy(L.user_len + L.begin, L.staged_len, (size_t)L.count * sizeof(int32_t), g);
+        if (L.staged_words)
+            h->copy_pool().copy(L.user_words + (size_t)L.begin * L.word_stride, L.staged_words,
                                 (size_t)L.count * L.word_stride * sizeof(uint64_t), g);
         h->copy_pool().wait(g);
     }
@@ -1040,70 +1065,96 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
         Lane &L = h->lanes[ci % nlanes];
         if ((s = finish_lane(h, L, tot))) return s;
         const int64_t cnt = std::min(chunk, count - begin);
-        CK(L.maps.reserve(cnt * rec), "allocating records");
-        if (ns) CK(L.ns.reserve(cnt), "allocating sizes");
-        if (out_len) CK(L.len.reserve(cnt * sizeof(int32_t)), "allocating lengths");
-        if (out_words) CK(L.words.reserve(cnt * word_stride * sizeof(uint64_t)), "allocating words");
-        CK(L.h_counters.reserve(sizeof(DevCounters)), "allocating pinned counters");
+        const bool only = !plain && count <= chunk;   // the call's only chunk
+        const size_t lb = out_len ? (size_t)cnt * sizeof(int32_t) : 0;
+        const size_t wb = out_words ? (size_t)cnt * word_stride * sizeof(uint64_t) : 0;
+        const size_t off_words = kCounterBytes + ((lb + 255) & ~(size_t)255);
+        const size_t fused_end = off_words + ((wb + 255) & ~(size_t)255);
+        const bool fused = only && !pin_out && fused_end <= kFusedBytes;
+        const size_t off_ns = (cnt * rec + 255) & ~(size_t)255;   // sizes behind the records
+        CK(L.maps.reserve(off_ns + (ns ? cnt : 0)), "allocating records");
+        int32_t *d_len = nullptr;
+        uint64_t *d_words = nullptr;
+        if (fused) {
+            CK(L.counters.reserve(fused_end + 2 * (size_t)cnt * sizeof(int32_t)), "allocating results");
+            CK(L.h_counters.reserve(fused_end), "allocating pinned staging");
+            if (out_len) d_len = reinterpret_cast<int32_t *>(L.counters.as<char>() + kCounterBytes);
+            if (out_words) d_words = reinterpret_cast<uint64_t *>(L.counters.as<char>() + off_words);
+        } else {
+            if (out_len) CK(L.len.reserve(lb), "allocating lengths");
+            if (out_words) CK(L.words.reserve(wb), "allocating words");
+            if (out_len) d_len = L.len.as<int32_t>();
+            if (out_words) d_words = L.words.as<uint64_t>();
+            CK(L.h_counters.reserve(sizeof(DevCounters)), "allocating pinned counters");
+        }
         const uint8_t *src_maps = maps + begin * rec;
         const uint8_t *src_ns = ns ? ns + begin : nullptr;
         if (!pin_in) {
-            CK(L.h_maps.reserve(cnt * rec), "allocating pinned staging");
-            if (ns) CK(L.h_ns.reserve(cnt), "allocating pinned staging");
+            CK(L.h_maps.reserve(off_ns + (ns ? cnt : 0)), "allocating pinned staging");
             CopyPool::Group g;
             h->copy_pool().copy(L.h_maps.ptr, src_maps, cnt * rec, g);
             src_maps = L.h_maps.as<uint8_t>();
             if (ns) {
-                h->copy_pool().copy(L.h_ns.ptr, src_ns, cnt, g);
-                src_ns = L.h_ns.as<uint8_t>();
+                h->copy_pool().copy(L.h_maps.as<uint8_t>() + off_ns, src_ns, cnt, g);
+                src_ns = L.h_maps.as<uint8_t>() + off_ns;
             }
             h->copy_pool().wait(g);
         }
-        L.staged_out = !pin_out;
         L.user_len = out_len;
         L.user_words = out_words;
         L.word_stride = word_stride;
-        void *dst_len = nullptr, *dst_words = nullptr;
-        const size_t wb = out_words ? (size_t)cnt * word_stride * sizeof(uint64_t) : 0;
-        if (out_len) {
-            dst_len = pin_out ? (void *)(out_len + begin) : nullptr;
-            if (!pin_out) {
-                CK(L.h_len.reserve(cnt * sizeof(int32_t)), "allocating pinned staging");
-                dst_len = L.h_len.ptr;
+        L.staged_len = L.staged_words = nullptr;
+        void *dst_len = out_len ? (void *)(out_len + begin) : nullptr;
+        void *dst_words = out_words ? (void *)(out_words + (size_t)begin * word_stride) : nullptr;
+        if (fused) {
+            if (out_len) L.staged_len = dst_len = L.h_counters.as<char>() + kCounterBytes;
+            if (out_words) L.staged_words = dst_words = L.h_counters.as<char>() + off_words;
+        } else if (!pin_out) {
+            if (out_len) {
+                CK(L.h_len.reserve(lb), "allocating pinned staging");
+                L.staged_len = dst_len = L.h_len.ptr;
             }
-        }
-        if (out_words) {
-            dst_words = pin_out ? (void *)(out_words + (size_t)begin * word_stride) : nullptr;
-            if (!pin_out) {
+            if (out_words) {
                 CK(L.h_words.reserve(wb), "allocating pinned staging");
-                dst_words = L.h_words.ptr;
+                L.staged_words = dst_words = L.h_words.ptr;
             }
         }
-        Job j{L.maps.as<uint8_t>(), lstride, ns ? L.ns.as<uint8_t>() : nullptr, n_uniform, max_n, cnt,
-              out_len ? L.len.as<int32_t>() : nullptr, out_words ? L.words.as<uint64_t>() : nullptr,
-              word_stride};
+        Job j{L.maps.as<uint8_t>(), lstride, ns ? L.maps.as<uint8_t>() + off_ns : nullptr, n_uniform, max_n, cnt,
+              d_len, d_words, word_stride};
         h2d += cnt * rec + (ns ? cnt : 0);
         d2h += (out_len ? cnt * (int64_t)sizeof(int32_t) : 0) + (int64_t)wb;
         if (!plain) {
-            // records in on the shared copy stream (chunk order), then the lane waits for them
-            CK(cudaMemcpyAsync(L.maps.ptr, src_maps, cnt * rec, cudaMemcpyHostToDevice, h->copy_in),
+            // records in on the shared copy stream (chunk order), then the lane waits for
+            // them; a single chunk's on the lane's own stream
+            cudaStream_t in = only ? L.stream : h->copy_in;
+            const bool one = ns && !pin_in;   // staged side by side: one copy
+            CK(cudaMemcpyAsync(L.maps.ptr, src_maps, one ? off_ns + cnt : cnt * rec, cudaMemcpyHostToDevice, in),
                "copying records");
-            if (ns) CK(cudaMemcpyAsync(L.ns.ptr, src_ns, cnt, cudaMemcpyHostToDevice, h->copy_in), "copying sizes");
-            CK(cudaEventRecord(L.ev_in, h->copy_in), "recording event");
-            CK(cudaStreamWaitEvent(L.stream, L.ev_in, 0), "ordering streams");
+            if (ns && !one)
+                CK(cudaMemcpyAsync(L.maps.as<uint8_t>() + off_ns, src_ns, cnt, cudaMemcpyHostToDevice, in),
+                   "copying sizes");
+            if (!only) {
+                CK(cudaEventRecord(L.ev_in, h->copy_in), "recording event");
+                CK(cudaStreamWaitEvent(L.stream, L.ev_in, 0), "ordering streams");
+            }
         }
         CK(cudaEventRecord(L.ev_k0, L.stream), "recording event");
         if (!plain) {
             // one chunk: counters, bucketing, class kernels, copies out
             auto body = [&]() -> sbfs_status {
-                sbfs_status bs = reset_counters(h, L, escal_list_entries(h, j));
+                sbfs_status bs =
+                    reset_counters(h, L, escal_list_entries(h, j), fused ? fused_end - kCounterBytes : 0);
                 if (bs) return bs;
                 if ((bs = enqueue_kernels(h, L, j, &launches))) return bs;
+                if (fused) {
+                    CK(cudaMemcpyAsync(L.h_counters.ptr, L.counters.ptr, fused_end, cudaMemcpyDeviceToHost, L.stream),
+                       "copying results");
+                    return SBFS_OK;
+                }
                 if (out_len)
-                    CK(cudaMemcpyAsync(dst_len, L.len.ptr, cnt * sizeof(int32_t), cudaMemcpyDeviceToHost, L.stream),
-                       "copying lengths");
+                    CK(cudaMemcpyAsync(dst_len, d_len, lb, cudaMemcpyDeviceToHost, L.stream), "copying lengths");
                 if (out_words)
-                    CK(cudaMemcpyAsync(dst_words, L.words.ptr, wb, cudaMemcpyDeviceToHost, L.stream), "copying words");
+                    CK(cudaMemcpyAsync(dst_words, d_words, wb, cudaMemcpyDeviceToHost, L.stream), "copying words");
                 CK(cudaMemcpyAsync(L.h_counters.ptr, L.counters.ptr, sizeof(DevCounters), cudaMemcpyDeviceToHost,
                                    L.stream),
                    "copying counters");
@@ -1117,7 +1168,9 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
             CK(cudaEventRecord(L.ev_k1, L.stream), "recording event");
         } else {
             CK(cudaMemcpyAsync(L.maps.ptr, src_maps, cnt * rec, cudaMemcpyHostToDevice, L.stream), "copying records");
-            if (ns) CK(cudaMemcpyAsync(L.ns.ptr, src_ns, cnt, cudaMemcpyHostToDevice, L.stream), "copying sizes");
+            if (ns)
+                CK(cudaMemcpyAsync(L.maps.as<uint8_t>() + off_ns, src_ns, cnt, cudaMemcpyHostToDevice, L.stream),
+                   "copying sizes");
             if ((s = reset_counters(h, L, 0))) return s;
             // one launch per automaton, same kernels, one-CTA grid
             Plan saved = h->plan;
@@ -1148,15 +1201,15 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
             h->plan = saved;
             CK(cudaEventRecord(L.ev_k1, L.stream), "recording event");
             if (out_len)
-                CK(cudaMemcpyAsync(dst_len, L.len.ptr, cnt * sizeof(int32_t), cudaMemcpyDeviceToHost, L.stream),
-                   "copying lengths");
+                CK(cudaMemcpyAsync(dst_len, d_len, lb, cudaMemcpyDeviceToHost, L.stream), "copying lengths");
             if (out_words)
-                CK(cudaMemcpyAsync(dst_words, L.words.ptr, wb, cudaMemcpyDeviceToHost, L.stream), "copying words");
+                CK(cudaMemcpyAsync(dst_words, d_words, wb, cudaMemcpyDeviceToHost, L.stream), "copying words");
             CK(cudaMemcpyAsync(L.h_counters.ptr, L.counters.ptr, sizeof(DevCounters), cudaMemcpyDeviceToHost,
                                L.stream),
                "copying counters");
         }
-        CK(cudaEventRecord(L.ev_done, L.stream), "recording event");
+        L.ev_end = plain ? L.ev_done : L.ev_k1;
+        if (plain) CK(cudaEventRecord(L.ev_done, L.stream), "recording event");
         L.busy = true;
         L.begin = begin;
         L.count = cnt;
@@ -1315,10 +1368,10 @@ sbfs_status sbfs_destroy(sbfs_handle *h)
         for (cudaStream_t a : L.aux)
             if (a) cudaStreamSynchronize(a);
         L.drop_graphs();
-        for (DevBuf *d : {&L.maps, &L.ns, &L.len, &L.words, &L.spill, &L.order, &L.counters,
+        for (DevBuf *d : {&L.maps, &L.len, &L.words, &L.spill, &L.order, &L.counters,
                           &L.cta_queue, &L.hbm_bitmap, &L.hbm_queue, &L.tickets})
             d->release();
-        for (HostBuf *b : {&L.h_counters, &L.h_maps, &L.h_ns, &L.h_len, &L.h_words}) b->release();
+        for (HostBuf *b : {&L.h_counters, &L.h_maps, &L.h_len, &L.h_words}) b->release();
         if (L.ev_k0) cudaEventDestroy(L.ev_k0);
         if (L.ev_k1) cudaEventDestroy(L.ev_k1);
         if (L.ev_done) cudaEventDestroy(L.ev_done);

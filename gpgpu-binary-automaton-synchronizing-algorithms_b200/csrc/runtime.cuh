@@ -45,6 +45,7 @@ struct DevCounters {
 };
 
 // A lane's counters, and the escalation lists behind them: one memset resets both.
+// (A small staged batch has its results between the two, see kFusedBytes.)
 constexpr size_t kCounterBytes = (sizeof(DevCounters) + 255) & ~(size_t)255;
 
 // Grow-only device allocation.
@@ -98,6 +99,8 @@ struct CtaShape {
 struct Lane {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr, ev_done = nullptr;
+    cudaEvent_t ev_end = nullptr;              // the one of them that ends the chunk's work
+    size_t list_off = kCounterBytes;           // escalation lists in `counters`
     cudaEvent_t ev_in = nullptr;               // this lane's records have arrived (host path)
     // a mixed batch's size classes 0..2 run on these, beside class 3 on `stream`
     // (their tails -- a Cerny C_16 or C_20 each -- then overlap instead of adding up)
@@ -106,17 +109,17 @@ struct Lane {
     DevBuf spill_c[3];                         // queue spill of a pooled class, one per class
     // a class's hand-off lists, their CTA queues, and k_mid's spill (classes 2, 3)
     DevBuf heavy[kNumClasses], heavy_queue[4], mid_spill[2];
-    DevBuf maps, ns, len, words, spill, order, counters, cta_queue, hbm_bitmap, hbm_queue,
+    DevBuf maps, len, words, spill, order, counters, cta_queue, hbm_bitmap, hbm_queue,
         tickets;
     LevelEngine level;                         // device-resident slots for n > 20
     bool level_ready = false;
     unsigned long long level_expanded = 0;     // subsets the level slots expanded for the current job
     HostBuf h_counters;                        // pinned copy of DevCounters
-    HostBuf h_maps, h_ns, h_len, h_words;      // pinned staging for pageable callers
+    HostBuf h_maps, h_len, h_words;      // pinned staging for pageable callers
     // chunk bookkeeping
     bool busy = false;
     int64_t begin = 0, count = 0;
-    bool staged_out = false;
+    const void *staged_len = nullptr, *staged_words = nullptr;   // pinned results of a pageable caller
     int32_t *user_len = nullptr;
     uint64_t *user_words = nullptr;
     int32_t word_stride = 0;
@@ -132,11 +135,11 @@ struct Lane {
     uint64_t signature() const
     {
         uint64_t x = 1469598103934665603ull;
-        for (const DevBuf *d : {&maps, &ns, &len, &words, &spill, &order, &counters, &cta_queue, &tickets,
+        for (const DevBuf *d : {&maps, &len, &words, &spill, &order, &counters, &cta_queue, &tickets,
                                 &spill_c[0], &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2],
                                 &heavy[3], &heavy[4], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3], &mid_spill[0], &mid_spill[1]})
             x = (x ^ reinterpret_cast<uint64_t>(d->ptr)) * 1099511628211ull;
-        for (const HostBuf *b : {&h_counters, &h_maps, &h_ns, &h_len, &h_words})
+        for (const HostBuf *b : {&h_counters, &h_maps, &h_len, &h_words})
             x = (x ^ reinterpret_cast<uint64_t>(b->ptr)) * 1099511628211ull;
         return x;
     }
