@@ -94,12 +94,18 @@ struct __align__(16) HashWarp {
     }
 };
 
+template <int MAXN, int SIZE>
+__device__ __forceinline__ uint32_t set_slot(uint32_t x)
+{
+    return (x * 0x9E3779B1u) >> HashGeom<MAXN, SIZE>::kSetShift;
+}
+
 // Inserts subset x into the store as a hash set; false when it was there.
 template <int MAXN, int SIZE>
 __device__ __forceinline__ bool set_insert(HashWarp<MAXN, SIZE> &W, uint32_t x)
 {
     using G = HashGeom<MAXN, SIZE>;
-    uint32_t p = (x * 0x9E3779B1u) >> G::kSetShift;
+    uint32_t p = set_slot<MAXN, SIZE>(x);
     for (int probe = 0; probe < G::kWords; ++probe) {
         uint32_t v = W.store[p];
         if (v == 0u) {
@@ -110,22 +116,6 @@ __device__ __forceinline__ bool set_insert(HashWarp<MAXN, SIZE> &W, uint32_t x)
         p = (p + 1) & (G::kWords - 1);
     }
     return false;   // unreachable: the set is never more than ~3/4 full
-}
-
-// The free slot where subset x would go, or -1 when it is in the set: every
-// lane of the warp looks up the same x.
-template <int MAXN, int SIZE>
-__device__ __forceinline__ int set_find(const HashWarp<MAXN, SIZE> &W, uint32_t x)
-{
-    using G = HashGeom<MAXN, SIZE>;
-    uint32_t p = (x * 0x9E3779B1u) >> G::kSetShift;
-    for (int probe = 0; probe < G::kWords; ++probe) {
-        const uint32_t v = W.store[p];
-        if (v == 0u) return (int)p;
-        if (v == x) return -1;
-        p = (p + 1) & (G::kWords - 1);
-    }
-    return -1;
 }
 
 // Zeroes the store's first `bits` bits (rounded up to 128).
@@ -198,11 +188,14 @@ __device__ __forceinline__ void write_not_synchronizing(const Batch &b, int64_t 
 // search stops at the first level wider than n sets.
 //
 // Hundreds of levels of one to n sets are a serial chain.  A level of one set
-// (every level of a Cerny automaton but the first) is run by all lanes alike on
-// the same set: both preimages and both hash probes in registers, no ballot,
-// shuffle or atomic on the way to the next level.  Wider levels keep set i in
-// lane i and give every image a lane of its own, one hash probe per lane.  C_28
-// (729 levels): 0.40 ms with every level on the lane-per-image form.
+// with one new preimage, found at the first probe (almost every level of a Cerny
+// automaton), is run by all lanes alike on the same set: both preimages and both
+// probes in registers, one branch, no ballot, shuffle or atomic on the way to the
+// next level.  Other levels keep set i in lane i and give every image a lane of
+// its own, one hash probe per lane.  C_28 (729 levels): 0.40 ms with every level
+// on the lane-per-image form, 0.26 ms with a branch per case on the narrow one,
+// 0.17 ms so.  (Looking up the next level's preimages of both while the probes
+// run: 0.18 ms; the warp's instructions bound it, not the latencies.)
 //
 // Before giving up, pairs of states settle the wide automata that never
 // synchronize: an automaton synchronizes iff every pair of its states is merged
@@ -239,49 +232,27 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
     bool hit = false, spent = true;   // spent: no set left to expand
     const uint32_t letter = (uint32_t)lane & 1u;
     while (true) {
-        while (width == 1) {
-            const uint32_t x = __shfl_sync(kFull, front, 0);
-            const uint64_t t = lookup(W, x);
-            const uint32_t ya = (uint32_t)(t >> 32), yb = (uint32_t)t;
-            expanded += lane < 2 ? 1u : 0u;
-            if (ya == full || yb == full) {
-                found = head;
-                found_letter = ya == full ? 0u : 1u;
-                hit = true;
-                break;
+        if (width == 1) {
+            uint32_t x = __shfl_sync(kFull, front, 0);
+            while (true) {
+                const uint64_t t = lookup(W, x);
+                const uint32_t ya = (uint32_t)(t >> 32), yb = (uint32_t)t;
+                const uint32_t pa = set_slot<MAXN, SIZE>(ya), pb = set_slot<MAXN, SIZE>(yb);
+                const uint32_t va = W.store[pa], vb = W.store[pb];
+                __syncwarp();   // every lane has probed before the set is written
+                const bool na = ya != 0u && va == 0u, nb = yb != 0u && vb == 0u && yb != ya;
+                const bool sure = (va == 0u || va == ya || ya == 0u) && (vb == 0u || vb == yb || yb == 0u || yb == ya);
+                if (!sure || na == nb || ya == full || yb == full || tail >= G::kSetLimit) break;
+                x = na ? ya : yb;
+                W.store[na ? pa : pb] = x;
+                W.push(tail, x, head, na ? 0u : 1u);
+                __syncwarp();
+                expanded += lane < 2 ? 1u : 0u;
+                head = tail++;
+                ++level;
             }
-            const int pa = ya ? set_find(W, ya) : -1, pb = yb && yb != ya ? set_find(W, yb) : -1;
-            __syncwarp();   // every lane has probed before lane 0 writes
-            if (pa < 0 && pb < 0) {
-                width = 0;
-                break;
-            }
-            if (tail + 2u > G::kSetLimit) {
-                spent = false;
-                break;
-            }
-            const uint32_t both = pa >= 0 && pb >= 0 ? 1u : 0u;
-            if (pa == pb) {   // two new sets for one free slot
-                if (lane == 0) {
-                    set_insert(W, ya);
-                    set_insert(W, yb);
-                }
-            } else {
-                if (lane == 0 && pa >= 0) W.store[pa] = ya;
-                if (lane == 0 && pb >= 0) W.store[pb] = yb;
-            }
-            if (lane == 0) {
-                if (pa >= 0) W.push(tail, ya, head, 0u);
-                if (pb >= 0) W.push(tail + both, yb, head, 1u);
-            }
-            __syncwarp();
-            front = both ? (lane == 0 ? ya : lane == 1 ? yb : 0u) : pa >= 0 ? ya : yb;
-            head = tail;
-            width = 1u + both;
-            tail += width;
-            ++level;
+            front = x;
         }
-        if (hit || !spent || width == 0) break;
         // image j of the level is letter j & 1 of set j >> 1: 32 images per pass, at most two passes
         uint32_t added = 0, next = 0;
         for (uint32_t base = 0; base < 2u * width; base += 32) {
