@@ -719,13 +719,12 @@ std::string graph_key(const void *a, const void *b, const void *c, const void *d
 //  - a pageable caller's records are staged into pinned memory chunk by
 //    chunk, and its results go on from pinned staging as each chunk lands,
 //    both by the handle's host copy threads.
-constexpr int64_t kStreamChunk = 1 << 17;   // x 2n bytes: whole 128-byte lines
-// Chunk 0's size.  A 2^14-automaton first chunk (the kernel starts after a
-// 0.4 MB copy instead of 3 MB) measured the same end to end with pinned buffers
-// (0.913-0.946 ms against 0.923-0.941 ms per 10^6 automata at n = 12) and
-// slower with pageable ones (2.06-2.20 ms against 1.44-1.63 ms): the kernel
-// then waits on chunk 1 while the host stages it.
-constexpr int64_t kStreamFirst = kStreamChunk;
+// 2^17 automata x 2n bytes: whole 128-byte lines.  Each copy of a chunk costs
+// both directions about 8 us beyond its bytes (24 MB in and 20 MB out at once: 0.61 ms
+// as 8 copies each way, 0.75 as 16; 10^6 n = 12 end to end 0.90 ms, 1.00 with
+// 2^16, 1.20 with 2^15), and a short first chunk (2^14 to 2^16) gains nothing.
+constexpr int kStreamChunkLog2 = 17;
+constexpr int64_t kStreamChunk = 1 << kStreamChunkLog2;
 constexpr int64_t kStreamJob = 1 << 24;     // automata per kernel launch
 
 bool stream_eligible(sbfs_handle *h, const uint8_t *ns, int32_t n_uniform, int64_t count, bool plain)
@@ -750,8 +749,7 @@ sbfs_status solve_streamed_job(sbfs_handle *h, const uint8_t *maps, int32_t lstr
     Streamer &S = h->streamer;
     const size_t rec = 2 * (size_t)lstride;
     LaneStream geo{};
-    geo.chunk = kStreamChunk;
-    geo.first = kStreamFirst;
+    geo.chunk_log2 = kStreamChunkLog2;
     const int64_t nch = geo.chunks(cnt);
     const int c = class_of_n(n);
     // n = 13 (class 2) runs on k_lane<13> with class 1's escalation counters

@@ -148,23 +148,17 @@ struct LaneStream {
     const unsigned int *chunk_ready;   // nonzero once chunk c's records are on the device
     unsigned int *chunk_done;          // lane outcomes recorded per chunk (starts at 0)
     unsigned int *host_flag;           // mapped host memory: 1 once chunk c's outcomes are all written
-    int64_t chunk;                     // automata per chunk after the first (whole 128-byte lines of records)
+    int chunk_log2;                    // 2^this automata per chunk (whole 128-byte lines of records)
     EscalResult *escal_out;            // by escalation slot: results the whole-warp search writes
     int wait_polls;                    // bounded wait for a chunk's records: polls before giving up
-    // automata in chunk 0, at most `chunk`: a short first copy lets the kernel
-    // start sooner (whole 128-byte lines of records too)
-    int64_t first;
 
-    // (a job's automata, 2^24 at most, are divided in 32 bits)
-    __host__ __device__ int64_t chunk_of(int64_t k) const
-    {
-        return k < first ? 0 : 1 + (int64_t)((uint32_t)(k - first) / (uint32_t)chunk);
-    }
-    __host__ __device__ int64_t chunk_begin(int64_t c) const { return c == 0 ? 0 : first + (c - 1) * chunk; }
+    // (a job has 2^24 automata at most)
+    __host__ __device__ int chunk_of(int64_t k) const { return (int)((uint32_t)k >> chunk_log2); }
+    __host__ __device__ int64_t chunk_begin(int64_t c) const { return c << chunk_log2; }
     // chunks of a batch of `count` automata, and the size of chunk c
     __host__ __device__ int64_t chunks(int64_t count) const
     {
-        return count <= first ? 1 : 1 + (count - first + chunk - 1) / chunk;
+        return (count + ((int64_t)1 << chunk_log2) - 1) >> chunk_log2;
     }
     __host__ __device__ int64_t chunk_size(int64_t c, int64_t count) const
     {

@@ -336,7 +336,7 @@ __device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, u
             // (if the chunk still had searches out after these results were stored, its
             // copy, which comes after the last of them, takes them along)
             __threadfence();
-            const int64_t c = ls.chunk_of(k);
+            const int c = ls.chunk_of(k);
             const bool early = *(volatile unsigned int *)(ls.chunk_done + c) < (unsigned)ls.chunk_size(c, b.count);
             EscalResult r;
             r.k = early ? kEscalInChunk : k;
@@ -378,6 +378,16 @@ __host__ __device__ constexpr size_t region_words(int ring)
     const size_t lanes = (size_t)(G::kLaneWords + G::kTable + ring) * 32 + G::kPoolWords;
     const size_t whole = (size_t)G::kBitmapWords + ((size_t)1 << NMAX);
     return lanes > whole ? lanes : whole;
+}
+
+// Streamed batches: `add` outcomes of chunk c are written (and fenced); whoever completes the
+// chunk tells the host that its lengths and words can be copied out.
+__device__ __forceinline__ void tell_chunk(const LaneStream &ls, int64_t c, unsigned add, int64_t count)
+{
+    if ((int64_t)(atomicAdd(ls.chunk_done + c, add) + add) == ls.chunk_size(c, count)) {
+        __threadfence_system();
+        *(volatile unsigned int *)(ls.host_flag + c) = 1u;
+    }
 }
 
 template <int NMAX, bool WORDS, bool STREAM>
@@ -422,6 +432,11 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
     uint32_t pass = 0, since = 0;   // passes that asked for the pool; the one this lane came in
     uint32_t checks = 0;
     int ready_upto = -1;            // streamed chunks known to be on the device
+    unsigned waiting = 0;           // streamed: lanes whose records are not there yet (set at the refill pass)
+    // Streamed outcomes that this warp has not told of yet: of the chunk its next
+    // ticket is in (`cur`; past the last one once all are handed out) and of the one before
+    int cur = 0;
+    unsigned own_cur = 0, own_old = 0;
 
     while (true) {
         // ---- phase: finish waiting lanes, load new automata -----------------
@@ -435,7 +450,7 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
         const unsigned not_active = __ballot_sync(kFull, state != kActive);
         // (streamed: lanes that wait for records ask for a look at the chunk flags,
         // one trip to L2, at every eighth check only)
-        const unsigned served = STREAM ? not_active & ~__ballot_sync(kFull, state == kWaiting) : not_active;
+        const unsigned served = STREAM ? not_active & ~waiting : not_active;
         if (not_active == kFull || (STREAM && served != not_active && (++checks & 7u) == 0u) ||
             (__popc(served) >= refill_k && (more || __any_sync(kFull, state == kDone || state == kEscalate)))) {
             const bool outcome = state == kDone || state == kEscalate;
@@ -464,22 +479,30 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     hslot = slot;
                 }
             }
-            if (STREAM) {
-                // streamed batch: count outcomes per chunk; whoever completes a
-                // chunk tells the host its lengths and words can be copied out
+            if (STREAM && !G::kOneWarp) {
+                // n <= 8: told at once (with the counts below the kernel spills: 10^6
+                // n = 8 end to end 0.672 ms against 0.657)
                 const unsigned om = __ballot_sync(kFull, outcome);
                 if (outcome) {
                     __threadfence();   // this lane's results before its count
-                    const int64_t c = ls.chunk_of(k);
-                    const unsigned grp = __match_any_sync(om, (unsigned long long)c);
-                    if (lane == __ffs(grp) - 1) {
-                        const unsigned add = (unsigned)__popc(grp);
-                        const unsigned old = atomicAdd(ls.chunk_done + c, add);
-                        const int64_t size = ls.chunk_size(c, count);
-                        if ((int64_t)(old + add) == size) {
-                            __threadfence_system();
-                            *(volatile unsigned int *)(ls.host_flag + c) = 1u;
-                        }
+                    const int c = ls.chunk_of(k);
+                    const unsigned grp = __match_any_sync(om, c);
+                    if (lane == __ffs(grp) - 1) tell_chunk(ls, c, (unsigned)__popc(grp), count);
+                }
+            } else if (STREAM) {
+                const int c = ls.chunk_of(k);
+                own_cur += (unsigned)__popc(__ballot_sync(kFull, outcome && c == cur));
+                if (__any_sync(kFull, outcome && c != cur)) {
+                    own_old += (unsigned)__popc(__ballot_sync(kFull, outcome && c == cur - 1));
+                    // (two chunks and more behind the tickets: told one by one)
+                    const bool late = outcome && c < cur - 1;
+                    const bool last = own_old && !__any_sync(kFull, c == cur - 1 && (state == kActive || state == kWaiting));
+                    if (__any_sync(kFull, late) || last) {
+                        __threadfence();   // every lane's results before the counts
+                        __syncwarp();
+                        if (late) tell_chunk(ls, c, 1u, count);
+                        if (last && lane == 0) tell_chunk(ls, cur - 1, own_old, count);
+                        if (last) own_old = 0;
                     }
                 }
             }
@@ -506,6 +529,29 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                         since = 0;
                     }
                 }
+                if (STREAM && G::kOneWarp) {
+                    const int next = more ? ls.chunk_of((int64_t)(got + __popc(idle))) : ls.chunk_of(count - 1) + 1;
+                    if (next != cur) {
+                        // The tickets enter a new chunk: what the warp still owes to the
+                        // chunk just left is told with its last search there, so a chunk
+                        // costs a warp one fence and one atomic, and the chunk is complete
+                        // no later for it.  (Told at every pass with an outcome, with the
+                        // chunk by division: 2^21 n = 13 end to end 1.66 ms against 1.61,
+                        // 500,000 n = 14 0.94 against 0.845, 10^6 n = 12 0.90 against 0.88.)
+                        const bool skip = next != cur + 1;   // others took a whole chunk meanwhile
+                        const bool done = !__any_sync(kFull, (state == kActive || state == kWaiting) && ls.chunk_of(k) == cur);
+                        if (own_old || (own_cur && (skip || done))) {
+                            __threadfence();   // every lane's results before the counts
+                            __syncwarp();
+                            if (lane == 0 && own_old) tell_chunk(ls, cur - 1, own_old, count);
+                            if (lane == 0 && own_cur && (skip || done)) tell_chunk(ls, cur, own_cur, count);
+                            if (skip || done) own_cur = 0;
+                        }
+                        own_old = own_cur;
+                        own_cur = 0;
+                        cur = next;
+                    }
+                }
             }
             // every lane that just received an automaton sets it up, and so does one
             // that waited (for the pool, or for its records)
@@ -516,8 +562,9 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                 // would hold back the results of the chunk before (1M n = 12 end to
                 // end: 1.17 ms with every such wait blocking, now that the kernel is
                 // faster than the link).
-                const int c = setup ? (int)ls.chunk_of(k) : -1;
-                const int c_last = (int)__reduce_max_sync(kFull, (unsigned)(c + 1)) - 1;
+                const int c = setup ? ls.chunk_of(k) : -1;
+                // (most passes know already that all chunks handed out are there)
+                const int c_last = !G::kOneWarp || cur > ready_upto ? (int)__reduce_max_sync(kFull, (unsigned)(c + 1)) - 1 : -1;
                 if (c_last > ready_upto) {
                     const int c_first = (int)__reduce_min_sync(kFull, setup ? (unsigned)c : ~0u);
                     const bool busy = __any_sync(kFull, state == kActive && !fresh);
@@ -551,10 +598,12 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     }
                     __threadfence();
                 }
-                if (setup && c > ready_upto) {
+                const bool absent = setup && c > ready_upto;
+                if (absent) {
                     setup = fresh = false;
                     state = kWaiting;
                 }
+                waiting = __ballot_sync(kFull, absent);
             }
             if (__any_sync(kFull, setup)) {
                 uint32_t words = 0, halves = 0;   // bitmap words, and pool halves they take
@@ -897,13 +946,21 @@ __global__ void k_escal_patch(const EscalResult *r, const unsigned long long *co
                               int ws)
 {
     const int64_t n = (int64_t)*count;
+    // a store is a packet on the link: 16 bytes of a word at once where they are aligned
+    // (10^6 n = 12 end to end 0.880 -> 0.858 ms)
+    const bool pairs = (ws & 1) == 0 && (reinterpret_cast<uintptr_t>(words) & 15u) == 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const EscalResult e = r[i];
         if (e.k == kEscalInChunk) continue;
         if (len) len[e.k] = e.len;
         if (words) {
             uint64_t *w = words + (size_t)e.k * (size_t)ws;
-            for (int j = 0; j < ws; ++j) w[j] = j < 3 ? e.word[j] : 0ull;
+            if (pairs)
+                for (int j = 0; j < ws; j += 2)
+                    *reinterpret_cast<ulonglong2 *>(w + j) =
+                        make_ulonglong2(j < 3 ? e.word[j] : 0ull, j + 1 < 3 ? e.word[j + 1] : 0ull);
+            else
+                for (int j = 0; j < ws; ++j) w[j] = j < 3 ? e.word[j] : 0ull;
         }
     }
 }
@@ -923,7 +980,7 @@ cudaError_t launch_lane(int nmax, int warps, int ring, int refill_k, int tail_k,
     if ((ring & (ring - 1)) || ring < 8 || warps < 1 || warps > 8 || ctas < 1 || refill_k < 1 || refill_k > 32 ||
         tail_k < 0 || tail_k > 32)
         return cudaErrorInvalidValue;
-    if (ls.chunk_done && (ls.chunk < 1 || ls.first < 1 || ls.first > ls.chunk || b.order || b.range_dev))
+    if (ls.chunk_done && (ls.chunk_log2 < 5 || ls.chunk_log2 > 30 || b.order || b.range_dev))
         return cudaErrorInvalidValue;
     const bool words = b.out_words != nullptr;
     if (nmax <= 8)
