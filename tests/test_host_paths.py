@@ -16,11 +16,11 @@ def _pinned(a):
     return torch.from_numpy(signed).pin_memory().numpy().view(a.dtype)
 
 
-def _mixed(count, seed):
+def _mixed(count, seed, lo=2, hi=14):
     rng = np.random.default_rng(seed)
-    ns = rng.integers(2, 15, count).astype(np.uint8)
+    ns = rng.integers(lo, hi + 1, count).astype(np.uint8)
     recs = np.zeros((count, 64), dtype=np.uint8)
-    for n in range(2, 15):
+    for n in range(lo, hi + 1):
         at = np.nonzero(ns == n)[0]
         recs[at] = P.uniform_maps(len(at), n, seed + n)
     return recs, ns
@@ -49,6 +49,23 @@ def test_small_calls(oracle_mod, use_graph, pin_in, pin_out):
             np.testing.assert_array_equal(r["len"], ref)
             assert oracle_mod.replay(recs, r["len"], r["words"], ns=ns)[0] == 0
             np.testing.assert_array_equal(eng.verify(recs, ns=ns)["len"], ref)
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_only_the_classes_of_the_sizes(oracle_mod, use_graph):
+    """Ranges of sizes that begin and end in each size class, one after another with
+    the same counts and buffers."""
+    count = 300
+    recs_at, ns_at = np.zeros((count, 64), dtype=np.uint8), np.zeros(count, dtype=np.uint8)
+    with sbfs.Engine(device=0, use_graph=use_graph) as eng:
+        for lo, hi in [(2, 8), (2, 9), (8, 20), (9, 12), (12, 13), (13, 16), (16, 17), (17, 20), (20, 21), (21, 22),
+                       (8, 22), (13, 20), (2, 20)] * 2:
+            recs_at[:], ns_at[:] = _mixed(count, 100 * lo + hi, lo, hi)
+            ref = oracle_mod.solve(recs_at, ns=ns_at, words=False, threads=8)["len"]
+            np.testing.assert_array_equal(eng.verify(recs_at, ns=ns_at)["len"], ref)
+        ns_at[17] = 0   # a malformed size is still found
+        with pytest.raises(Exception):
+            eng.verify(recs_at, ns=ns_at)
 
 
 @pytest.mark.parametrize("n", [7, 12, 13, 14])
