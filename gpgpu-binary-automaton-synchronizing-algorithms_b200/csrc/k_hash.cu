@@ -21,12 +21,12 @@
 //     subset, parent index and letter in 32 bits (a separate parent array
 //     where they do not fit).
 // 10.5 KB per warp for n <= 16 (21 warps per SM), 14.6 KB for n <= 20 (15).
-// Sizes above 20 keep 3072 subsets and a 16 KB store (6 warps per SM): at
-// n = 24 5 % of random automata pass that, 25 % would pass 1536.
+// Sizes above 20 have a 16 KB store and room for 3072 subsets (6 warps per SM),
+// of which the forward search takes 1024.
 // The warp expands 32 subsets of the current level per step (level-
 // synchronous, as GPGPU/CPU/SlimCPUUntweaked.cs:119-184), tests the images
 // against the store, and appends the new ones compacted by ballots in queue
-// order.  An automaton that needs more than 1536 subsets (or kHashLevelCap
+// order.  An automaton that needs more subsets than that (or kHashLevelCap
 // levels) is tried backwards by the same warp (inverse_search below), which
 // settles the slowly synchronizing families and the automata that never
 // synchronize; one with a permutation letter and a letter merging at most one
@@ -50,6 +50,12 @@ constexpr uint32_t kUnsettled = 1u << 31;
 template <int MAXN, int SIZE>
 struct HashGeom {
     static constexpr uint32_t kLimit = 1536u << (SIZE - 1);      // subsets a warp keeps
+    // Subsets the forward search keeps.  Above n = 20 a third of the room, which is
+    // the backward search's: a warp takes 60 us per thousand of them, and k_wide
+    // settles what is left in 10 to 50.  64 random n = 24 in one call 233 us with
+    // 3072, 129 with 1536, 115 with 1024, 102 with 512; 3000 n = 21 298, 183, 178
+    // and 210, 3000 n = 28 955, 855, 867 and 903.
+    static constexpr uint32_t kForward = MAXN > 20 ? 1024u : kLimit;
     static constexpr int kIdxBits = 10 + SIZE;                   // of a queue index
     // words of the visited store: 2^15 bits for n <= 16, 2^16 for n <= 20 (twice that at SIZE 2)
     static constexpr int kWords = (MAXN <= 16 ? 1024 : 2048) << (SIZE - 1);
@@ -352,7 +358,7 @@ __device__ __forceinline__ Forward forward_search(const Batch &b, int n, HashWar
                                                   unsigned long long &expanded)
 {
     using G = HashGeom<MAXN, SIZE>;
-    constexpr uint32_t kKeep = BITS ? G::kLimit : G::kSetLimit;
+    constexpr uint32_t kKeep = BITS || G::kForward < G::kSetLimit ? G::kForward : G::kSetLimit;
     Forward r{false, kLenNonSync, 0u, 0u, 0u};
     // n = 1: the visited root is the only singleton, the search generates nothing new
     uint32_t head = 0, lvl_end = n > 1 ? 1u : 0u, tail = lvl_end, level = 0;

@@ -1,9 +1,9 @@
 // k_wide.cu -- power-set BFS of automata with up to 28 states, one automaton
 // per CTA, with the visited set, the queue and the parents in shared memory.
 //
-// It takes the automata of 21..28 states whose search outgrows a warp's hash
-// set (k_hash.cu: 3072 subsets; 5 % of random automata at n = 24, 12 % at
-// n = 28) and is not settled backwards either.  The CTA holds 24,576 subsets:
+// It takes the automata of 21..28 states whose search outgrows what a warp
+// keeps (k_hash.cu: 1024 subsets; 25 % of random automata at n = 24 pass 1536,
+// 5 % pass 3072) and is not settled backwards either.  The CTA holds 24,576 subsets:
 // all but about 0.2 % of random n = 28.  What is wider still goes on to the
 // level slots in HBM (k_level.cu), whose levels each cost a launch.
 //   * set: 32,768 slots of a 32-bit subset (0 = free), linear probing, filled
@@ -17,7 +17,7 @@
 // for the rotation of the counters).  Bound by the barrier and the dependent
 // shared-memory accesses of a level; a level is a microsecond or two.
 // n = 24, 26, 28 x (64 random + C_n + permutation-plus-merge), one Verify call:
-// 18.0 ms with every automaton on the level slots, 0.73 ms with k_hash and this
+// 18.0 ms with every automaton on the level slots, 0.42 ms with k_hash and this
 // kernel before them.
 #include <atomic>
 
