@@ -1568,11 +1568,11 @@ int32_t sbfs_describe_plan(sbfs_handle *h, char *buf, int32_t len)
         const bool lane = c < 2 && !P.use_pool[c];
         if (c == 2 && P.class2_hash && P.use_lane13) {
             std::snprintf(tmp, sizeof tmp,
-                          "{\"class\":2,\"max_n\":16,\"kernel\":\"k_hash+k_cta\",\"slots\":%d,"
+                          "{\"class\":2,\"max_n\":16,\"kernel\":\"k_hash+k_mid\",\"slots\":%d,"
                           "\"uniform_n13\":\"k_lane<13>\",\"ring13\":%d,\"ctas13\":%d,"
                           "\"uniform_n14\":\"%s\",\"ring14\":%d,\"ctas14\":%d},",
                           P.class2_hash == 2 ? 4096 : 2048, P.lane13.ring, P.lane13.ctas,
-                          P.use_lane14 ? "k_lane<14>" : "k_hash+k_cta", P.lane14.ring, P.lane14.ctas);
+                          P.use_lane14 ? "k_lane<14>" : "k_hash+k_mid", P.lane14.ring, P.lane14.ctas);
         } else if (lane) {
             const LaneShape &l = P.lane[c];
             std::snprintf(tmp, sizeof tmp,
@@ -1580,7 +1580,7 @@ int32_t sbfs_describe_plan(sbfs_handle *h, char *buf, int32_t len)
                           "\"refill\":%d,\"ctas\":%d},",
                           c, kClassMaxN[c], l.nmax, l.warps, l.ring, l.refill_k, l.ctas);
         } else if (c == 2 && P.class2_hash) {
-            std::snprintf(tmp, sizeof tmp, "{\"class\":2,\"max_n\":16,\"kernel\":\"k_hash+k_cta\",\"slots\":%d},",
+            std::snprintf(tmp, sizeof tmp, "{\"class\":2,\"max_n\":16,\"kernel\":\"k_hash+k_mid\",\"slots\":%d},",
                           P.class2_hash == 2 ? 4096 : 2048);
         } else {
             const PoolShape &q = P.pool[c];
@@ -1593,8 +1593,8 @@ int32_t sbfs_describe_plan(sbfs_handle *h, char *buf, int32_t len)
     }
     std::snprintf(tmp, sizeof tmp,
                   "{\"class\":3,\"max_n\":20,\"kernel\":\"%s\",\"threads\":%d,\"ctas\":%d},"
-                  "{\"class\":4,\"max_n\":28,\"kernel\":\"k_level\",\"threads\":512,\"slots\":%d}]}",
-                  P.class3_level ? "k_level" : P.class3_hash ? "k_hash+k_cta" : "k_cta", P.cta.threads, P.cta.ctas,
+                  "{\"class\":4,\"max_n\":28,\"kernel\":\"k_hash+k_wide+k_level\",\"threads\":512,\"slots\":%d}]}",
+                  P.class3_level ? "k_level" : P.class3_hash ? "k_hash+k_mid+k_cta" : "k_cta", P.cta.threads, P.cta.ctas,
                   kMaxLevelSlots);
     js += tmp;
     if (buf && len > 0) {

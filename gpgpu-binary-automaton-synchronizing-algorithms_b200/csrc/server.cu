@@ -9,18 +9,18 @@
 //     them in and runs the batch kernels (per-lane / warp-pooled) on the
 //     slot's own stream.  The kernels store each automaton's length and word
 //     straight into mapped host memory and then flag it, so every request is
-//     delivered as soon as its own search ends -- a mini-batch holding a
-//     Cerny search (C_20: 361 levels, ~1 ms in one CTA) does not hold back the
-//     other requests in it;
+//     delivered as soon as its own search ends -- a mini-batch's longest search
+//     does not hold back the other requests in it;
 //   * large requests (n >= 21): when the previous level launch batch is done,
 //     collects finished slots, admits waiting requests in arrival order while
-//     their bitmap + queue fit the arena (the 2^n-bit budget), and launches
-//     the next few levels of every admitted request (k_level.cu).  Requests
+//     their bitmap + queue fit the arena (the 2^n-bit budget), tries the new
+//     ones on chip (k_hash.cu, k_wide.cu: all but the widest end there), and
+//     launches the next few levels of those that are left (k_level.cu).  Requests
 //     that arrive while others are running are admitted at the next turn and
 //     advance together with them: their work overlaps on the device.
 //     (n = 17..20 went through level slots too, at a p99 of 7 ms at 32K
 //     requests/s: every level of a Cerny C_20 cost one launch shared with all
-//     admitted requests.  In the mini-batches a CTA runs it alone.)
+//     admitted requests.  The mini-batches settle it on chip.)
 // Completion order follows the GPU, not submission order.
 #include <atomic>
 #include <chrono>

@@ -7,9 +7,9 @@
 //   classes 0, 1 (n <= 8, n <= 12): one automaton per lane (warps per CTA,
 //                 frontier ring, refill threshold) vs the warp-pooled kernel
 //                 (automata per warp, warps per CTA, on-chip queue entries);
-//   class 2 (n <= 16): warp-pooled shapes;
-//   class 3 (n <= 20): bitmap placement -- shared memory (one automaton per
-//                 CTA, threads per CTA) vs HBM (device-resident level slots).
+//   class 2 (n <= 16): one automaton per warp (k_hash, two sizes) vs warp-pooled shapes;
+//   class 3 (n <= 20): one automaton per warp first vs one per CTA (threads per
+//                 CTA), in shared memory, vs HBM (device-resident level slots).
 // The choice is cached per device (name, SM count, library version) in the
 // file named by sbfs_config.tune_cache, so later handles skip the measurement.
 #include <cstdio>
@@ -252,7 +252,7 @@ cudaError_t plan_autotune(sbfs_handle *h, Plan &plan)
         P.lane[c] = best.lane[c];
         P.pool[c] = best.pool[c];
     }
-    // ---- class 2: hash-set warps (long searches handed to k_cta) vs pooled shapes
+    // ---- class 2: a warp each (long searches handed to k_mid) vs pooled shapes
     if (e == cudaSuccess && (e = prepare(b, 16, 1 << 16)) == cudaSuccess) {
         Plan best = P;
         double best_ms = 1e30;
@@ -290,7 +290,7 @@ cudaError_t plan_autotune(sbfs_handle *h, Plan &plan)
         P.class2_hash = best.class2_hash;
         P.pool[2] = best.pool[2];
     }
-    // ---- class 3: hash-set warps (long searches handed to k_cta) vs shared-memory
+    // ---- class 3: a warp each (long searches handed to k_mid and k_cta) vs shared-memory
     // bitmaps (per CTA) vs HBM bitmaps (level slots)
     // (2 % Cerny C_20 in the batch: their long thin searches set a class-3
     // launch's makespan in the mixed and serving configurations)

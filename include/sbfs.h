@@ -211,8 +211,9 @@ SBFS_API int32_t sbfs_describe_plan(sbfs_handle *h, char *buf, int32_t len);
  * mini-batches (several in flight) and solved by the batch kernels, which
  * deliver each result as soon as its own search ends; automata with n >= 21
  * are admitted into device-resident BFS slots while their 2^n-bit bitmap and
- * queue fit the arena budget, and advance a few levels per launch alongside
- * every other admitted request, so a request that arrives while others run is
+ * queue fit the arena budget, are tried on chip in the turn that admits them
+ * and, the few that are wider than that, advance a few levels per launch
+ * alongside every other admitted request, so a request that arrives while others run is
  * taken in as soon as memory frees up.  No reference counterpart (the reference solves fixed
  * batches only, GPGPU/Program.cs:76-111).
  * ------------------------------------------------------------------------- */
