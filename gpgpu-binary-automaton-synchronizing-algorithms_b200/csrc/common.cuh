@@ -10,6 +10,13 @@ namespace sbfs {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
+// All the dynamic shared memory an sm_100a CTA may have (a kernel without any
+// static one).  The cap belongs to a kernel on a device, not to a handle: a
+// kernel whose launches differ in footprint gets this same cap from each of them.
+// With each launch's own footprint, handles in two threads could lower it between
+// the other's setting and its launch, which was then refused.
+constexpr int kMaxDynamicSmem = 227 * 1024;
+
 // Length codes written to out_len besides real lengths.
 constexpr int32_t kLenNonSync = -1;   // queue emptied without a singleton
 constexpr int32_t kLenInvalid = -2;   // malformed record (state >= n); host turns into EINVAL

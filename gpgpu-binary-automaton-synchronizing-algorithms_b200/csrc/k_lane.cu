@@ -905,7 +905,7 @@ cudaError_t launch_t(int warps, int ring, int refill_k, int tail_k, int ctas, co
     const size_t smem = smem_for<NMAX>(w, ring);
     // the streamed form's bookkeeping is compiled out of the resident-batch kernel
     auto kernel = ls.chunk_done ? k_lane<NMAX, WORDS, true> : k_lane<NMAX, WORDS, false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess) return e;
     kernel<<<ctas * (warps / w), w * 32, smem, st>>>(b, ring, refill_k, tail_k, escal_list, escal_capacity,
                                                      escal_count, escal_claim, ticket, ls);
@@ -927,7 +927,7 @@ int lane_max_ctas_per_sm(int nmax, int warps, int ring)
                         : nmax <= 12 ? smem_for<12>(w, ring)
                         : nmax == 13 ? smem_for<13>(w, ring)
                                      : smem_for<14>(w, ring);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }

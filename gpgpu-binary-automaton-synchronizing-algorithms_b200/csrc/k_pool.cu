@@ -338,7 +338,7 @@ cudaError_t launch_t(const PoolShape &s, const Batch &b, uint32_t *spill,
 {
     const size_t smem = pool_smem_bytes(s);
     cudaError_t e = cudaFuncSetAttribute(k_pool<NMAX, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         kMaxDynamicSmem);
     if (e != cudaSuccess) return e;
     k_pool<NMAX, S><<<s.ctas, s.warps * 32, smem, st>>>(b, s.queue_smem, s.grab > 0 ? s.grab : 16, spill, ticket,
                                                          hv);
@@ -402,7 +402,7 @@ int pool_max_ctas_per_sm(const PoolShape &s)
     const void *k = pool_kernel(s);
     if (!k) return 0;
     const size_t smem = pool_smem_bytes(s);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
