@@ -259,7 +259,9 @@ __device__ unsigned long long level_transition(LevelSlot *slots, LevelCtl *ctl, 
                         e = __ldcg(sl.queue + ((e >> 28) & 0x7FFFFFFFFull));
                     }
                 }
-                if (out.out_len && sl.tag >= 0 && next == kSlotDone) {
+                // a batch counts violations and takes words without lengths too; the
+                // serving loop (no counters) takes both from the slot
+                if (out.first_violation && sl.tag >= 0 && next == kSlotDone) {
                     record_result(out, sl.tag, sl.n, len);
                     if (out.out_words) {
                         uint64_t *w = out.out_words + (size_t)sl.tag * (size_t)out.word_stride;
