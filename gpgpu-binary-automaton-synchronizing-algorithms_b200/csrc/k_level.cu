@@ -484,9 +484,11 @@ __global__ void __launch_bounds__(kMaxLevelSlots) k_level_settle(LevelSlot *slot
     __syncthreads();
     if (settled) {
         LevelSlot &sl = slots[s];
-        sl.result_len = t->len[i];
-        for (int c = 0; c < kLevelWordU64; ++c) sl.word[c] = t->words[i * kLevelWordU64 + c];
-        sl.state = kSlotDone;
+        // an error of the try may have cut any of its searches short: no result is told
+        const bool failed = t->error != 0;
+        sl.result_len = failed ? kLenNonSync : t->len[i];
+        for (int c = 0; c < kLevelWordU64; ++c) sl.word[c] = failed ? 0ull : t->words[i * kLevelWordU64 + c];
+        sl.state = failed ? kSlotFail : kSlotDone;
         atomicAdd(&ctl->finished, 1u);
     } else if (i < n) {
         ctl->init_list[atomicAdd(&left, 1)] = s;

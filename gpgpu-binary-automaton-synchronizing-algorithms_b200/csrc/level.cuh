@@ -67,15 +67,16 @@ struct LevelTry {
     int32_t len[kMaxLevelSlots];
     int32_t list[2][kMaxLevelSlots];                 // left by k_hash, left by k_wide
     uint64_t words[kMaxLevelSlots * kLevelWordU64];
-    unsigned long long ticket[2], range[2][2];       // zeroed before every try
-    unsigned long long first_violation, expanded;
+    // from here on zeroed before every try
+    unsigned long long ticket[2], range[2][2];
+    unsigned long long first_violation;
     int error, pad;
 };
 
 int level_max_ctas_per_sm();
 // Ends the slots init_list[0..n) whose automaton the on-chip kernels settled
-// (t->len[i] is not kLenUntried) and takes them off the list that the launch of
-// parity `par` sets up.
+// (t->len[i] is not kLenUntried; as failed when the try left an error) and takes
+// them off the list that the launch of parity `par` sets up.
 cudaError_t launch_level_settle(LevelSlot *slots, LevelCtl *ctl, const LevelTry *t, int n, int par, cudaStream_t st);
 cudaError_t launch_level(int ctas, int parity, LevelSlot *slots, uint64_t *tables, LevelCtl *ctl, const Batch &out,
                          cudaStream_t st);
@@ -120,8 +121,9 @@ public:
     static size_t footprint(int n);
     // From now on freshly admitted slots (with host maps) are first tried on chip,
     // one warp and then one CTA each (k_hash.cu, k_wide.cu), in the launch that
-    // admits them; only what is wider than that runs level by level.
-    cudaError_t try_on_chip();
+    // admits them; only what is wider than that runs level by level.  (For tests,
+    // try number `fail_try` starts with its error word set; 0 = none.)
+    cudaError_t try_on_chip(long long fail_try = 0);
     // admitted slots that a past launch has not settled: their levels are still to run
     int running() const { return in_flight_ - (int)pending_init_.size(); }
     // admit one automaton whose record is at d_rec (device); returns slot or -1 (no slot/memory)
@@ -177,6 +179,7 @@ private:
     int *h_init_ = nullptr;          // pinned: nslots, n_init, init_list[]
     LevelTry *d_try_ = nullptr;      // set by try_on_chip
     LevelTry *h_try_ = nullptr;      // pinned: recs and ns
+    long long tries_ = 0, fail_try_ = 0;
     int sm_count_ = 0;
     Arena own_;
     Arena *shared_ = nullptr;

@@ -3,6 +3,7 @@
 // launches and collection of finished automata.
 #include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cstring>
 
 #include "level.cuh"
@@ -143,8 +144,9 @@ void LevelEngine::destroy()
     ev_ = nullptr;
 }
 
-cudaError_t LevelEngine::try_on_chip()
+cudaError_t LevelEngine::try_on_chip(long long fail_try)
 {
+    fail_try_ = fail_try;
     cudaError_t e = cudaHostAlloc(&h_try_, sizeof(LevelTry), cudaHostAllocDefault);
     if (e != cudaSuccess) {
         h_try_ = nullptr;
@@ -170,8 +172,9 @@ cudaError_t LevelEngine::launch_try(int n)
         return e;
     if ((e = cudaMemcpyAsync(d_try_->ns, h_try_->ns, (size_t)n, cudaMemcpyHostToDevice, st_)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(d_try_->len, 0x80, sizeof(int32_t) * (size_t)n, st_)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(d_try_->ticket, 0, sizeof(d_try_->ticket) + sizeof(d_try_->range), st_)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(d_try_->ticket, 0, sizeof(LevelTry) - offsetof(LevelTry, ticket), st_)) != cudaSuccess)
         return e;
+    if (++tries_ == fail_try_ && (e = cudaMemsetAsync(&d_try_->error, 1, sizeof(int), st_)) != cudaSuccess) return e;
     Batch b{};
     b.maps = d_try_->recs;
     b.lstride = LevelTry::kRec / 2;
@@ -181,7 +184,6 @@ cudaError_t LevelEngine::launch_try(int n)
     b.out_words = d_try_->words;
     b.word_stride = kLevelWordU64;
     b.first_violation = &d_try_->first_violation;
-    b.expanded = &d_try_->expanded;
     b.error = &d_try_->error;
     const int per_sm = hash_max_ctas_per_sm(2, SBFS_MAX_N);
     if (per_sm < 1) return cudaErrorInvalidConfiguration;

@@ -110,6 +110,9 @@ struct sbfs_server {
     // mini-batch k is reported as failed once its work has completed, as a
     // failed cudaEventQuery would report it; no GPU fault is involved
     int64_t inject_fail_batch = 0;
+    // SBFS_SERVER_FAIL_TRY=k: the error word of the k-th on-chip try of large
+    // requests is set by the host, as a failed check of a checked build sets it
+    int64_t inject_fail_try = 0;
 
     double now_ms() const
     {
@@ -498,6 +501,7 @@ sbfs_status sbfs_server_start(const sbfs_server_config *cfg, sbfs_server **out)
     if (s->cfg.arena_bytes <= 0) s->cfg.arena_bytes = (int64_t)16 << 30;
     if (s->cfg.small_budget_bytes <= 0) s->cfg.small_budget_bytes = (int64_t)1 << 30;
     if (const char *inj = std::getenv("SBFS_SERVER_FAIL_BATCH")) s->inject_fail_batch = std::atoll(inj);
+    if (const char *inj = std::getenv("SBFS_SERVER_FAIL_TRY")) s->inject_fail_try = std::atoll(inj);
     sbfs_config hc;
     sbfs_config_default(&hc);
     hc.device = s->cfg.device;
@@ -525,7 +529,7 @@ sbfs_status sbfs_server_start(const sbfs_server_config *cfg, sbfs_server **out)
     }
     if (e == cudaSuccess && (e = s->arena.reserve((size_t)s->cfg.arena_bytes)) == cudaSuccess)
         e = s->big.init(s->h->sm_count, 0, s->h->lanes[kSmallSlots].stream, &s->arena);
-    if (e == cudaSuccess) e = s->big.try_on_chip();
+    if (e == cudaSuccess) e = s->big.try_on_chip(s->inject_fail_try);
     if (e == cudaSuccess) e = prime_small(s);
     if (e != cudaSuccess) {
         cudaGetLastError();
