@@ -21,7 +21,12 @@
 // all of them apart.  Ranks average 0.65 n; 1536 bits serve 98 % of random n = 12
 // (512 B of one bit per subset became 192 B, 7 warps per SM became 10), 3072 and
 // 6400 bits over 99 % at n = 13 and 14 (4 became 6, 2 became 3).  The other
-// automata take bitmaps from a pool of the warp's, in the order in which they came.
+// automata take bitmaps from a pool of the warp's, in the order in which they came,
+// and when that is used up the whole column (bitmap, table, ring) of a lane that
+// does not search.  Batches of such automata alone, one permutation and one random
+// map: half of the lanes search, 200,000 n = 12 in 0.73 ms and 100,000 n = 13 in
+// 0.76 (with the pool alone 2.02 and 4.44, with a bitmap of 2^n bits per lane 0.95
+// and 0.99).
 // Relabelling changes neither the order of the search nor its words.  1M n = 12
 // device-resident: 0.592 -> 0.472 ms; 500K n = 14: 1.158 -> 0.760 ms; a Verify call
 // on 2^21 n = 13: 2.25 -> 1.95 ms.
@@ -72,7 +77,8 @@
 namespace sbfs {
 namespace {
 
-constexpr int kActive = 0, kDone = 1, kEscalate = 2, kIdle = 3, kHeld = 4, kWaiting = 5;
+// (kLent: waiting, and its column serves its partner's search)
+constexpr int kActive = 0, kDone = 1, kEscalate = 2, kIdle = 3, kHeld = 4, kWaiting = 5, kLent = 6;
 constexpr int kStep = 4;   // subsets a lane expands per step (their 2 * kStep images are tested together)
 // Warps of a launched CTA when `warps` are asked for (n > 8: one, see kOneWarp),
 // and CTAs of that many that the registers must allow for
@@ -103,6 +109,7 @@ struct LaneGeom {
     static constexpr int kHalves = NMAX <= 8 ? 0 : NMAX <= 12 ? 6 : NMAX == 13 ? 2 : 8;
     static constexpr int kPoolWords = kHalves * kHalfWords;
     static constexpr uint32_t kAllHalves = (1u << kHalves) - 1u;
+    static constexpr uint32_t kBorrowed = 1u << 31;   // beside the halves a lane holds: its partner's column
     // One warp per CTA, so that its region starts at a constant address and every
     // access of a step is a lane's offset plus an immediate (1M n = 12: 0.514 ->
     // 0.490 ms at ten warps per SM).  n <= 8 keeps more warps than that allows.
@@ -142,6 +149,12 @@ __device__ __forceinline__ uint32_t table_entry(const uint8_t *rec, int lstride,
             t |= (1u << (__ldg(rec + st) + 16)) | (1u << __ldg(rec + lstride + st));
     }
     return t;
+}
+
+// The lanes beside those of m: 2i for 2i + 1 and 2i + 1 for 2i.
+__device__ __forceinline__ unsigned partners(unsigned m)
+{
+    return ((m & 0x55555555u) << 1) | ((m >> 1) & 0x55555555u);
 }
 
 // v << (c & 31)
@@ -429,6 +442,8 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
     uint32_t stride = 32, low_end = 1u << NMAX, index0 = 0, shift = 0;
     uint32_t held = 0;              // halves of the pool this lane's bitmap is in
     uint32_t pool_free = G::kAllHalves;   // halves nobody holds (alike in every lane)
+    unsigned away = 0;              // lanes that only another's end can start: lent, or without a bitmap
+    int enough = refill_k;          // idle lanes that trigger a refill, as a share of those not away
     uint32_t pass = 0, since = 0;   // passes that asked for the pool; the one this lane came in
     uint32_t checks = 0;
     int ready_upto = -1;            // streamed chunks known to be on the device
@@ -450,9 +465,9 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
         const unsigned not_active = __ballot_sync(kFull, state != kActive);
         // (streamed: lanes that wait for records ask for a look at the chunk flags,
         // one trip to L2, at every eighth check only)
-        const unsigned served = STREAM ? not_active & ~waiting : not_active;
-        if (not_active == kFull || (STREAM && served != not_active && (++checks & 7u) == 0u) ||
-            (__popc(served) >= refill_k && (more || __any_sync(kFull, state == kDone || state == kEscalate)))) {
+        const unsigned served = not_active & ~(STREAM ? waiting | away : away);
+        if (not_active == kFull || (STREAM && waiting && (++checks & 7u) == 0u) ||
+            (__popc(served) >= enough && (more || __any_sync(kFull, state == kDone || state == kEscalate)))) {
             const bool outcome = state == kDone || state == kEscalate;
             if (state == kDone) {
                 record_result(b, k, n, res_len);
@@ -496,7 +511,7 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     own_old += (unsigned)__popc(__ballot_sync(kFull, outcome && c == cur - 1));
                     // (two chunks and more behind the tickets: told one by one)
                     const bool late = outcome && c < cur - 1;
-                    const bool last = own_old && !__any_sync(kFull, c == cur - 1 && (state == kActive || state == kWaiting));
+                    const bool last = own_old && !__any_sync(kFull, c == cur - 1 && (state == kActive || state >= kWaiting));
                     if (__any_sync(kFull, late) || last) {
                         __threadfence();   // every lane's results before the counts
                         __syncwarp();
@@ -506,10 +521,12 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     }
                 }
             }
-            if (state != kActive && state != kHeld && state != kWaiting) state = kIdle;
+            if (state == kDone || state == kEscalate) state = kIdle;
             if (G::kRelabel) {
                 if (state != kActive) held = 0;
                 pool_free = G::kAllHalves & ~__reduce_or_sync(kFull, held);
+                const unsigned lent = partners(__ballot_sync(kFull, held & G::kBorrowed));
+                if (state == kLent && !((lent >> lane) & 1u)) state = kWaiting;
             }
             const unsigned idle = __ballot_sync(kFull, state == kIdle);
             bool fresh = false;   // the lane just received an automaton
@@ -539,7 +556,7 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                         // chunk by division: 2^21 n = 13 end to end 1.66 ms against 1.61,
                         // 500,000 n = 14 0.94 against 0.845, 10^6 n = 12 0.90 against 0.88.)
                         const bool skip = next != cur + 1;   // others took a whole chunk meanwhile
-                        const bool done = !__any_sync(kFull, (state == kActive || state == kWaiting) && ls.chunk_of(k) == cur);
+                        const bool done = !__any_sync(kFull, (state == kActive || state >= kWaiting) && ls.chunk_of(k) == cur);
                         if (own_old || (own_cur && (skip || done))) {
                             __threadfence();   // every lane's results before the counts
                             __syncwarp();
@@ -690,15 +707,17 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                         state = kDone;
                         res_len = kLenInvalid;
                         res_word = 0;
-                    } else if (n == 1) {
+                    } else if (n == 1 || (G::kRelabel && ra + rb == 2u * (uint32_t)n)) {
                         // the root is the only singleton and it is visited, so the
                         // search never generates a new one: not synchronizing, as in
                         // GPGPU/CPU/SlimCPUUntweaked.cs:149-157 (and the singleton-first
                         // test below, which relies on no singleton being visited, is
-                        // never reached)
+                        // never reached).  Nor do two permutations generate anything but
+                        // the root, and would ask for the largest bitmap to find that out.
                         state = kDone;
                         res_len = kLenNonSync;
                         res_word = 0;
+                        steps_expanded += n > 1;
                     } else {
                         uint32_t bits = 1u << n;
                         index0 = shift = 0;
@@ -719,9 +738,9 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                 }
                 if (G::kRelabel) {
                     // The pool goes to the lanes that need it, in the order in which they
-                    // came; the others wait.  (Out of order, a lane could wait until the
-                    // end of the batch: a streamed batch's first chunk was then complete
-                    // only with its last.)
+                    // came.  (Out of order, a lane could wait until the end of the
+                    // batch: a streamed batch's first chunk was then complete only with
+                    // its last.)
                     unsigned want = __ballot_sync(kFull, halves != 0u);
                     if (want) ++pass;
                     if (halves != 0u && since == 0u) since = pass;
@@ -747,10 +766,27 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                             held = take;
                         }
                     }
-                    if (halves != 0u) {
-                        words = 0;
-                        if (!held) state = kWaiting;
+                    if (want) {
+                        // Batches of permutations and other large ranks need more bitmaps
+                        // than the pool has.  A lane that it leaves out takes its partner's
+                        // column (bitmap, table and ring: 160, 288 and 520 words at n = 12,
+                        // 13 and 14, for 128, 256 and 512) when that lane does not search:
+                        // of two left out the one that came first.
+                        const bool out = halves != 0u && !held;
+                        const uint32_t key = out ? since : state == kActive || state == kDone ? 0u : ~0u;
+                        const uint32_t other = __shfl_xor_sync(kFull, key, 1);
+                        const bool borrow = out && words <= (uint32_t)(LW + T + ring) &&
+                                            (other > since || (other == since && !(lane & 1)));
+                        if (out && !borrow) state = kWaiting;
+                        if (partners(__ballot_sync(kFull, borrow)) >> lane & 1u) state = state == kWaiting ? kLent : state;
+                        __syncwarp();   // every lane is done with its own column
+                        if (borrow) {
+                            bm = base + (lane ^ 1);
+                            held = G::kBorrowed;
+                            for (uint32_t w = 0; w < words; ++w) bm[w * 32] = 0u;
+                        }
                     }
+                    if (halves != 0u) words = 0;
                 }
                 const uint32_t most = __reduce_max_sync(kFull, words);
 #pragma unroll 8
@@ -767,6 +803,11 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     lvl_end = 1;
                     level = 0;
                 }
+            }
+            if (G::kRelabel) {
+                // lanes away neither count as idle nor are waited for
+                away = __ballot_sync(kFull, state >= kWaiting) & ~(STREAM ? waiting : 0u);
+                enough = max(1, refill_k - ((refill_k * __popc(away)) >> 5));
             }
             if (__ballot_sync(kFull, state == kActive) == 0u) {
                 // no lane is searching: the region is free for whole-warp searches,
@@ -852,7 +893,10 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     for (int c = 0; c < 2 * P; ++c) {
                         // an a-image is always below low_end
                         at[c] = !G::kRelabel || (c & 1) == 0 || y[c] < low_end ? y[c] : index0 + (y[c] >> shift);
-                        old[c] = SBFS_CHECK((at[c] >> 5) < (held ? 2u * (uint32_t)G::kHalfWords : (uint32_t)LW), b.error)
+                        old[c] = SBFS_CHECK((at[c] >> 5) < (held & G::kBorrowed ? (uint32_t)(LW + T + ring)
+                                                        : held               ? (uint32_t)(__popc(held) * G::kHalfWords)
+                                                                             : (uint32_t)LW),
+                                            b.error)
                                      ? atomicOr(&bm[(at[c] >> 5) * (G::kRelabel ? stride : 32u)], 1u << (at[c] & 31u))
                                      : ~0u;
                     }
