@@ -108,11 +108,18 @@ __device__ __forceinline__ void publish_result(const Batch &b, int64_t k)
     }
 }
 
-__device__ __forceinline__ void record_result(const Batch &b, int64_t k, int n, int32_t len)
+// The length and the violation index.
+__device__ __forceinline__ void store_result(const Batch &b, int64_t k, int n, int32_t len)
 {
     if (b.out_len) b.out_len[k] = len;
-    if (len >= 0 && b.synchronizing) atomicAdd(b.synchronizing, 1ull);
     if (len > cerny_bound(n, b.slack)) atomicMax(b.first_violation, ~(unsigned long long)k);
+}
+
+// ... and the count of synchronizing automata, for kernels that keep none of their own.
+__device__ __forceinline__ void record_result(const Batch &b, int64_t k, int n, int32_t len)
+{
+    store_result(b, k, n, len);
+    if (len >= 0 && b.synchronizing) atomicAdd(b.synchronizing, 1ull);
 }
 
 // Host-side launch helpers implemented in the kernel translation units.

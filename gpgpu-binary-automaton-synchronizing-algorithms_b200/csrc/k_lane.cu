@@ -192,10 +192,25 @@ __device__ __forceinline__ void load_map(const uint8_t *p, int n, uint32_t (&w)[
     for (int c = 0; c < CHUNKS; ++c) w[c] = __funnelshift_r(v[c], v[c + 1], 8u * off);
 }
 
+// The same byte by byte, both maps, into words that are zero.
+template <int NMAX>
+__device__ __forceinline__ void load_bytes(const uint8_t *rec, int lstride, int n, uint32_t (&aw)[(NMAX + 3) / 4],
+                                           uint32_t (&bw)[(NMAX + 3) / 4])
+{
+#pragma unroll
+    for (int c = 0; c < (NMAX + 3) / 4; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (4 * c + j < n) {
+                aw[c] |= (uint32_t)__ldg(rec + 4 * c + j) << (8 * j);
+                bw[c] |= (uint32_t)__ldg(rec + lstride + 4 * c + j) << (8 * j);
+            }
+}
+
 // Automaton k's maps, four images per word.  Aligned words whatever the record
 // stride: a first or last record whose words would reach outside the batch is
 // read byte by byte.
-template <int NMAX>
+template <int NMAX, bool STREAM>
 __device__ __forceinline__ void load_maps(const Batch &b, int64_t k, int n, int64_t count, bool valid,
                                           uint32_t (&aw)[(NMAX + 3) / 4], uint32_t (&bw)[(NMAX + 3) / 4])
 {
@@ -204,6 +219,21 @@ __device__ __forceinline__ void load_maps(const Batch &b, int64_t k, int n, int6
 #pragma unroll
     for (int c = 0; c < CH; ++c) aw[c] = bw[c] = 0u;
     if (!valid) return;
+    if (NMAX <= 8 && !STREAM) {
+        // aligned words or bytes: shorter than words at any alignment (10^6 n = 8
+        // 201 -> 195 us; the streamed form would spill)
+        if (((reinterpret_cast<uintptr_t>(rec) | (uintptr_t)b.lstride) & 3u) == 0) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c)
+                if (4 * c < n) {
+                    aw[c] = __ldg(reinterpret_cast<const uint32_t *>(rec) + c);
+                    bw[c] = __ldg(reinterpret_cast<const uint32_t *>(rec + b.lstride) + c);
+                }
+        } else {
+            load_bytes<NMAX>(rec, b.lstride, n, aw, bw);
+        }
+        return;
+    }
     // an order array may point anywhere in the batch: only its own record is known to be there
     const uint8_t *first = b.order ? rec : b.maps;
     const uint8_t *end = b.order ? rec + 2 * b.lstride : b.maps + (size_t)count * 2u * (size_t)b.lstride;
@@ -214,14 +244,7 @@ __device__ __forceinline__ void load_maps(const Batch &b, int64_t k, int n, int6
         load_map<CH>(rec + b.lstride, n, bw);
         return;
     }
-#pragma unroll
-    for (int c = 0; c < CH; ++c)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (4 * c + j < n) {
-                aw[c] |= (uint32_t)__ldg(rec + 4 * c + j) << (8 * j);
-                bw[c] |= (uint32_t)__ldg(rec + b.lstride + 4 * c + j) << (8 * j);
-            }
+    load_bytes<NMAX>(rec, b.lstride, n, aw, bw);
 }
 
 // Claims the next escalated automaton of the launch for a warp with no lane
@@ -242,23 +265,27 @@ __device__ int64_t claim_escalated(int32_t *list, unsigned long long capacity, u
 
 // One automaton (n <= NMAX) solved by the whole warp inside its region of
 // `region_words` shared words (>= 2^NMAX / 32 + 2^NMAX).  Queue entry:
-// subset | parent index << NMAX | letter << 2*NMAX (letter 1 = b).  Returns the
-// subsets this lane expanded.
-template <int NMAX, bool WORDS, bool STREAM>
-__device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, uint32_t *region, int lane,
-                                            const LaneStream &ls, unsigned long long slot)
+// subset | parent index << NMAX | letter << 2*NMAX (letter 1 = b).  `expanded`:
+// the subsets this lane expanded; the word is lane 0's.
+struct WarpFound {
+    int32_t len;
+    uint32_t expanded;
+    uint64_t w0, w1, w2;
+};
+
+template <int NMAX, bool WORDS>
+__device__ __forceinline__ WarpFound warp_search(const uint8_t *rec, int lstride, int n, uint32_t *region, int lane,
+                                                 int *error)
 {
     uint32_t expanded = 0;
     using G = LaneGeom<NMAX>;
     constexpr int BW = G::kBitmapWords;
     uint32_t *bm = region;        // linear bitmap
     uint32_t *q = region + BW;    // linear queue, 2^NMAX entries
-    const int n = automaton_n(b, k);
-    const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
     // chunks 0 and 1 in lanes 0-15 / 16-31 of t01, chunk 2 (and 3) likewise in t23
-    const uint32_t t01 = table_entry<NMAX>(rec, b.lstride, n, lane >> 4, lane & 15);
-    const uint32_t t23 = G::kChunks > 3   ? table_entry<NMAX>(rec, b.lstride, n, 2 + (lane >> 4), lane & 15)
-                         : G::kChunks > 2 ? table_entry<NMAX>(rec, b.lstride, n, 2, lane & 15)
+    const uint32_t t01 = table_entry<NMAX>(rec, lstride, n, lane >> 4, lane & 15);
+    const uint32_t t23 = G::kChunks > 3   ? table_entry<NMAX>(rec, lstride, n, 2 + (lane >> 4), lane & 15)
+                         : G::kChunks > 2 ? table_entry<NMAX>(rec, lstride, n, 2, lane & 15)
                                           : 0u;
     for (int w = lane; w < BW; w += 32) bm[w] = 0u;
     __syncwarp();
@@ -292,7 +319,7 @@ __device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, u
             break;
         }
         bool fa = false, fb = false;
-        if (has && SBFS_CHECK((ya >> 5) < (uint32_t)BW && (yb >> 5) < (uint32_t)BW, b.error)) {
+        if (has && SBFS_CHECK((ya >> 5) < (uint32_t)BW && (yb >> 5) < (uint32_t)BW, error)) {
             fa = !(atomicOr(&bm[ya >> 5], 1u << (ya & 31u)) & (1u << (ya & 31u)));
             fb = !(atomicOr(&bm[yb >> 5], 1u << (yb & 31u)) & (1u << (yb & 31u)));
         }
@@ -301,9 +328,9 @@ __device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, u
         uint32_t pos = tail + (uint32_t)(__popc(ma & lt) + __popc(mb & lt));
         const uint32_t par = idx << NMAX;
         // every subset enters the queue at most once: 2^NMAX entries never overflow
-        if (fa && SBFS_CHECK(pos < (1u << NMAX), b.error)) q[pos] = ya | par;
+        if (fa && SBFS_CHECK(pos < (1u << NMAX), error)) q[pos] = ya | par;
         pos += fa ? 1u : 0u;
-        if (fb && SBFS_CHECK(pos < (1u << NMAX), b.error)) q[pos] = yb | par | (1u << (2 * NMAX));
+        if (fb && SBFS_CHECK(pos < (1u << NMAX), error)) q[pos] = yb | par | (1u << (2 * NMAX));
         tail += (uint32_t)(__popc(ma) + __popc(mb));
         head = min(head + 32u, lvl_end);
         __syncwarp();
@@ -313,32 +340,45 @@ __device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, u
             ++level;
         }
     }
+    WarpFound r{len, expanded, 0ull, 0ull, 0ull};
+    // at most (NMAX - 1)^2 letters: 2 words at n = 12, 3 at n = 13
+    static_assert(G::kWordU64 <= 3, "words of at most 192 letters");
+    if (WORDS && lane == 0 && len > 0) {
+        // letters from the root: entry at depth d + 1 holds letter d
+        auto set = [&](uint32_t d) {
+            if (d < 64) r.w0 |= 1ull << d;
+            else if (d < 128) r.w1 |= 1ull << (d - 64);
+            else if (G::kWordU64 > 2) r.w2 |= 1ull << (d - 128);
+        };
+        if (found_letter) set(level);
+        uint32_t i = found;
+        for (int d = (int)level - 1; d >= 0; --d) {
+            const uint32_t e = q[i];
+            if ((e >> (2 * NMAX)) & 1u) set((uint32_t)d);
+            i = (e >> NMAX) & G::kMask;
+        }
+    }
+    return r;
+}
+
+// Automaton k searched by the whole warp, and its results.  Returns the subsets
+// this lane expanded.
+template <int NMAX, bool WORDS, bool STREAM>
+__device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, uint32_t *region, int lane,
+                                                    const LaneStream &ls, unsigned long long slot)
+{
+    using G = LaneGeom<NMAX>;
+    const int n = automaton_n(b, k);
+    const uint8_t *rec = b.maps + (size_t)k * 2u * (size_t)b.lstride;
+    const WarpFound r = warp_search<NMAX, WORDS>(rec, b.lstride, n, region, lane, b.error);
     if (lane == 0) {
-        record_result(b, k, n, len);
-        // at most (NMAX - 1)^2 letters: 2 words at n = 12, 3 at n = 13
-        static_assert(G::kWordU64 <= 3, "words of at most 192 letters");
-        uint64_t w0 = 0, w1 = 0, w2 = 0;
+        record_result(b, k, n, r.len);
         if (WORDS) {
-            // letters from the root: entry at depth d + 1 holds letter d
-            if (len > 0) {
-                auto set = [&](uint32_t d) {
-                    if (d < 64) w0 |= 1ull << d;
-                    else if (d < 128) w1 |= 1ull << (d - 64);
-                    else if (G::kWordU64 > 2) w2 |= 1ull << (d - 128);
-                };
-                if (found_letter) set(level);
-                uint32_t i = found;
-                for (int d = (int)level - 1; d >= 0; --d) {
-                    const uint32_t e = q[i];
-                    if ((e >> (2 * NMAX)) & 1u) set((uint32_t)d);
-                    i = (e >> NMAX) & G::kMask;
-                }
-            }
             uint64_t *w = b.out_words + (size_t)k * (size_t)b.word_stride;
-            w[0] = w0;
-            if (b.word_stride > 1) w[1] = w1;
+            w[0] = r.w0;
+            if (b.word_stride > 1) w[1] = r.w1;
             if (G::kWordU64 > 2) {
-                if (b.word_stride > 2) w[2] = w2;
+                if (b.word_stride > 2) w[2] = r.w2;
                 for (int c = 3; c < b.word_stride; ++c) w[c] = 0ull;
             } else {
                 for (int c = 2; c < b.word_stride; ++c) w[c] = 0ull;
@@ -351,22 +391,22 @@ __device__ __forceinline__ uint32_t warp_solve_body(const Batch &b, int64_t k, u
             __threadfence();
             const int c = ls.chunk_of(k);
             const bool early = *(volatile unsigned int *)(ls.chunk_done + c) < (unsigned)ls.chunk_size(c, b.count);
-            EscalResult r;
-            r.k = early ? kEscalInChunk : k;
-            r.len = len;
-            r.pad = 0;
-            r.word[0] = w0;
-            r.word[1] = w1;
-            r.word[2] = w2;
-            ls.escal_out[slot] = r;
+            EscalResult e;
+            e.k = early ? kEscalInChunk : k;
+            e.len = r.len;
+            e.pad = 0;
+            e.word[0] = r.w0;
+            e.word[1] = r.w1;
+            e.word[2] = r.w2;
+            ls.escal_out[slot] = e;
         }
         publish_result(b, k);
     }
     __syncwarp();
-    return expanded;
+    return r.expanded;
 }
 
-// (a call of its own in the streamed kernel, which has three places for it)
+// (a call of its own in the streamed kernel, which has two places for it)
 template <int NMAX, bool WORDS>
 __device__ __noinline__ uint32_t warp_solve_call(const Batch &b, int64_t k, uint32_t *region, int lane,
                                                  const LaneStream &ls, unsigned long long slot)
@@ -435,6 +475,7 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
     bool more = true;
     unsigned long long expanded = 0;   // whole-warp searches
     uint32_t steps_expanded = 0;       // this lane's own searches
+    uint32_t solved = 0;               // lengths it found
     unsigned long long hslot = 0;   // escalation slot of a held automaton
     // The lane's visited bitmap: bit y of subset y below low_end, bit index0 +
     // (y >> shift) of the others (b-images only), word w at bm[w * stride].
@@ -470,7 +511,13 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
             (__popc(served) >= enough && (more || __any_sync(kFull, state == kDone || state == kEscalate)))) {
             const bool outcome = state == kDone || state == kEscalate;
             if (state == kDone) {
-                record_result(b, k, n, res_len);
+                if (STREAM) {
+                    record_result(b, k, n, res_len);
+                } else {
+                    // (counted at the kernel's end: 10^6 n = 5 127 -> 123 us)
+                    store_result(b, k, n, res_len);
+                    solved += res_len >= 0;
+                }
                 if (WORDS) {
                     uint64_t *w = b.out_words + (size_t)k * (size_t)b.word_stride;
                     w[0] = res_len > 0 ? (uint64_t)res_word : 0ull;
@@ -629,7 +676,7 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     bool bad = (n < 1 || n > NMAX || n > b.lstride);
                     const int nn = bad ? 1 : n;
                     uint32_t aw[G::kChunks], bw[G::kChunks];   // four images each, 15 past the last state
-                    load_maps<NMAX>(b, k, nn, count, !bad, aw, bw);
+                    load_maps<NMAX, STREAM>(b, k, nn, count, !bad, aw, bw);
                     {
                         uint32_t high = 0;   // top bits: an image that is no state
                         const uint32_t over = (0x80u - (uint32_t)nn) * 0x01010101u;
@@ -788,10 +835,15 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
                     }
                     if (halves != 0u) words = 0;
                 }
-                const uint32_t most = __reduce_max_sync(kFull, words);
+                if (G::kRelabel) {
+                    const uint32_t most = __reduce_max_sync(kFull, words);
 #pragma unroll 8
-                for (uint32_t w = 0; w < most; ++w)
-                    if (setup) own[w * 32] = 0u;
+                    for (uint32_t w = 0; w < most; ++w)
+                        if (setup) own[w * 32] = 0u;
+                } else if (setup) {
+#pragma unroll
+                    for (int w = 0; w < LW; ++w) own[w * 32] = 0u;
+                }
                 if (setup && state == kActive) {
                     const uint32_t full = (1u << n) - 1u;
                     // the root comes back only through a permutation, and then every
@@ -811,29 +863,31 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
             }
             if (__ballot_sync(kFull, state == kActive) == 0u) {
                 // no lane is searching: the region is free for whole-warp searches,
-                // first of the automata this warp kept
-                for (unsigned held = __ballot_sync(kFull, state == kHeld); held; held &= held - 1u) {
-                    const int64_t e = __shfl_sync(kFull, k, __ffs(held) - 1);
-                    const unsigned long long slot = __shfl_sync(kFull, hslot, __ffs(held) - 1);
-                    expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
-                }
+                // first of the automata this warp kept; then, with no new automata
+                // either, of escalated ones while any can be claimed.  (One loop for
+                // both: with two copies of the search, 10^6 n = 8 took 196 us, not 189,
+                // and n = 7 176, not 167.)
+                unsigned kept = __ballot_sync(kFull, state == kHeld);
                 if (state == kHeld) state = kIdle;
-                if (!more) {
-                    // an outcome decided during set-up (n = 1, a malformed record) is
-                    // written by the next refill pass: take that pass before leaving
-                    if (__any_sync(kFull, state == kDone || state == kEscalate)) continue;
-                    // no new automata either: solve escalated ones while any can be claimed
-                    while (true) {
-                        int64_t e = -1;
-                        unsigned long long slot = 0;
+                // (an outcome decided during set-up -- n = 1, a malformed record -- is
+                // written by the next refill pass: that pass comes before leaving)
+                const bool last = !more && !__any_sync(kFull, state == kDone || state == kEscalate);
+                while (true) {
+                    int64_t e = -1;
+                    unsigned long long slot = 0;
+                    if (kept) {
+                        e = __shfl_sync(kFull, k, __ffs(kept) - 1);
+                        slot = __shfl_sync(kFull, hslot, __ffs(kept) - 1);
+                        kept &= kept - 1u;
+                    } else if (last) {
                         if (lane == 0) e = claim_escalated(escal_list, escal_capacity, escal_claim, slot);
                         e = __shfl_sync(kFull, e, 0);
                         slot = __shfl_sync(kFull, slot, 0);
-                        if (e < 0) break;
-                        expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
                     }
-                    break;
+                    if (e < 0) break;
+                    expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
                 }
+                if (last) break;
                 continue;
             }
         }
@@ -930,6 +984,10 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
     expanded += steps_expanded;
     for (int o = 16; o; o >>= 1) expanded += __shfl_down_sync(kFull, expanded, o);
     if (lane == 0 && b.expanded) atomicAdd(b.expanded, expanded);
+    if (!STREAM) {
+        solved = __reduce_add_sync(kFull, solved);
+        if (lane == 0 && b.synchronizing && solved) atomicAdd(b.synchronizing, (unsigned long long)solved);
+    }
 }
 
 template <int NMAX>
