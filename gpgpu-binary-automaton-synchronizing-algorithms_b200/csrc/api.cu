@@ -35,8 +35,9 @@ cudaError_t plan_autotune(sbfs_handle *h, Plan &plan);
 int hash_max_ctas_per_sm(int size, int max_n);
 cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
                         unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st);
-size_t mid_spill_entries(int sm_count);
-cudaError_t launch_mid(int sm_count, const Batch &b, uint64_t *spill, int32_t *left_list,
+int mid_ctas(int sm_count, int64_t count);
+size_t mid_spill_entries(int max_n);
+cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, int32_t *left_list,
                        unsigned long long *left_count, unsigned long long *ticket, cudaStream_t st);
 cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
                         unsigned long long *ticket, cudaStream_t st);
@@ -392,9 +393,11 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                 bh.order = list;
                 bh.range_dev = ctr->heavy_range[c];
                 DevBuf &spill = L.mid_spill[c - 2];
-                CK(spill.reserve(mid_spill_entries(h->sm_count) * sizeof(uint64_t)), "allocating queue spill");
-                CK(launch_mid(h->sm_count, bh, spill.as<uint64_t>(), list + escal_entries, &ctr->left_range[c][1],
-                              &ctr->heavy_ticket[c], cs),
+                const int mctas = mid_ctas(h->sm_count, j.count);
+                CK(spill.reserve(std::max<size_t>(1, mctas * mid_spill_entries(kClassMaxN[c])) * sizeof(uint64_t)),
+                   "allocating queue spill");
+                CK(launch_mid(mctas, kClassMaxN[c], bh, spill.as<uint64_t>(), list + escal_entries,
+                              &ctr->left_range[c][1], &ctr->heavy_ticket[c], cs),
                    "launching hand-off kernel");
                 *launches += 1;
                 if (c == 3) {

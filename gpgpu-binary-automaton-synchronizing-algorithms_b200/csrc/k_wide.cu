@@ -19,6 +19,7 @@
 // n = 24, 26, 28 x (64 random + C_n + permutation-plus-merge), one Verify call:
 // 18.0 ms with every automaton on the level slots, 0.42 ms with k_hash and this
 // kernel before them.
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -221,15 +222,15 @@ __global__ void __launch_bounds__(kWideThreads, 1)
 // 2^rank(a) + 2^rank(b) bits, 2^17 at most -- and a queue whose first 8192
 // subsets stay on chip: 65 KB, so three CTAs per SM instead of the one that
 // k_cta.cu's 2^20-bit bitmap allows, and no trips to global memory but for the
-// widest searches.  Those continue in a spill of 2^17 entries per CTA, which no
-// search can outgrow: its subsets have different bits.  Ranks that need more bits
-// (n > 16 only) are left to k_cta.  The widest search of a batch bounds the
+// widest searches.  Those continue in a spill of 2^17 entries per CTA, those on
+// chip included (2^16 for n <= 16), which no search can outgrow: its subsets have
+// different bits.  Ranks that need more bits (n > 17 only) are left to k_cta.  The widest search of a batch bounds the
 // launch, hence 512 threads: 30K random n = 20 took 0.330 ms with k_cta alone,
 // 0.334 with 256 threads here, 0.315 with 512, 0.326 with 1024 (two CTAs per SM);
 // 200K mixed n = 6..20 0.611, 0.599, 0.591 and 0.611 ms.
 constexpr int kMidThreads = 512;
 constexpr uint32_t kMidLimit = 8192;
-constexpr uint32_t kMidSpill = 1u << 17;
+constexpr uint32_t kMidMaxSubsets = 1u << 17;   // a search's, by its bitmap
 constexpr int kMidWords = 4096;
 constexpr int kMidChunks = 5;
 
@@ -249,14 +250,14 @@ struct MidCtl {
 };
 
 __global__ void __launch_bounds__(kMidThreads, 3)
-    k_mid(const __grid_constant__ Batch b, uint2 *spill_base, int32_t *left_list, unsigned long long *left_count,
-          unsigned long long *ticket)
+    k_mid(const __grid_constant__ Batch b, uint2 *spill_base, uint32_t spill_entries, int32_t *left_list,
+          unsigned long long *left_count, unsigned long long *ticket)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MidSmem &S = *reinterpret_cast<MidSmem *>(smem_raw);
     __shared__ MidCtl ctl;
     // {subset | letter-is-b << 31, parent} of the queue entries from kMidLimit on
-    uint2 *const spill = spill_base + (size_t)blockIdx.x * kMidSpill;
+    uint2 *const spill = spill_base + (size_t)blockIdx.x * spill_entries;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const unsigned lt = (1u << lane) - 1u;
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(kMidThreads, 3)
                     if (p < kMidLimit) {
                         S.queue[p] = e;
                         S.parent[p] = (uint16_t)i;
-                    } else if (SBFS_CHECK(p - kMidLimit < kMidSpill, b.error)) {
+                    } else if (SBFS_CHECK(p - kMidLimit < spill_entries, b.error)) {
                         spill[p - kMidLimit] = make_uint2(e, i);
                     }
                 };
@@ -438,23 +439,32 @@ cudaError_t allow_smem(F *kernel, size_t bytes, std::atomic<int> (&done)[16])
 
 }  // namespace
 
-// uint64 entries of the spill that launch_mid takes
-size_t mid_spill_entries(int sm_count)
+// CTAs that `count` hand-offs at most can keep busy
+int mid_ctas(int sm_count, int64_t count)
 {
-    return 3 * (size_t)sm_count * kMidSpill;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(3 * (int64_t)sm_count, count));
 }
 
-// Solves the automata of b (n <= 20, three CTAs per SM); those whose ranks need
-// more than 2^17 bits (n > 16) are appended to left_list.
-cudaError_t launch_mid(int sm_count, const Batch &b, uint64_t *spill, int32_t *left_list,
+// uint64 entries per CTA of the spill that launch_mid takes, for automata of
+// up to max_n states
+size_t mid_spill_entries(int max_n)
+{
+    const size_t most = max_n < 17 ? (size_t)1 << max_n : kMidMaxSubsets;
+    return most > kMidLimit ? most - kMidLimit : 0;
+}
+
+// Solves the automata of b (at most max_n <= 20 states); those whose ranks need
+// more than 2^17 bits (n > 17 only) are appended to left_list.
+cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, int32_t *left_list,
                        unsigned long long *left_count, unsigned long long *ticket, cudaStream_t st)
 {
-    if (sm_count < 1 || !left_list || !left_count) return cudaErrorInvalidValue;
+    if (ctas < 1 || !left_list || !left_count) return cudaErrorInvalidValue;
     static std::atomic<int> done[16];
     const cudaError_t e = allow_smem(k_mid, sizeof(MidSmem), done);
     if (e != cudaSuccess) return e;
-    k_mid<<<3 * sm_count, kMidThreads, sizeof(MidSmem), st>>>(b, reinterpret_cast<uint2 *>(spill), left_list,
-                                                              left_count, ticket);
+    k_mid<<<ctas, kMidThreads, sizeof(MidSmem), st>>>(b, reinterpret_cast<uint2 *>(spill),
+                                                      (uint32_t)mid_spill_entries(max_n), left_list, left_count,
+                                                      ticket);
     return cudaGetLastError();
 }
 
