@@ -373,7 +373,10 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
             if (per_sm < 1) return fail(h, SBFS_ECUDA, "CTA-wide kernel does not fit on an SM");
             const int ctas = std::min(P.cta.ctas, per_sm * h->sm_count);
             const bool direct = plain || ticket_override;
-            if (direct || c == 3)
+            // k_mid leaves nothing of n <= 17.  (A device batch's largest n is the caller's
+            // word: its members are launched for whatever they are.)
+            const bool leaves = c == 3 && (j.ns ? !(j.min_n > 0 && j.max_n <= 17) : j.n_uniform > 17);
+            if (direct || leaves)
                 CK(L.heavy_queue[c].reserve(cta_queue_entries(nb, ctas) * sizeof(uint64_t)), "allocating CTA queues");
             if (direct) {
                 CK(launch_cta(nb, threads, ctas, bc, L.heavy_queue[c].as<uint64_t>(), ticket, cs),
@@ -400,7 +403,7 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                               &ctr->left_range[c][1], &ctr->heavy_ticket[c], cs),
                    "launching hand-off kernel");
                 *launches += 1;
-                if (c == 3) {
+                if (leaves) {
                     bh.order = list + escal_entries;
                     bh.range_dev = ctr->left_range[c];
                     CK(launch_cta(nb, threads, ctas, bh, L.heavy_queue[c].as<uint64_t>(), &ctr->left_ticket[c], cs),
