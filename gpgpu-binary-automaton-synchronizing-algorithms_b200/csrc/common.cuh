@@ -78,6 +78,7 @@ __device__ __forceinline__ void resolve_work(const Batch &b, int64_t &count, con
     if (b.range_dev) {
         order = b.order + b.range_dev[0];
         count = (int64_t)b.range_dev[1];
+        if (!SBFS_CHECK(count <= b.count, b.error)) count = b.count;
     } else {
         order = b.order;
         count = b.count;
@@ -120,6 +121,14 @@ __device__ __forceinline__ void record_result(const Batch &b, int64_t k, int n, 
 {
     store_result(b, k, n, len);
     if (len >= 0 && b.synchronizing) atomicAdd(b.synchronizing, 1ull);
+}
+
+// Appends automaton k to a hand-off list with room for every automaton of the
+// launch's job.
+__device__ __forceinline__ void hand_off(const Batch &b, int32_t *list, unsigned long long *count, int64_t k)
+{
+    const unsigned long long slot = atomicAdd(count, 1ull);
+    if (SBFS_CHECK(slot < (unsigned long long)b.count, b.error)) list[slot] = (int32_t)k;
 }
 
 // Host-side launch helpers implemented in the kernel translation units.

@@ -251,7 +251,7 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
                 if (!sure || na == nb || ya == full || yb == full || tail >= G::kSetLimit) break;
                 x = na ? ya : yb;
                 W.store[na ? pa : pb] = x;
-                W.push(tail, x, head, na ? 0u : 1u);
+                if (SBFS_CHECK(tail < G::kLimit, b.error)) W.push(tail, x, head, na ? 0u : 1u);
                 __syncwarp();
                 expanded += lane < 2 ? 1u : 0u;
                 head = tail++;
@@ -282,7 +282,7 @@ __device__ __noinline__ uint32_t inverse_search(const Batch &b, int64_t k, int n
             const unsigned m = __ballot_sync(kFull, fresh);
             if (m) {
                 const uint32_t p = tail + added + (uint32_t)__popc(m & ((1u << lane) - 1u));
-                if (fresh && p < G::kSetLimit) W.push(p, y, head + set, letter);
+                if (fresh && p < G::kSetLimit) W.push(p, y, head + set, letter);   // (the limit ends the search)
                 if (!(m & (m - 1u))) next = __shfl_sync(kFull, y, __ffs(m) - 1);
                 added += (uint32_t)__popc(m);
             }
@@ -406,6 +406,7 @@ __device__ __forceinline__ Forward forward_search(const Batch &b, int n, HashWar
             break;
         }
         uint32_t p = tail + (uint32_t)(__popc(ma & lt) + __popc(mb & lt));
+        if (!SBFS_CHECK(p + (fa ? 1u : 0u) + (fb ? 1u : 0u) <= G::kLimit, b.error)) fa = fb = false;
         if (fa) W.push(p++, ya, idx, 0u);
         if (fb) W.push(p, yb, idx, 1u);
         tail += added;
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32, HashGeom<MA
                 r = inverse_search(b, k, n, av, bv, W, lane);
                 expanded += r & ~kUnsettled;
             }
-            if ((r & kUnsettled) && lane == 0) heavy_list[atomicAdd(heavy_count, 1ull)] = (int32_t)k;
+            if ((r & kUnsettled) && lane == 0) hand_off(b, heavy_list, heavy_count, k);
             __syncwarp();
             continue;
         }

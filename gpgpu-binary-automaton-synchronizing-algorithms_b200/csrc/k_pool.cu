@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(512) k_pool(Batch b, int q_smem, int grab, uin
             const int leader = __ffs(em) - 1;
             if (lane == leader) pos = atomicAdd(heavy.count, (unsigned long long)__popc(em));
             pos = __shfl_sync(kFull, pos, leader);
-            if (esc) heavy.list[pos + __popc(em & ((1u << lane) - 1u))] = (int32_t)my_k;
+            const unsigned long long slot = pos + __popc(em & ((1u << lane) - 1u));
+            if (esc && SBFS_CHECK(slot < (unsigned long long)b.count, b.error)) heavy.list[slot] = (int32_t)my_k;
         }
 
         // ---- finished slots: result, word, bitmap clear ---------------------

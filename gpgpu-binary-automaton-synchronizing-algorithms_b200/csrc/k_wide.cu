@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 break;
             }
             if (outgrown) {
-                if (tid == 0) left_list[atomicAdd(left_count, 1ull)] = (int32_t)k;
+                if (tid == 0) hand_off(b, left_list, left_count, k);
                 break;
             }
             if (added == 0) {
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kMidThreads, 3)
         const int n = ctl.n;
         const uint32_t low_end = ctl.low_end, index0 = ctl.index0, shift = ctl.shift, bits = ctl.bits;
         if (bits > 32u * kMidWords) {
-            if (tid == 0) left_list[atomicAdd(left_count, 1ull)] = (int32_t)k;
+            if (tid == 0) hand_off(b, left_list, left_count, k);
             __syncthreads();   // every thread has read ctl
             continue;
         }
