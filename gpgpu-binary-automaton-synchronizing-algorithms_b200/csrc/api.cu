@@ -1577,7 +1577,7 @@ int32_t sbfs_describe_plan(sbfs_handle *h, char *buf, int32_t len)
                           "{\"class\":2,\"max_n\":16,\"kernel\":\"k_hash+k_mid\",\"slots\":%d,"
                           "\"uniform_n13\":\"k_lane<13>\",\"ring13\":%d,\"ctas13\":%d,"
                           "\"uniform_n14\":\"%s\",\"ring14\":%d,\"ctas14\":%d},",
-                          P.class2_hash == 2 ? 4096 : 2048, P.lane13.ring, P.lane13.ctas,
+                          P.class2_hash == 2 ? 2048 : 1024, P.lane13.ring, P.lane13.ctas,
                           P.use_lane14 ? "k_lane<14>" : "k_hash+k_mid", P.lane14.ring, P.lane14.ctas);
         } else if (lane) {
             const LaneShape &l = P.lane[c];
@@ -1587,7 +1587,7 @@ int32_t sbfs_describe_plan(sbfs_handle *h, char *buf, int32_t len)
                           c, kClassMaxN[c], l.nmax, l.warps, l.ring, l.refill_k, l.ctas);
         } else if (c == 2 && P.class2_hash) {
             std::snprintf(tmp, sizeof tmp, "{\"class\":2,\"max_n\":16,\"kernel\":\"k_hash+k_mid\",\"slots\":%d},",
-                          P.class2_hash == 2 ? 4096 : 2048);
+                          P.class2_hash == 2 ? 2048 : 1024);
         } else {
             const PoolShape &q = P.pool[c];
             std::snprintf(tmp, sizeof tmp,
