@@ -165,7 +165,7 @@ struct EscalResult {
     int64_t k;          // automaton, or kEscalInChunk: its chunk's copy has the result
     int32_t len;
     int32_t pad;
-    uint64_t word[3];   // n <= 13: at most 144 letters
+    uint64_t word[3];   // n <= 14: at most 169 letters
 };
 struct LaneStream {
     const unsigned int *chunk_ready;   // nonzero once chunk c's records are on the device

@@ -613,7 +613,8 @@ struct HashLaunch {
 
 }  // namespace
 
-// size 1: 2048 hash slots per warp (1536 subsets), size 2: 4096 (3072 subsets);
+// size 1: 1536 subsets per warp and a store of 1024 words (n <= 16) or 2048, size 2:
+// twice that; as a hash set three quarters of the store's words.
 // max_n: the largest n of the launch's automata (more than 20 states: size 2 only)
 int hash_max_ctas_per_sm(int size, int max_n)
 {

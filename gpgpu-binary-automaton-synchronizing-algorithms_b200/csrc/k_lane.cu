@@ -84,9 +84,10 @@ constexpr int kStep = 4;   // subsets a lane expands per step (their 2 * kStep i
 // and CTAs of that many that the registers must allow for
 __host__ __device__ constexpr int lane_cta_warps(int nmax, int warps) { return nmax <= 8 ? warps : 1; }
 __host__ __device__ constexpr int lane_min_ctas(int nmax) { return nmax <= 8 ? 4 : 11; }
-// At n = 13 and 14 fewer warps fit on an SM (four, two), and six subsets per
+// At n = 13 and 14 fewer warps fit on an SM (six, three), and six subsets per
 // step hide more of each warp's latency: 2^21 automata at n = 14 4.83 -> 4.64 ms,
-// the n = 13 streamed kernel 2.19 -> 2.09 ms (eight: no better than six)
+// the n = 13 streamed kernel 2.19 -> 2.09 ms (eight: no better than six; measured
+// with four and two warps, one bit per subset and lane)
 constexpr int kStepWide = 6;
 
 __host__ __device__ constexpr int low_bit4(int v)

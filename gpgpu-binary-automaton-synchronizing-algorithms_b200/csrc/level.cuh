@@ -133,7 +133,7 @@ public:
     // levels are narrow and nothing awaits set-up, one launch of an 8-CTA
     // cluster that runs up to `narrow_levels` narrow levels -- then copy slot
     // states back
-    // (async); results go to `out` when out.out_len is set (batch mode)
+    // (async); results go to `out` too when out.first_violation is set (batch mode)
     cudaError_t launch(int levels, const Batch &out, int narrow_levels = 0);
     cudaError_t launch_try(int n);
     // wait for the last launch and collect finished slots (frees their memory)

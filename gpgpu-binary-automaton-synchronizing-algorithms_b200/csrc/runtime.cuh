@@ -166,8 +166,9 @@ struct Plan {
     int use_pool[2];     // classes 0, 1: 1 = warp-pooled kernel instead of one automaton per lane
     int class3_level;    // class 3: 1 = bitmaps in HBM (level slots) instead of shared memory (k_cta)
     // classes 2 and 3 (class 3 in shared memory): a warp each first (k_hash), k_mid
-    // and k_cta for their hand-offs, with 1 = 1536 or 2 = 3072 subsets per warp;
-    // 0 = the pooled kernel (class 2) or k_cta alone (class 3)
+    // and k_cta for their hand-offs, with 1 = 1536 or 2 = 3072 subsets per warp (768
+    // or 1536 for n <= 16 where ranks need the hash set); 0 = the pooled kernel
+    // (class 2) or k_cta alone (class 3)
     int class2_hash;
     int class3_hash;
     int tuned;           // 1 when the autotuner (or its cache) chose the shapes
