@@ -865,22 +865,29 @@ __global__ void __launch_bounds__(lane_cta_warps(NMAX, 8) * 32, lane_min_ctas(NM
             if (__ballot_sync(kFull, state == kActive) == 0u) {
                 // no lane is searching: the region is free for whole-warp searches,
                 // first of the automata this warp kept; then, with no new automata
-                // either, of escalated ones while any can be claimed.  (One loop for
-                // both: with two copies of the search, 10^6 n = 8 took 196 us, not 189,
-                // and n = 7 176, not 167.)
+                // either, of escalated ones while any can be claimed.
                 unsigned kept = __ballot_sync(kFull, state == kHeld);
+                if (G::kRelabel)
+                    for (; kept; kept &= kept - 1u) {
+                        const int64_t e = __shfl_sync(kFull, k, __ffs(kept) - 1);
+                        const unsigned long long slot = __shfl_sync(kFull, hslot, __ffs(kept) - 1);
+                        expanded += warp_solve<NMAX, WORDS, STREAM>(b, e, base, lane, ls, slot);
+                    }
                 if (state == kHeld) state = kIdle;
                 // (an outcome decided during set-up -- n = 1, a malformed record -- is
                 // written by the next refill pass: that pass comes before leaving)
                 const bool last = !more && !__any_sync(kFull, state == kDone || state == kEscalate);
-                while (true) {
+                // (n <= 8: one loop for both.  With two copies of the search 10^6 n = 8
+                // took 196 us, not 191, and n = 7 176, not 170; 500,000 n = 14 take
+                // 766 with one, 759 with two.)
+                while (kept || last) {
                     int64_t e = -1;
                     unsigned long long slot = 0;
-                    if (kept) {
+                    if (!G::kRelabel && kept) {
                         e = __shfl_sync(kFull, k, __ffs(kept) - 1);
                         slot = __shfl_sync(kFull, hslot, __ffs(kept) - 1);
                         kept &= kept - 1u;
-                    } else if (last) {
+                    } else {
                         if (lane == 0) e = claim_escalated(escal_list, escal_capacity, escal_claim, slot);
                         e = __shfl_sync(kFull, e, 0);
                         slot = __shfl_sync(kFull, slot, 0);
