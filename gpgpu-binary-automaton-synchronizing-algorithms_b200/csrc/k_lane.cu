@@ -24,8 +24,8 @@
 // automata take bitmaps from a pool of the warp's, in the order in which they came,
 // and when that is used up the whole column (bitmap, table, ring) of a lane that
 // does not search.  Batches of such automata alone, one permutation and one random
-// map: half of the lanes search, 200,000 n = 12 in 0.73 ms and 100,000 n = 13 in
-// 0.76 (with the pool alone 2.02 and 4.44, with a bitmap of 2^n bits per lane 0.95
+// map: half of the lanes search, 200,000 n = 12 in 0.72 ms and 100,000 n = 13 in
+// 0.75 (with the pool alone 2.02 and 4.44, with a bitmap of 2^n bits per lane 0.95
 // and 0.99).
 // Relabelling changes neither the order of the search nor its words.  1M n = 12
 // device-resident: 0.592 -> 0.472 ms; 500K n = 14: 1.158 -> 0.760 ms; a Verify call
