@@ -42,51 +42,6 @@ cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, int
 cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
                         unsigned long long *ticket, cudaStream_t st);
 
-cudaError_t DevBuf::reserve(size_t want)
-{
-    if (want <= bytes && ptr) return cudaSuccess;
-    release();
-    size_t sz = std::max<size_t>(want, 256);
-    cudaError_t e = cudaMalloc(&ptr, sz);
-    if (e != cudaSuccess) {
-        ptr = nullptr;
-        cudaGetLastError();
-        return e;
-    }
-    bytes = sz;
-    return cudaSuccess;
-}
-
-void DevBuf::release()
-{
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-}
-
-cudaError_t HostBuf::reserve(size_t want)
-{
-    if (want <= bytes && ptr) return cudaSuccess;
-    release();
-    size_t sz = std::max<size_t>(want, 256);
-    // mapped, so kernels may store into it (the streamed host path's chunk flags)
-    cudaError_t e = cudaHostAlloc(&ptr, sz, cudaHostAllocMapped);
-    if (e != cudaSuccess) {
-        ptr = nullptr;
-        cudaGetLastError();
-        return e;
-    }
-    bytes = sz;
-    return cudaSuccess;
-}
-
-void HostBuf::release()
-{
-    if (ptr) cudaFreeHost(ptr);
-    ptr = nullptr;
-    bytes = 0;
-}
-
 }  // namespace sbfs
 
 using namespace sbfs;
@@ -1152,7 +1107,16 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
         }
         CK(cudaEventRecord(L.ev_k0, L.stream), "recording event");
         if (!plain) {
-            // one chunk: counters, bucketing, class kernels, copies out
+            auto copy_results = [&]() -> sbfs_status {
+                if (out_len)
+                    CK(cudaMemcpyAsync(dst_len, d_len, lb, cudaMemcpyDeviceToHost, L.stream), "copying lengths");
+                if (out_words)
+                    CK(cudaMemcpyAsync(dst_words, d_words, wb, cudaMemcpyDeviceToHost, L.stream), "copying words");
+                return SBFS_OK;
+            };
+            // one chunk: counters, bucketing, class kernels, copies out.  (Those into a
+            // caller's pinned buffers stay out of a graph: the buffers are the caller's to
+            // free, and others may come at their addresses.)
             auto body = [&]() -> sbfs_status {
                 sbfs_status bs =
                     reset_counters(h, L, escal_list_entries(h, j), fused ? fused_end - kCounterBytes : 0);
@@ -1163,10 +1127,7 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
                        "copying results");
                     return SBFS_OK;
                 }
-                if (out_len)
-                    CK(cudaMemcpyAsync(dst_len, d_len, lb, cudaMemcpyDeviceToHost, L.stream), "copying lengths");
-                if (out_words)
-                    CK(cudaMemcpyAsync(dst_words, d_words, wb, cudaMemcpyDeviceToHost, L.stream), "copying words");
+                if (!pin_out && (bs = copy_results())) return bs;
                 CK(cudaMemcpyAsync(L.h_counters.ptr, L.counters.ptr, sizeof(DevCounters), cudaMemcpyDeviceToHost,
                                    L.stream),
                    "copying counters");
@@ -1177,6 +1138,7 @@ sbfs_status solve_host(sbfs_handle *h, const uint8_t *maps, int32_t lstride, con
                                                           n_uniform, min_n, max_n, word_stride)
                                               : std::string();
             if ((s = run_maybe_captured(h, L, key, graphable, &launches, body))) return s;
+            if (pin_out && (s = copy_results())) return s;
             CK(cudaEventRecord(L.ev_k1, L.stream), "recording event");
         } else {
             CK(cudaMemcpyAsync(L.maps.ptr, src_maps, cnt * rec, cudaMemcpyHostToDevice, L.stream), "copying records");

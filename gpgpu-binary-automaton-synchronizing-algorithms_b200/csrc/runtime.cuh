@@ -13,6 +13,7 @@
 
 #include <cuda_runtime.h>
 
+#include "buffers.hpp"
 #include "classes.cuh"
 #include "common.cuh"
 #include "copy_pool.hpp"
@@ -47,24 +48,6 @@ struct DevCounters {
 // A lane's counters, and the escalation lists behind them: one memset resets both.
 // (A small staged batch has its results between the two, see kFusedBytes.)
 constexpr size_t kCounterBytes = (sizeof(DevCounters) + 255) & ~(size_t)255;
-
-// Grow-only device allocation.
-struct DevBuf {
-    void *ptr = nullptr;
-    size_t bytes = 0;
-    cudaError_t reserve(size_t want);
-    void release();
-    template <class T> T *as() const { return static_cast<T *>(ptr); }
-};
-
-// Grow-only pinned host allocation.
-struct HostBuf {
-    void *ptr = nullptr;
-    size_t bytes = 0;
-    cudaError_t reserve(size_t want);
-    void release();
-    template <class T> T *as() const { return static_cast<T *>(ptr); }
-};
 
 // The streamed host path (uniform n <= 14 on the per-lane kernels): records go
 // in chunk by chunk on the handle's copy-in stream while one kernel runs, and
@@ -124,7 +107,7 @@ struct Lane {
     uint64_t *user_words = nullptr;
     int32_t word_stride = 0;
     // CUDA graphs of launch sequences already seen on this lane, keyed by their
-    // pointers and sizes; `sig` is the lane's buffer addresses at capture time
+    // pointers and sizes; `sig` stands for the lane's buffers at capture time
     struct Graph {
         cudaGraphExec_t exec;
         uint64_t sig;
@@ -134,14 +117,10 @@ struct Lane {
     std::set<std::string> seen;
     uint64_t signature() const
     {
-        uint64_t x = 1469598103934665603ull;
-        for (const DevBuf *d : {&maps, &len, &words, &spill, &order, &counters, &cta_queue, &tickets,
-                                &spill_c[0], &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2],
-                                &heavy[3], &heavy[4], &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3], &mid_spill[0], &mid_spill[1]})
-            x = (x ^ reinterpret_cast<uint64_t>(d->ptr)) * 1099511628211ull;
-        for (const HostBuf *b : {&h_counters, &h_maps, &h_len, &h_words})
-            x = (x ^ reinterpret_cast<uint64_t>(b->ptr)) * 1099511628211ull;
-        return x;
+        return buffers_signature({&maps, &len, &words, &spill, &order, &counters, &cta_queue, &tickets, &spill_c[0],
+                                  &spill_c[1], &spill_c[2], &heavy[0], &heavy[1], &heavy[2], &heavy[3], &heavy[4],
+                                  &heavy_queue[0], &heavy_queue[1], &heavy_queue[2], &heavy_queue[3], &mid_spill[0],
+                                  &mid_spill[1], &h_counters, &h_maps, &h_len, &h_words});
     }
     void drop_graphs()
     {
