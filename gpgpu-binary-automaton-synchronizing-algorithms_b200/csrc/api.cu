@@ -34,11 +34,12 @@ cudaError_t launch_cta(int nb_max, int threads, int ctas, const Batch &b, uint64
 cudaError_t plan_autotune(sbfs_handle *h, Plan &plan);
 int hash_max_ctas_per_sm(int size, int max_n);
 cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
-                        unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st);
+                        unsigned long long *heavy_count, int32_t *wide_list, unsigned long long *wide_count,
+                        unsigned long long *ticket, cudaStream_t st);
 int mid_ctas(int sm_count, int64_t count);
 size_t mid_spill_entries(int max_n);
-cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, int32_t *left_list,
-                       unsigned long long *left_count, unsigned long long *ticket, cudaStream_t st);
+cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, unsigned long long *ticket,
+                       cudaStream_t st);
 cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
                         unsigned long long *ticket, cudaStream_t st);
 
@@ -328,8 +329,8 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
             if (per_sm < 1) return fail(h, SBFS_ECUDA, "CTA-wide kernel does not fit on an SM");
             const int ctas = std::min(P.cta.ctas, per_sm * h->sm_count);
             const bool direct = plain || ticket_override;
-            // k_mid leaves nothing of n <= 17.  (A device batch's largest n is the caller's
-            // word: its members are launched for whatever they are.)
+            // No automaton of n <= 17 needs more bits than k_mid has.  (A device batch's largest
+            // n is the caller's word: its members are launched for whatever they are.)
             const bool leaves = c == 3 && (j.ns ? !(j.min_n > 0 && j.max_n <= 17) : j.n_uniform > 17);
             if (direct || leaves)
                 CK(L.heavy_queue[c].reserve(cta_queue_entries(nb, ctas) * sizeof(uint64_t)), "allocating CTA queues");
@@ -337,15 +338,18 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                 CK(launch_cta(nb, threads, ctas, bc, L.heavy_queue[c].as<uint64_t>(), ticket, cs),
                    "launching CTA-wide kernel");
             } else {
-                // one warp per automaton; what is wide both ways goes on to k_mid, and
-                // class 3's largest ranks from there to the CTA-wide kernel, on the same stream
+                // one warp per automaton; what is wide both ways goes on to k_mid, and class 3's
+                // largest ranks to the CTA-wide kernel.  Those two run side by side, each as long
+                // as its widest searches (600 n = 18 of two rank 17 letters: 736 us after one
+                // another, 546 so), k_cta, whose are wider, first
                 const int hper = hash_max_ctas_per_sm(size, kClassMaxN[c]);
                 if (hper < 1) return fail(h, SBFS_ECUDA, "hash-set kernel does not fit on an SM");
-                // left by k_hash | left by k_mid
+                // for k_mid | for k_cta
                 CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off lists");
                 int32_t *list = L.heavy[c].as<int32_t>();
                 const int hctas = (int)std::min<int64_t>(hper * h->sm_count, std::max<int64_t>(j.count, 1));
-                CK(launch_hash(size, kClassMaxN[c], hctas, bc, list, &ctr->heavy_range[c][1], ticket, cs),
+                CK(launch_hash(size, kClassMaxN[c], hctas, bc, list, &ctr->heavy_range[c][1],
+                               leaves ? list + escal_entries : nullptr, &ctr->left_range[c][1], ticket, cs),
                    "launching hash-set kernel");
                 Batch bh = bc;
                 bh.order = list;
@@ -354,17 +358,22 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                 const int mctas = mid_ctas(h->sm_count, j.count);
                 CK(spill.reserve(std::max<size_t>(1, mctas * mid_spill_entries(kClassMaxN[c])) * sizeof(uint64_t)),
                    "allocating queue spill");
-                CK(launch_mid(mctas, kClassMaxN[c], bh, spill.as<uint64_t>(), list + escal_entries,
-                              &ctr->left_range[c][1], &ctr->heavy_ticket[c], cs),
-                   "launching hand-off kernel");
-                *launches += 1;
                 if (leaves) {
-                    bh.order = list + escal_entries;
-                    bh.range_dev = ctr->left_range[c];
-                    CK(launch_cta(nb, threads, ctas, bh, L.heavy_queue[c].as<uint64_t>(), &ctr->left_ticket[c], cs),
+                    Batch bw = bc;
+                    bw.order = list + escal_entries;
+                    bw.range_dev = ctr->left_range[c];
+                    CK(cudaEventRecord(L.ev_wide, cs), "recording event");
+                    CK(cudaStreamWaitEvent(L.aux[3], L.ev_wide, 0), "ordering streams");
+                    CK(launch_cta(nb, threads, ctas, bw, L.heavy_queue[c].as<uint64_t>(), &ctr->left_ticket[c],
+                                  L.aux[3]),
                        "launching CTA-wide kernel");
+                    CK(cudaEventRecord(L.ev_join[3], L.aux[3]), "recording event");
                     *launches += 1;
                 }
+                CK(launch_mid(mctas, kClassMaxN[c], bh, spill.as<uint64_t>(), &ctr->heavy_ticket[c], cs),
+                   "launching hand-off kernel");
+                *launches += 1;
+                if (leaves) CK(cudaStreamWaitEvent(cs, L.ev_join[3], 0), "ordering streams");
             }
         } else if (c < 3) {
             const PoolShape &s = P.pool[c];
@@ -410,7 +419,7 @@ sbfs_status enqueue_kernels(sbfs_handle *h, Lane &L, const Job &j, int *launches
                 CK(L.heavy[c].reserve(2 * escal_entries * sizeof(int32_t)), "allocating hand-off list");
                 int32_t *list = L.heavy[c].as<int32_t>();
                 const int hctas = (int)std::min<int64_t>(hper * h->sm_count, std::max<int64_t>(j.count, 1));
-                CK(launch_hash(2, SBFS_MAX_N, hctas, bc, list, &ctr->heavy_range[c][1], ticket, cs),
+                CK(launch_hash(2, SBFS_MAX_N, hctas, bc, list, &ctr->heavy_range[c][1], nullptr, nullptr, ticket, cs),
                    "launching hash-set kernel");
                 bc.order = list;
                 bc.range_dev = ctr->heavy_range[c];
@@ -1316,11 +1325,12 @@ sbfs_status sbfs_create(const sbfs_config *cfg, sbfs_handle **out)
             (e = cudaEventCreate(&L.ev_k0)) != cudaSuccess || (e = cudaEventCreate(&L.ev_k1)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&L.ev_done, cudaEventDisableTiming)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&L.ev_in, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&L.ev_fork, cudaEventDisableTiming)) != cudaSuccess) {
+            (e = cudaEventCreateWithFlags(&L.ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
+            (e = cudaEventCreateWithFlags(&L.ev_wide, cudaEventDisableTiming)) != cudaSuccess) {
             sbfs_destroy(h);
             return cuda_fail(nullptr, e, "creating streams");
         }
-        for (int c = 0; c < 3; ++c)
+        for (int c = 0; c < 4; ++c)
             // (class 3 runs on the lane's own stream; smaller classes come after it)
             if ((e = cudaStreamCreateWithPriority(&L.aux[c], cudaStreamNonBlocking,
                                                   std::min(prio_least, prio + 3 - c))) != cudaSuccess ||
@@ -1351,11 +1361,12 @@ sbfs_status sbfs_destroy(sbfs_handle *h)
         if (L.ev_done) cudaEventDestroy(L.ev_done);
         if (L.ev_in) cudaEventDestroy(L.ev_in);
         if (L.ev_fork) cudaEventDestroy(L.ev_fork);
-        for (int c = 0; c < 3; ++c) {
-            if (L.aux[c]) cudaStreamDestroy(L.aux[c]);
-            if (L.ev_join[c]) cudaEventDestroy(L.ev_join[c]);
-            L.spill_c[c].release();
-        }
+        if (L.ev_wide) cudaEventDestroy(L.ev_wide);
+        for (cudaStream_t a : L.aux)
+            if (a) cudaStreamDestroy(a);
+        for (cudaEvent_t ev : L.ev_join)
+            if (ev) cudaEventDestroy(ev);
+        for (DevBuf &d : L.spill_c) d.release();
         for (DevBuf &d : L.heavy) d.release();
         for (DevBuf &d : L.heavy_queue) d.release();
         for (DevBuf &d : L.mid_spill) d.release();

@@ -123,6 +123,10 @@ __device__ __forceinline__ void record_result(const Batch &b, int64_t k, int n, 
     if (len >= 0 && b.synchronizing) atomicAdd(b.synchronizing, 1ull);
 }
 
+// Bits of k_mid's visited bitmap; k_hash hands automata whose images need more
+// (n > 17 only: 2^n bits bound them) to k_cta.
+constexpr uint32_t kMidBits = 1u << 17;
+
 // Appends automaton k to a hand-off list with room for every automaton of the
 // launch's job.
 __device__ __forceinline__ void hand_off(const Batch &b, int32_t *list, unsigned long long *count, int64_t k)

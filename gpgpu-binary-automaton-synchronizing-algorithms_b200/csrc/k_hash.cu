@@ -31,7 +31,7 @@
 // settles the slowly synchronizing families and the automata that never
 // synchronize; one with a permutation letter and a letter merging at most one
 // pair is tried backwards at once.  What is left -- wide both ways -- goes to
-// one CTA per automaton (k_mid, or k_wide above n = 20) through a list.  Random
+// one CTA per automaton (k_mid or k_cta, or k_wide above n = 20) through a list.  Random
 // n = 17..20: 1.7 % of the automata pass 1536 subsets, 0.3 % pass 4096.
 // 200K mixed n = 6..20 with 1 % Cerny automata: 3.04 ms with every such
 // automaton on the CTA-wide kernel, 1.17 ms with the inverse search, 0.67 ms
@@ -427,8 +427,8 @@ __device__ __forceinline__ Forward forward_search(const Batch &b, int n, HashWar
 
 template <int MAXN, int SIZE>
 __global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32, HashGeom<MAXN, SIZE>::kCtas)
-    k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count,
-           unsigned long long *ticket)
+    k_hash(const __grid_constant__ Batch b, int32_t *heavy_list, unsigned long long *heavy_count, int32_t *wide_list,
+           unsigned long long *wide_count, unsigned long long *ticket)
 {
     using G = HashGeom<MAXN, SIZE>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -521,7 +521,9 @@ __global__ void __launch_bounds__(HashGeom<MAXN, SIZE>::kWarps * 32, HashGeom<MA
                 r = inverse_search(b, k, n, av, bv, W, lane);
                 expanded += r & ~kUnsettled;
             }
-            if ((r & kUnsettled) && lane == 0) hand_off(b, heavy_list, heavy_count, k);
+            const bool wide = MAXN == 20 && wide_list && bits > kMidBits;
+            if ((r & kUnsettled) && lane == 0)
+                hand_off(b, wide ? wide_list : heavy_list, wide ? wide_count : heavy_count, k);
             __syncwarp();
             continue;
         }
@@ -601,12 +603,13 @@ struct HashLaunch {
         if (cached && blocks > 0) known[dev].store(blocks, std::memory_order_relaxed);
         return blocks;
     }
-    static cudaError_t launch(int ctas, const Batch &b, int32_t *list, unsigned long long *count,
-                              unsigned long long *ticket, cudaStream_t st)
+    static cudaError_t launch(int ctas, const Batch &b, int32_t *list, unsigned long long *count, int32_t *wide_list,
+                              unsigned long long *wide_count, unsigned long long *ticket, cudaStream_t st)
     {
         cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
-        k_hash<MAXN, SIZE><<<ctas, HashGeom<MAXN, SIZE>::kWarps * 32, smem(), st>>>(b, list, count, ticket);
+        k_hash<MAXN, SIZE><<<ctas, HashGeom<MAXN, SIZE>::kWarps * 32, smem(), st>>>(b, list, count, wide_list,
+                                                                                    wide_count, ticket);
         return cudaGetLastError();
     }
 };
@@ -615,7 +618,9 @@ struct HashLaunch {
 
 // size 1: 1536 subsets per warp and a store of 1024 words (n <= 16) or 2048, size 2:
 // twice that; as a hash set three quarters of the store's words.
-// max_n: the largest n of the launch's automata (more than 20 states: size 2 only)
+// max_n: the largest n of the launch's automata (more than 20 states: size 2 only).
+// What a warp does not settle goes to heavy_list, or to wide_list (not null where
+// max_n is 18..20) if its images need more than kMidBits.
 int hash_max_ctas_per_sm(int size, int max_n)
 {
     if (max_n > 20) return size == 2 ? HashLaunch<28, 2>::per_sm() : 0;
@@ -624,19 +629,22 @@ int hash_max_ctas_per_sm(int size, int max_n)
 }
 
 cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
-                        unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st)
+                        unsigned long long *heavy_count, int32_t *wide_list, unsigned long long *wide_count,
+                        unsigned long long *ticket, cudaStream_t st)
 {
     if (ctas < 1 || !heavy_list || !heavy_count || max_n > SBFS_MAX_N) return cudaErrorInvalidValue;
     if (max_n > 20)
-        return size == 2 ? HashLaunch<28, 2>::launch(ctas, b, heavy_list, heavy_count, ticket, st)
+        return size == 2 ? HashLaunch<28, 2>::launch(ctas, b, heavy_list, heavy_count, nullptr, nullptr, ticket, st)
                          : cudaErrorInvalidValue;
     if (max_n > 16) {
-        if (size == 1) return HashLaunch<20, 1>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
-        if (size == 2) return HashLaunch<20, 2>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+        if (size == 1)
+            return HashLaunch<20, 1>::launch(ctas, b, heavy_list, heavy_count, wide_list, wide_count, ticket, st);
+        if (size == 2)
+            return HashLaunch<20, 2>::launch(ctas, b, heavy_list, heavy_count, wide_list, wide_count, ticket, st);
         return cudaErrorInvalidValue;
     }
-    if (size == 1) return HashLaunch<16, 1>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
-    if (size == 2) return HashLaunch<16, 2>::launch(ctas, b, heavy_list, heavy_count, ticket, st);
+    if (size == 1) return HashLaunch<16, 1>::launch(ctas, b, heavy_list, heavy_count, nullptr, nullptr, ticket, st);
+    if (size == 2) return HashLaunch<16, 2>::launch(ctas, b, heavy_list, heavy_count, nullptr, nullptr, ticket, st);
     return cudaErrorInvalidValue;
 }
 

@@ -224,14 +224,16 @@ __global__ void __launch_bounds__(kWideThreads, 1)
 // k_cta.cu's 2^20-bit bitmap allows, and no trips to global memory but for the
 // widest searches.  Those continue in a spill of 2^17 entries per CTA, those on
 // chip included (2^16 for n <= 16), which no search can outgrow: its subsets have
-// different bits.  Ranks that need more bits (n > 17 only) are left to k_cta.  The widest search of a batch bounds the
-// launch, hence 512 threads: 30K random n = 20 took 0.330 ms with k_cta alone,
-// 0.334 with 256 threads here, 0.315 with 512, 0.326 with 1024 (two CTAs per SM);
-// 200K mixed n = 6..20 0.611, 0.599, 0.591 and 0.611 ms.
+// different bits.  k_hash sends ranks that need more bits (n > 17 only) to k_cta,
+// which runs beside this kernel: after it 600 n = 18 of two rank 17 letters took
+// 736 us, so 546 (k_cta alone for all of them: 587), 30K random n = 20 322 and 295.
+// The widest search of a batch bounds the launch, hence 512 threads: 30K random
+// n = 20 took 0.330 ms with k_cta alone, 0.334 with 256 threads here, 0.315 with
+// 512, 0.326 with 1024 (two CTAs per SM); 200K mixed n = 6..20 0.611, 0.599, 0.591
+// and 0.611 ms (all with k_cta after it).
 constexpr int kMidThreads = 512;
 constexpr uint32_t kMidLimit = 8192;
-constexpr uint32_t kMidMaxSubsets = 1u << 17;   // a search's, by its bitmap
-constexpr int kMidWords = 4096;
+constexpr int kMidWords = kMidBits / 32;
 constexpr int kMidChunks = 5;
 
 struct MidSmem {
@@ -250,8 +252,7 @@ struct MidCtl {
 };
 
 __global__ void __launch_bounds__(kMidThreads, 3)
-    k_mid(const __grid_constant__ Batch b, uint2 *spill_base, uint32_t spill_entries, int32_t *left_list,
-          unsigned long long *left_count, unsigned long long *ticket)
+    k_mid(const __grid_constant__ Batch b, uint2 *spill_base, uint32_t spill_entries, unsigned long long *ticket)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MidSmem &S = *reinterpret_cast<MidSmem *>(smem_raw);
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kMidThreads, 3)
                     bits = 1u << n;
                     ctl.index0 = ctl.shift = 0u;
                 }
-                ctl.bits = bits;
+                ctl.bits = SBFS_CHECK(bits <= kMidBits, b.error) ? bits : kMidBits;
                 ctl.found[0] = ctl.found[1] = ~0u;
                 ctl.cnt[0] = ctl.cnt[1] = ctl.cnt[2] = 0u;
             }
@@ -312,11 +313,6 @@ __global__ void __launch_bounds__(kMidThreads, 3)
         if (k < 0) break;
         const int n = ctl.n;
         const uint32_t low_end = ctl.low_end, index0 = ctl.index0, shift = ctl.shift, bits = ctl.bits;
-        if (bits > 32u * kMidWords) {
-            if (tid == 0) hand_off(b, left_list, left_count, k);
-            __syncthreads();   // every thread has read ctl
-            continue;
-        }
         if (tid < 16 * kMidChunks) {
             const int c = tid >> 4, v = tid & 15;
             uint64_t acc = 0;
@@ -333,7 +329,8 @@ __global__ void __launch_bounds__(kMidThreads, 3)
         // the root comes back only through a permutation, and then the index is plain:
         // the first level sets its bit before any other thread reads the store
         uint32_t ls = 0, le = n > 1 ? 1u : 0u, level = 0;
-        if (tid == 0 && (index0 == 0u || low_end > full)) S.store[full >> 5] |= 1u << (full & 31u);
+        if (tid == 0 && (index0 == 0u || low_end > full) && SBFS_CHECK((full >> 5) < (uint32_t)kMidWords, b.error))
+            S.store[full >> 5] |= 1u << (full & 31u);
         while (true) {
             uint32_t *cnt = &ctl.cnt[level % 3];
             uint32_t *found = &ctl.found[level & 1];
@@ -449,22 +446,21 @@ int mid_ctas(int sm_count, int64_t count)
 // up to max_n states
 size_t mid_spill_entries(int max_n)
 {
-    const size_t most = max_n < 17 ? (size_t)1 << max_n : kMidMaxSubsets;
+    const size_t most = max_n < 17 ? (size_t)1 << max_n : kMidBits;   // by its bitmap
     return most > kMidLimit ? most - kMidLimit : 0;
 }
 
-// Solves the automata of b (at most max_n <= 20 states); those whose ranks need
-// more than 2^17 bits (n > 17 only) are appended to left_list.
-cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, int32_t *left_list,
-                       unsigned long long *left_count, unsigned long long *ticket, cudaStream_t st)
+// Solves the automata of b (at most max_n <= 20 states, images of at most
+// kMidBits bits).
+cudaError_t launch_mid(int ctas, int max_n, const Batch &b, uint64_t *spill, unsigned long long *ticket,
+                       cudaStream_t st)
 {
-    if (ctas < 1 || !left_list || !left_count) return cudaErrorInvalidValue;
+    if (ctas < 1) return cudaErrorInvalidValue;
     static std::atomic<int> done[16];
     const cudaError_t e = allow_smem(k_mid, sizeof(MidSmem), done);
     if (e != cudaSuccess) return e;
     k_mid<<<ctas, kMidThreads, sizeof(MidSmem), st>>>(b, reinterpret_cast<uint2 *>(spill),
-                                                      (uint32_t)mid_spill_entries(max_n), left_list, left_count,
-                                                      ticket);
+                                                      (uint32_t)mid_spill_entries(max_n), ticket);
     return cudaGetLastError();
 }
 

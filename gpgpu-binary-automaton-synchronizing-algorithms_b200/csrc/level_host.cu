@@ -12,7 +12,8 @@ namespace sbfs {
 
 int hash_max_ctas_per_sm(int size, int max_n);
 cudaError_t launch_hash(int size, int max_n, int ctas, const Batch &b, int32_t *heavy_list,
-                        unsigned long long *heavy_count, unsigned long long *ticket, cudaStream_t st);
+                        unsigned long long *heavy_count, int32_t *wide_list, unsigned long long *wide_count,
+                        unsigned long long *ticket, cudaStream_t st);
 cudaError_t launch_wide(int sm_count, const Batch &b, int32_t *left_list, unsigned long long *left_count,
                         unsigned long long *ticket, cudaStream_t st);
 
@@ -188,7 +189,7 @@ cudaError_t LevelEngine::launch_try(int n)
     const int per_sm = hash_max_ctas_per_sm(2, SBFS_MAX_N);
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     if ((e = launch_hash(2, SBFS_MAX_N, std::min(n, per_sm * sm_count_), b, d_try_->list[0], &d_try_->range[0][1],
-                         &d_try_->ticket[0], st_)) != cudaSuccess)
+                         nullptr, nullptr, &d_try_->ticket[0], st_)) != cudaSuccess)
         return e;
     b.order = d_try_->list[0];
     b.range_dev = d_try_->range[0];

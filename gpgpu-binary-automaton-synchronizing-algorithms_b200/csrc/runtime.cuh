@@ -36,8 +36,8 @@ struct DevCounters {
     // {offset 0, count} work ranges, and the tickets of the kernel that takes them
     unsigned long long heavy_range[kNumClasses][2];
     unsigned long long heavy_ticket[kNumClasses];
-    // what k_mid (classes 2 and 3) or k_wide (class 4) hands on in turn, to k_cta
-    // or the level slots, and k_cta's tickets
+    // what k_hash hands to k_cta (class 3), or k_wide to the level slots (class 4),
+    // and k_cta's tickets
     unsigned long long left_range[kNumClasses][2];
     unsigned long long left_ticket[kNumClasses];
     int error;
@@ -87,8 +87,9 @@ struct Lane {
     cudaEvent_t ev_in = nullptr;               // this lane's records have arrived (host path)
     // a mixed batch's size classes 0..2 run on these, beside class 3 on `stream`
     // (their tails -- a Cerny C_16 or C_20 each -- then overlap instead of adding up)
-    cudaStream_t aux[3] = {nullptr, nullptr, nullptr};
-    cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr};
+    // -- and k_cta on aux[3] beside k_mid
+    cudaStream_t aux[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_wide = nullptr, ev_join[4] = {nullptr, nullptr, nullptr, nullptr};
     DevBuf spill_c[3];                         // queue spill of a pooled class, one per class
     // a class's hand-off lists, their CTA queues, and k_mid's spill (classes 2, 3)
     DevBuf heavy[kNumClasses], heavy_queue[4], mid_spill[2];
